@@ -489,8 +489,12 @@ static void backproject(bsar_ctx* ctx, bsar_scene_id id, const bsar_grid* g, con
     MixedReq r = mixed_request(s, a, o->precision == BSAR_MIXED_FP16, o->flags);
     // small grids: each tile's pulses in K chunks, so the work items fill the GPU
     const int64_t vtiles = (a.v_count + 127) / 128;
-    const int K = mixed_chunks(nv_grid, a.np);
+    int K = mixed_chunks(nv_grid, a.np);
     std::unique_ptr<DevBuf> partial, tile_done, chunks;
+    // a budget that has no room for the chunks' sums takes the whole pulse range at once
+    if (ctx->used + sizeof(double2) * (size_t)K * (size_t)nv_grid + sizeof(int) * (size_t)vtiles + sizeof(MixedChunks) >
+        ctx->budget)
+        K = 1;
     if (K > 1) {
         partial = dev_alloc(ctx, sizeof(double2) * (size_t)K * (size_t)(g->nx * g->ny * g->nz));
         tile_done = dev_alloc(ctx, sizeof(int) * (size_t)vtiles);

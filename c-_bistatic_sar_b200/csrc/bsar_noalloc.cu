@@ -80,11 +80,14 @@ extern "C" bsar_status bsar_backproject_mixed_noalloc(bsar_ctx* ctx, bsar_scene_
         const size_t o_axes = o_off + up256(32 * (size_t)np);
         const size_t o_img = o_axes + up256(8 * (size_t)(g->nx + g->ny + g->nz));
         const int64_t vtiles = (nv + 127) / 128;
-        const int K = mixed_chunks(nv, (int)np);
+        int K = mixed_chunks(nv, (int)np);
         const size_t o_chk = o_img + up256(16 * (size_t)nv);
-        const size_t o_part = o_chk + (K > 1 ? up256(sizeof(MixedChunks)) : 0);
-        const size_t o_done = o_part + (K > 1 ? up256(16 * (size_t)K * (size_t)nv) : 0);
-        const size_t need = o_done + (K > 1 ? up256(4 * (size_t)vtiles) : 0);
+        const size_t o_part = o_chk + up256(sizeof(MixedChunks));
+        auto part_bytes = [&] { return up256(16 * (size_t)K * (size_t)nv); };
+        // a scratch that has no room for the chunks' sums takes the whole pulse range at once
+        if (o_part + part_bytes() + up256(4 * (size_t)vtiles) > kScratchBytes) K = 1;
+        const size_t o_done = o_part + part_bytes();
+        const size_t need = K > 1 ? o_done + up256(4 * (size_t)vtiles) : o_chk;
         if (need > kScratchBytes)
             fail(BSAR_ERR_INVALID_ARG, "the call needs %zu bytes of scratch; the fixed scratch holds %zu", need,
                  kScratchBytes);

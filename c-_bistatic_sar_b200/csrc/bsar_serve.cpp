@@ -71,13 +71,12 @@ struct Req {
     double deadline_s = 0;          // scheduling deadline, seconds after the server started
 };
 
-// Upper bound of the pulse-chunk buffers of a grid of nv voxels: at most 8 chunks per
-// 128-voxel tile, and chunks only while the tiles leave resident CTAs idle (fewer than
-// 4096 tiles on any device).  Host-only, so it does not ask the device.
+// Upper bound of the pulse-chunk buffers of a grid of nv voxels (mixed_chunks).  Host-only,
+// so it does not ask the device.
 uint64_t chunk_bytes(uint64_t nv)
 {
     const uint64_t tiles = (nv + 127) / 128;
-    return tiles < 4096 ? 16 * 8 * nv + 4 * tiles : 0;
+    return tiles <= kMaxChunkedTiles ? 16 * kMaxChunks * nv + 4 * tiles : 0;
 }
 
 uint64_t estimate_bytes(const Req& r)

@@ -1,34 +1,46 @@
 // k_mixed.cu -- the mixed-precision back-projection kernel.
 //
-// One thread per voxel, voxels of a CTA consecutive in the reference's flat order
-// (y fastest), every thread walking the pulses in order.  Lanes of a warp solve the same
-// pulse for neighbouring voxels, so their DEM windows, Tx/Rx loads and sample gathers
-// coincide or sit next to each other.
+// One thread per voxel; the 32 voxels of a warp are a compact block of the grid
+// (compact_voxel) and walk the pulses in order, in blocks of up to 16 consecutive pulses
+// whose antennas lie close together.
 //
-// DEM tile: at start every CTA stages a TI x TJ FP32 tile of the DEM around its voxels
-// (shifted by the scene's mean crossing offset) into shared memory with one TMA 2-D
-// tiled load (cp.async.bulk.tensor, no multicast) completing on an mbarrier; node scans
-// whose window lies inside the tile read it from there, others read the FP32 DEM in
-// global memory.
-//
-// Per (voxel, pulse):
-//   Fermat, twice (Tx -> voxel, voxel -> Rx):
-//     FP32  flat-interface start; node scan of the (2W+1)^2 DEM nodes around it
-//           (compile-time W for the common widths) ranking na|N-A| + nb|N-B|; when the
-//           runner-up is within kTieM metres of the best, the candidates within kTieM are
-//           re-ranked in FP64 with the FP64 solver's arithmetic and scan order, so both
-//           forms pick the same node; active-set Newton polish on the 4 facets around it
-//     FP64  one final Newton step on the winning facet; its leg lengths give the
-//           bistatic optical path L in FP64
+// Per pulse block and leg (Tx -> voxel, voxel -> Rx), by the warp together:
+//   candidate list: the DEM nodes that can win the node scan of any (voxel, pulse) pair of
+//           the block, found by one bounded ranking for the block's centre antenna and the
+//           warp's centre voxel (build_list); lists of up to four nodes carry the nodes' FP64
+//           path legs per pulse and per voxel, and whether each node is itself the crossing
+//           for the whole block (node_pinned)
+// Per (voxel, pulse) and leg:
+//   node    the list's best node: the smallest sum of two tabled FP64 legs, or FP32 values
+//           with near ties re-ranked in FP64 -- the node the FP64 solver's scan picks
+//   path    a pinned node's sum is the path; otherwise FP32 active-set Newton polish of the
+//           four facets around the node and one FP64 final Newton step
 //   delay / phase: dL = L - L_ref(pulse) rounded to FP32; the fast-time bin and carrier
 //           phase are FP32 offsets from per-pulse FP64 anchors (integer bin + fraction,
 //           phase reduced to [-pi, pi) in FP64)
 //   gather: two complex64 (or FP16 complex x pulse scale) samples, linear interpolation
 //           (proc_test_script.cpp:589-636), times exp(j phi), Kahan-compensated FP32 sum.
+// A block's legs are solved leg by leg over its pulses, then all its delays, gathers and
+// sums run in one short loop: the warps of an SM stay in small pieces of code.
+//
+// What bounds it: instruction issue and fetch (47 % of issue slots on the medium scene; the
+// rough DEM leaves about a quarter of the leg solves to polish).  Against the scan of every
+// lane's own window with per-lane lower bounds, one B200: 161 x 161 x 81 voxels x 1024
+// pulses on a 0.25 m DEM 528 -> 88 ms; 256 x 256 x 8 x 2048 on 0.125 m 647 -> 48 ms;
+// 97 x 83 x 11 x 701 on 0.2 m (no compile-time scan width) 74.7 -> 5.8 ms.  Block length
+// (kBlockSlope) 0.006 / 0.0125 / 0.025 / 0.05: 25.4 / 24.1 / 26.4 / 30.4 ms on 16 slices of
+// the medium grid; 5 CTAs per SM instead of 4 (96 registers): 15 % slower.
+//
+// DEM tile: for wide scans (25 x 25 and generic widths) every CTA stages a TI x TJ FP32
+// tile of the DEM around its voxels (shifted by the scene's mean crossing offset) into
+// shared memory with one TMA 2-D tiled load (cp.async.bulk.tensor, no multicast) completing
+// on an mbarrier; rankings whose nodes lie inside the tile read it from there, others read
+// the FP32 DEM in global memory.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 
@@ -50,6 +62,9 @@ constexpr float kTieM = 5.0e-5f;
 // 7.6e-6 m) plus the FP32 quantisation of the node coordinate (ulps of the largest index).
 constexpr float kStartBandM = 2.5e-5f;
 constexpr float kStartBandUlps = 8.0f;
+// A polish step shorter than this (cell units) is the last: Newton's next one would be about
+// its square, 1e-5 cells, which moves the path by 1e-11 m and which the FP64 step makes.
+constexpr float kConverged = 4e-3f;
 constexpr long kWaitSpins = 1L << 24;
 
 struct Facet32 {
@@ -66,8 +81,8 @@ struct MixedCtx {
     double ox, oy;                  // origin of the FP32 frame (first DEM node)
     double idx64, idy64;            // 1 / spacing, FP64
     float start_band;               // node units: FP32 starts this close to a cell boundary go FP64
-    int prune;                      // node scans may skip what the lower bound excludes
-    float zmin;                     // lowest FP32 height of the DEM
+    int lists;                      // node scans may run on candidate lists
+    float extent;                   // largest coordinate of the FP32 frame
 };
 
 // Start heights under a voxel (the lower endpoint of both of its paths when the ground
@@ -177,11 +192,25 @@ __device__ __forceinline__ float facet_eval32(const Facet32& F, const float A[3]
     return na * (q1 * rsqrtf(q1)) + nb * (q2 * rsqrtf(q2));
 }
 
+// FP64 distance of (x, y, z) from a leg's endpoint, and a path from its two legs, with the
+// FP64 solver's operations (no contraction): a node's path has the same bits wherever it is
+// formed (a pulse block's tables, the FP64 re-rank, the final step), and ranks as there.
+__device__ __forceinline__ double leg_len64(double x, double y, double z, const double E[3])
+{
+    const double dx = __dsub_rn(x, E[0]), dy = __dsub_rn(y, E[1]), dz = __dsub_rn(z, E[2]);
+    return __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
+}
+
+__device__ __forceinline__ double path64(double lenE, double lenG, double nE, double nG)
+{
+    return __dadd_rn(__dmul_rn(nE, lenE), __dmul_rn(nG, lenG));
+}
+
 // FP64 final Newton step on facet (fi, fj) from (u, v); returns the optical path of the
-// result and its two leg lengths (|X-A|, |X-B|).
+// result.
 __device__ __forceinline__ double final_step64(const DemView& d, int fi, int fj, const double A[3], const double B[3],
-                                               double na, double nb, double u, double v, double& dA, double& dB,
-                                               double* X, double idx_, double idy)
+                                               double na, double nb, double u, double v, double* X, double idx_,
+                                               double idy)
 {
     Facet64 F;
     facet_load(d, fi, fj, F);
@@ -235,29 +264,27 @@ __device__ __forceinline__ double final_step64(const DemView& d, int fi, int fj,
     }
     double x = F.x0 + u * F.dx, y = F.y0 + v * F.dy;
     double h = F.z00 + F.b * u + F.c * v + F.e * u * v;
-    double r1x = x - A[0], r1y = y - A[1], r1z = h - A[2];
-    double r2x = x - B[0], r2y = y - B[1], r2z = h - B[2];
-    dA = sqrt(r1x * r1x + r1y * r1y + r1z * r1z);
-    dB = sqrt(r2x * r2x + r2y * r2y + r2z * r2z);
+    if ((u == 0.0 || u == 1.0) && (v == 0.0 || v == 1.0)) {
+        // a node: its own coordinates, so that the path is the one node_leg64 gives
+        const int i = fi + (int)u, j = fj + (int)v;
+        x = __ldg(d.xv + i);
+        y = __ldg(d.yv + j);
+        h = __ldg(d.z + (int64_t)j * d.nx + i);
+    }
     if (X) {
         X[0] = x;
         X[1] = y;
         X[2] = h;
     }
-    return na * dA + nb * dB;
+    return path64(leg_len64(x, y, h, A), leg_len64(x, y, h, B), na, nb);
 }
 
-// Node optical path in FP64 with the FP64 solver's exact arithmetic (no contraction):
-// na*sqrt(|N-A|^2) + nb*sqrt(|N-B|^2), sums and products in the same order.
-__device__ __forceinline__ double node_l64(const DemView& d, int i, int j, const double A[3], const double B[3],
-                                           double na, double nb)
+// Node optical path in FP64.
+__device__ __forceinline__ double node_l64(const DemView& d, int i, int j, const double E[3], const double G[3],
+                                           double nE, double nG)
 {
-    double xi = __ldg(d.xv + i), yj = __ldg(d.yv + j), zij = __ldg(d.z + (int64_t)j * d.nx + i);
-    double r1x = __dsub_rn(xi, A[0]), r1y = __dsub_rn(yj, A[1]), r1z = __dsub_rn(zij, A[2]);
-    double r2x = __dsub_rn(xi, B[0]), r2y = __dsub_rn(yj, B[1]), r2z = __dsub_rn(zij, B[2]);
-    double q1 = __dadd_rn(__dadd_rn(__dmul_rn(r1x, r1x), __dmul_rn(r1y, r1y)), __dmul_rn(r1z, r1z));
-    double q2 = __dadd_rn(__dadd_rn(__dmul_rn(r2x, r2x), __dmul_rn(r2y, r2y)), __dmul_rn(r2z, r2z));
-    return __dadd_rn(__dmul_rn(na, __dsqrt_rn(q1)), __dmul_rn(nb, __dsqrt_rn(q2)));
+    const double x = __ldg(d.xv + i), y = __ldg(d.yv + j), z = __ldg(d.z + (int64_t)j * d.nx + i);
+    return path64(leg_len64(x, y, z, E), leg_len64(x, y, z, G), nE, nG);
 }
 
 // Node ranking values.  G is the voxel-side endpoint of the path (index ng), E the
@@ -308,7 +335,7 @@ __device__ __noinline__ Rank scan_generic(const MixedCtx m, const float* ts, int
 constexpr int TBJ = 32;
 // table rows for a compile-time node-scan half width: the window plus slack for the
 // spread of the 32 lanes' window centres
-template <int WT> struct TableRows { static constexpr int v = WT > 0 ? 2 * WT + 1 + (WT >= 12 ? 5 : 7) : 1; };
+template <int WT> struct TableRows { static constexpr int v = WT > 0 ? 2 * WT + 1 + (WT >= 12 ? 1 : 7) : 1; };
 
 struct AirTable {
     float2* t;
@@ -348,8 +375,8 @@ __device__ __forceinline__ AirTable build_air_table(const MixedCtx& m, const Til
 // table (one 8-byte load per node), the G leg per node, columns unrolled with
 // compile-time offsets.  The best node's row is updated once per row.
 template <int W>
-__device__ __forceinline__ void scan_table_inl(const MixedCtx& m, const AirTable& AT, int is, int js, float gx,
-                                               float gy, float gz, float& v1, float& v2, int& bi, int& bj)
+__device__ __forceinline__ void scan_table(const MixedCtx& m, const AirTable& AT, int is, int js, float gx, float gy,
+                                           float gz, float& v1, float& v2, int& bi, int& bj)
 {
     constexpr int NJ = 2 * W + 1;
     float syg[NJ];
@@ -381,202 +408,6 @@ __device__ __forceinline__ void scan_table_inl(const MixedCtx& m, const AirTable
         bi = (v1 < v1_row) ? i : bi;
     }
     bj = js - W + bc;
-}
-
-// Out of line for the widths that prune: it runs for the exhaustive flag and for warps
-// whose lanes do not all have full windows, so its body stays out of the pulse loop's
-// instruction stream.
-template <int W>
-__device__ __noinline__ Rank scan_table(const MixedCtx m, const float2* tab, int ti0, int tj0, int is, int js, float gx,
-                                        float gy, float gz, Rank rk)
-{
-    const AirTable AT{const_cast<float2*>(tab), ti0, tj0, true};
-    scan_table_inl<W>(m, AT, is, js, gx, gy, gz, rk.v1, rk.v2, rk.bi, rk.bj);
-    return rk;
-}
-
-// Columns of a window row in groups of four for the pruned scan; a trailing single column
-// joins the last group (13 columns: 0-3, 4-7, 8-12).
-template <int W> struct ColGroups {
-    static constexpr int NJ = 2 * W + 1;
-    static constexpr int N = (NJ % 4 == 1) ? NJ / 4 : (NJ + 3) / 4;
-    __host__ __device__ static constexpr int first(int k) { return 4 * k; }
-    __host__ __device__ static constexpr int last(int k) { return k == N - 1 ? NJ - 1 : 4 * k + 3; }
-};
-
-// The table scan with exact pruning: rows, and groups of columns inside a row, whose
-// ranking values provably all exceed the pruning threshold are skipped.  The result (best
-// value, best node, and whether the runner-up lies within the tie band) is that of
-// scan_table, bit for bit:
-//  * a skipped node's value exceeds v1 + tie at the time of the skip, so it is neither the
-//    minimum nor within the tie band of the final minimum, and v2 - v1 >= tie is decided
-//    as before;
-//  * an exact FP32 tie between two nodes puts v2 == v1 and sends the lane to the FP64
-//    re-rank, so the order in which rows are visited (centre outward) does not choose
-//    between equal values.
-// The bound.  The E leg e(N) = re |N - E| is convex, so it lies above its tangent plane
-// at the start node N0: e(N) >= K + a.(N - G), a = re (N0 - E) / |N0 - E|.  On a row
-// (x fixed) with every height above zlo, the ranking value is at least
-//     K + a_x X + a_z Zl + min_Y [a_y Y + sqrt(X^2 + Zl^2 + Y^2)]
-// (X, Y, Zl: offsets from the voxel G; Zl from the row's lowest height), valid while
-// a_z Z + |N - G| grows with the height Z over the window (checked once per solve).  With
-// t = thr - K - a_x X - a_z Zl, the row holds no node at or below thr when t < 0 or
-// t^2 < (1 - a_y^2)(X^2 + Zl^2); a column group, whose Y lies in [Ylo, Yhi] and whose own
-// lowest height gives Zl, holds none when t < 0 or the parabola
-// (1 - a_y^2) Y^2 + 2 t a_y Y + X^2 + Zl^2 - t^2 is positive on [Ylo, Yhi].  The
-// threshold is v1 + tie, or sooner the value of `seed` (the previous pulse's best node,
-// when it lies in this window) + tie, widened by a margin far above the FP32 rounding of
-// the values and of the bound.  Warp-uniform: a row or group is skipped only when no lane
-// of the warp needs it, so all 32 lanes must call together.
-template <int W>
-__device__ __forceinline__ void scan_pruned(const MixedCtx& m, const AirTable& AT, int is, int js, const float E[3],
-                                            float gx, float gy, float gz, float re, float tie, int seed, float& v1,
-                                            float& v2, int& bi, int& bj)
-{
-    using CG = ColGroups<W>;
-    constexpr int NJ = 2 * W + 1;
-    const unsigned full = 0xffffffffu;
-    float syg[NJ];
-#pragma unroll
-    for (int c = 0; c < NJ; c++) {
-        float dy = (float)(js - W + c) * m.stepy - gy;
-        syg[c] = dy * dy;
-    }
-    const float2* row0 = AT.t + (is - W - AT.i0) * TBJ + (js - W - AT.j0);
-    // tangent plane of the E leg at the start node N0
-    const float2 n0 = row0[W * TBJ + W];
-    const float x0 = (float)is * m.stepx, y0 = (float)js * m.stepy;
-    // approximate divisions (2 ulp): the tangent plane and the parabola's vertex move by
-    // ~1e-7 relative, which changes the bound by far less than the threshold's margin
-    // (2e-4 m + 4e-6 |T|), so the skips stay exact
-    const float kk = __fdividef(re * re, n0.y);                    // re / |N0 - E|
-    const float ax = (x0 - E[0]) * kk, ay = (y0 - E[1]) * kk, az = (n0.x - E[2]) * kk;
-    const float K = n0.y + ax * (gx - x0) + ay * (gy - y0) + az * (gz - n0.x);
-    const float sy2 = 1.0f - ay * ay;
-    const float yv_t = __fdividef(-ay, sy2);                       // vertex of the parabola: Y = t * yv_t
-    const float ay2 = 2.0f * ay;
-    const float yfirst = (float)(js - W) * m.stepy - gy;
-    // height monotonicity over the window, from the DEM's lowest height (else nothing is
-    // pruned): d/dZ [a_z Z + |N - G|] = a_z + Z / |N - G| (Z above the voxel) is positive
-    // for every node only if the voxel lies below the DEM's lowest height (Z >= Zt > 0),
-    // and, for a_z < 0, Z^2 >= a_z^2 |N - G|^2 at the window's farthest corner
-    const float Zt = m.zmin - gz;
-    const float hx = fabsf(x0 - gx) + (float)W * m.stepx, hy = fabsf(y0 - gy) + (float)W * m.stepy;
-    const bool bound_ok = sy2 > 1e-3f &&           // |a| = re: the bound needs the E leg's index below the G leg's
-                          Zt > 0.0f && (az >= 0.0f || az * az * (hx * hx + hy * hy + Zt * Zt) <= Zt * Zt);
-    // seed: the previous pulse's best node, ranked with the scan's own arithmetic
-    float thr_seed = INFINITY;
-    {
-        const int si = seed >> 16, sj = seed & 0xffff;
-        if (seed >= 0 && abs(si - is) <= W && abs(sj - js) <= W) {
-            const float2 e = row0[(si - is + W) * TBJ + (sj - js + W)];
-            const float dx = (float)si * m.stepx - gx, dy = (float)sj * m.stepy - gy;
-            const float dz = e.x - gz;
-            const float q = fmaf(dz, dz, dx * dx + dy * dy);
-            thr_seed = fmaf(q, rsqrtf(q), e.y);
-        }
-    }
-    const float never = bound_ok ? 0.0f : INFINITY;     // +inf: keep every node
-    int bc = bj - (js - W);
-#pragma unroll 1
-    for (int k = 0; k < NJ; k++) {
-        const int d = (k + 1) >> 1;
-        const int r = (k & 1) ? W - d : W + d;          // rows from the start node outward
-        const int i = is - W + r;
-        const float dx = (float)i * m.stepx - gx;
-        const float sxg = dx * dx;
-        const float2* row = row0 + r * TBJ;
-        float T = fminf(thr_seed, v1) + tie + never;
-        T = T + fmaf(4e-6f, fabsf(T), 2e-4f);
-        const float R = T - K - ax * dx;
-        float2 e[NJ];
-#pragma unroll
-        for (int c = 0; c < NJ; c++) e[c] = row[c];
-        float zg[CG::N];
-#pragma unroll
-        for (int g = 0; g < CG::N; g++) {
-            zg[g] = e[CG::first(g)].x;
-#pragma unroll
-            for (int c = CG::first(g) + 1; c <= CG::last(g); c++) zg[g] = fminf(zg[g], e[c].x);
-        }
-        // the whole row (Y free) against its lowest height
-        {
-            float zr = zg[0];
-#pragma unroll
-            for (int g = 1; g < CG::N; g++) zr = fminf(zr, zg[g]);
-            const float zl = zr - gz;
-            const float t = R - az * zl;
-            const bool skip = t < 0.0f || t * t < sy2 * fmaf(zl, zl, sxg);
-            if (!__any_sync(full, !skip)) continue;
-        }
-        const float v1_row = v1;
-#pragma unroll
-        for (int g = 0; g < CG::N; g++) {
-            const int c0 = CG::first(g), c1 = CG::last(g);
-            const float zl = zg[g] - gz;
-            const float t = R - az * zl;
-            const float ylo = fmaf((float)c0, m.stepy, yfirst), yhi = fmaf((float)c1, m.stepy, yfirst);
-            const float yc = fminf(fmaxf(t * yv_t, ylo), yhi);
-            const float q = fmaf(fmaf(sy2, yc, ay2 * t), yc, fmaf(-t, t, fmaf(zl, zl, sxg)));
-            const bool skip = t < 0.0f || q > 0.0f;
-            if (!__any_sync(full, !skip)) continue;
-#pragma unroll
-            for (int c = c0; c <= c1; c++) {
-                const float dz = e[c].x - gz;
-                const float qq = fmaf(dz, dz, sxg + syg[c]);
-                const float L = fmaf(qq, rsqrtf(qq), e[c].y);
-                v2 = fminf(v2, fmaxf(v1, L));
-                const bool p = L < v1;
-                v1 = p ? L : v1;
-                bc = p ? c : bc;
-            }
-        }
-        bi = (v1 < v1_row) ? i : bi;
-    }
-    bj = js - W + bc;
-}
-
-// Narrowest node-scan half width whose table scan is pruned.
-constexpr int kPruneMinW = 6;
-
-template <int W, bool TABLE>
-__device__ __forceinline__ void node_scan(const MixedCtx& m, const Tile& T, const AirTable& AT, int is, int js, int Wr,
-                                          const float E[3], const float G[3], float re, float tie, int seed, float& v1,
-                                          float& v2, int& bi, int& bj)
-{
-    const int ia = max(is - Wr, 0), ib = min(is + Wr, m.nx - 1);
-    const int ja = max(js - Wr, 0), jb = min(js + Wr, m.ny - 1);
-    const bool in_tile = T.ok && ia >= T.i0 && ib < T.i0 + TI && ja >= T.j0 && jb < T.j0 + TJ;
-    if constexpr (W > 0 && W < kPruneMinW && TABLE) {
-        // small windows: every node, inline (the bound tests would cost more than they save)
-        if (AT.ok && Wr == W && ia == is - W && ib == is + W && ja == js - W && jb == js + W) {
-            scan_table_inl<W>(m, AT, is, js, G[0], G[1], G[2], v1, v2, bi, bj);
-            return;
-        }
-    }
-    if constexpr (W >= kPruneMinW && TABLE) {
-        const bool full_window = AT.ok && Wr == W && ia == is - W && ib == is + W && ja == js - W && jb == js + W;
-        // the pruned scan votes across the warp: only when every lane takes it
-        const bool all_full = __all_sync(0xffffffffu, full_window);
-        if (all_full && m.prune) {
-            scan_pruned<W>(m, AT, is, js, E, G[0], G[1], G[2], re, tie, seed, v1, v2, bi, bj);
-            return;
-        }
-        if (full_window) {
-            const Rank r = scan_table<W>(m, AT.t, AT.i0, AT.j0, is, js, G[0], G[1], G[2], Rank{v1, v2, bi, bj});
-            v1 = r.v1;
-            v2 = r.v2;
-            bi = r.bi;
-            bj = r.bj;
-            return;
-        }
-    }
-    Rank r = scan_generic(m, T.s, T.i0, T.j0, in_tile, ia, ib, ja, jb, E[0], E[1], E[2], G[0], G[1], G[2], re,
-                          Rank{v1, v2, bi, bj});
-    v1 = r.v1;
-    v2 = r.v2;
-    bi = r.bi;
-    bj = r.bj;
 }
 
 // FP64 re-ranking of the nodes within the FP32 ambiguity band, with the FP64 solver's
@@ -674,100 +505,512 @@ __device__ __noinline__ int2 rerank64_warp(const DemView d, const MixedCtx m, co
 
 // FP64 flat-interface start and its nearest node, exactly as the FP64 solver makes them
 // (used when the FP32 start lies within rounding distance of a node-cell boundary).
-__device__ __noinline__ int2 start_node64(const DemView d, double Ax, double Ay, double Az, double Bx, double By,
-                                          double Bz, double na, double nb, double h0_known)
+__device__ __noinline__ int2 start_node64(const DemView d, double Ex, double Ey, double Ez, double Gx, double Gy,
+                                          double Gz, double nE, double nG, bool g_lower, double h0_known)
 {
-    const double A[3] = {Ax, Ay, Az}, B[3] = {Bx, By, Bz};
-    const bool lower_b = nb >= na;
-    const double* Lp = lower_b ? B : A;
-    const double* Up = lower_b ? A : B;
-    double nl = lower_b ? nb : na, nu = lower_b ? na : nb;
+    const double E[3] = {Ex, Ey, Ez}, G[3] = {Gx, Gy, Gz};
+    const double* Lp = g_lower ? G : E;
+    const double* Up = g_lower ? E : G;
+    double nl = g_lower ? nG : nE, nu = g_lower ? nE : nG;
     const double h0 = isnan(h0_known) ? dem_elevation(d, Lp[0], Lp[1]) : h0_known;
     double sx, sy;
     flat_start(Up, Lp, nu, nl, h0, kFlatIters, sx, sy);
     return make_int2(nearest_node(d.x0, d.stepx, d.nx, sx), nearest_node(d.y0, d.stepy, d.ny, sy));
 }
 
-// Mixed-precision crossing solve A (index na) -> B (index nb); the voxel-side endpoint G
-// is B when g_is_b, else A.  A32/B32: the endpoints in the FP32 frame.  With TABLE the
-// warp builds and uses the shared E-leg table (all 32 lanes must call together).
-// Returns the FP64 optical path; dA, dB: FP64 leg lengths; X (optional): the crossing.
-// seed (table form): in, the node this lane chose for the same leg at the previous pulse
-// ((i << 16) | j, or -1), which only speeds up the pruned scan; out, the node chosen now.
-template <int WT, bool TABLE>
-__device__ __forceinline__ double solve_mixed(const DemView& d, const MixedCtx& m, const Tile& T, float2* table_buf,
-                                              const double A[3], const double B[3],
-                                              const float A32[3], const float B32[3], float na, float nb,
-                                              bool g_is_b, int W, const VoxelStart& vs, int& seed, double& dA,
-                                              double& dB, double* X = nullptr)
+// Flat-interface start (FP32) of the path Up (index nu) -> Lp (index nl) over the height h0:
+// (sx, sy), the horizontal distance D of the endpoints and the length of the last step.
+struct FlatStart {
+    float sx, sy, D, last;
+};
+
+__device__ __forceinline__ FlatStart flat_start32(const float Up[3], const float Lp[3], float nu, float nl, float h0)
 {
-    // 1. flat-interface start (FP32); the lower endpoint is normally the voxel itself
-    const bool lower_b = nb >= na;
-    const bool lp_is_g = lower_b == g_is_b;
-    const float* Lp = lower_b ? B32 : A32;
-    const float* Up = lower_b ? A32 : B32;
-    const float nl = lower_b ? nb : na, nu = lower_b ? na : nb;
-    const float h0 = lp_is_g ? vs.h32 : height32(m, Lp[0], Lp[1]);
-    float hx = Lp[0] - Up[0], hy = Lp[1] - Up[1];
+    FlatStart f;
+    const float hx = Lp[0] - Up[0], hy = Lp[1] - Up[1];
     const float D2 = hx * hx + hy * hy;
-    float D = D2 * rsqrtf(D2);
-    float sx = Lp[0], sy = Lp[1];
+    const float D = D2 * rsqrtf(D2);
+    f.sx = Lp[0];
+    f.sy = Lp[1];
+    f.D = 0.0f;
+    f.last = 0.0f;
     if (D >= 1e-6f) {
         float ha = fabsf(Up[2] - h0), hb = fabsf(Lp[2] - h0);
         float s = fminf(fmaxf(__fdividef(D * ha, ha + hb + 1e-30f), 0.f), D);
+        float before = s;
 #pragma unroll
         for (int it = 0; it < kFlatIters; it++) {
             float q1 = s * s + ha * ha, r = D - s, q2 = r * r + hb * hb;
             float i1 = rsqrtf(q1), i2 = rsqrtf(q2);
             float g = nu * s * i1 - nl * r * i2;
             float gp = nu * ha * ha * i1 * i1 * i1 + nl * hb * hb * i2 * i2 * i2;
+            before = s;
             if (gp > 0.f) s = fminf(fmaxf(s - __fdividef(g, gp), 0.f), D);
         }
         const float t = __fdividef(s, D);
-        sx = Up[0] + hx * t;
-        sy = Up[1] + hy * t;
+        f.sx = Up[0] + hx * t;
+        f.sy = Up[1] + hy * t;
+        f.D = D;
+        f.last = fabsf(s - before);
     }
-    // 2. node scan (FP32, L / ng), FP64 re-rank of near ties.  The window centre is the
-    //    node nearest the start; a start within rounding distance of a cell boundary is
-    //    redone in FP64 so both forms scan the same window.
-    const float fx = sx * m.istepx, fy = sy * m.istepy;
-    int is = min(max(__float2int_rn(fx), 0), m.nx - 1);
-    int js = min(max(__float2int_rn(fy), 0), m.ny - 1);
-    if (fabsf(fabsf(fx - rintf(fx)) - 0.5f) < m.start_band || fabsf(fabsf(fy - rintf(fy)) - 0.5f) < m.start_band) {
-        const int2 s64 = start_node64(d, A[0], A[1], A[2], B[0], B[1], B[2], (double)na, (double)nb,
-                                      lp_is_g ? vs.h64 : (double)NAN);
-        is = s64.x;
-        js = s64.y;
-    }
-    const float* E = g_is_b ? A32 : B32;
-    const float* G = g_is_b ? B32 : A32;
-    const float ng = g_is_b ? nb : na;
-    const float re = __fdividef(g_is_b ? na : nb, ng);
-    AirTable AT{table_buf, 0, 0, false};
-    if constexpr (TABLE && WT > 0)
-        AT = build_air_table<TableRows<WT>::v>(m, T, table_buf, is, js, W, E[0], E[1], E[2], re);
-    float v1 = INFINITY, v2 = INFINITY;
-    int bi = is, bj = js;
-    const float tie = kTieM / ng;
-    node_scan<WT, TABLE>(m, T, AT, is, js, W, E, G, re, tie, seed, v1, v2, bi, bj);
-    const bool need = !(v2 - v1 >= tie);
-    if constexpr (TABLE) {
-        if (__any_sync(0xffffffffu, need)) {
-            const int2 b = rerank64_warp(d, m, T.s, T.i0, T.j0, T.ok, need, is, js, W, E[0], E[1], E[2], G[0], G[1],
-                                         G[2], re, v1 + tie, A[0], A[1], A[2], B[0], B[1], B[2], (double)na,
-                                         (double)nb, make_int2(bi, bj));
-            bi = b.x;
-            bj = b.y;
+    return f;
+}
+
+// One leg of one (voxel, pulse): the antenna E (index nE) and the voxel G (index nG), in
+// FP64 and in the FP32 frame.  The path is the same in both directions; only the flat start
+// asks which endpoint is the lower one (the one of the larger index, the leg's second
+// endpoint when they are equal).
+struct Leg {
+    double E[3], G[3];
+    float E32[3], G32[3];
+    float nE, nG;
+    double nE64, nG64;
+    bool g_lower;
+};
+
+__device__ __forceinline__ bool lower_is_voxel(float nE, float nG, bool to_voxel)
+{
+    return to_voxel ? nG >= nE : nG > nE;
+}
+
+// Window centre of a leg's node scan: the node nearest the flat start.  A start within
+// rounding distance of a cell boundary is redone in FP64 so both forms scan the same
+// window.
+__device__ __forceinline__ int2 start_node(const DemView& d, const MixedCtx& m, const Leg& l, const VoxelStart& vs)
+{
+    const float* Lp = l.g_lower ? l.G32 : l.E32;      // the lower endpoint is normally the voxel itself
+    const float* Up = l.g_lower ? l.E32 : l.G32;
+    const float h0 = l.g_lower ? vs.h32 : height32(m, Lp[0], Lp[1]);
+    const FlatStart f = flat_start32(Up, Lp, l.g_lower ? l.nE : l.nG, l.g_lower ? l.nG : l.nE, h0);
+    const float fx = f.sx * m.istepx, fy = f.sy * m.istepy;
+    int2 c = make_int2(min(max(__float2int_rn(fx), 0), m.nx - 1), min(max(__float2int_rn(fy), 0), m.ny - 1));
+    if (fabsf(fabsf(fx - rintf(fx)) - 0.5f) < m.start_band || fabsf(fabsf(fy - rintf(fy)) - 0.5f) < m.start_band)
+        c = start_node64(d, l.E[0], l.E[1], l.E[2], l.G[0], l.G[1], l.G[2], l.nE64, l.nG64, l.g_lower,
+                         l.g_lower ? vs.h64 : (double)NAN);
+    return c;
+}
+
+// Best node of one lane's own window, every node ranked (FP32, near ties in FP64).
+__device__ __forceinline__ int2 scan_lane(const DemView& d, const MixedCtx& m, const Tile& T, const Leg& l,
+                                          const VoxelStart& vs, int W)
+{
+    const int2 c = start_node(d, m, l, vs);
+    const float* E = l.E32;
+    const float* G = l.G32;
+    const float re = __fdividef(l.nE, l.nG);
+    const float tie = kTieM / l.nG;
+    const int ia = max(c.x - W, 0), ib = min(c.x + W, m.nx - 1);
+    const int ja = max(c.y - W, 0), jb = min(c.y + W, m.ny - 1);
+    const bool in_tile = T.ok && ia >= T.i0 && ib < T.i0 + TI && ja >= T.j0 && jb < T.j0 + TJ;
+    const Rank r = scan_generic(m, T.s, T.i0, T.j0, in_tile, ia, ib, ja, jb, E[0], E[1], E[2], G[0], G[1], G[2], re,
+                                Rank{INFINITY, INFINITY, c.x, c.y});
+    if (r.v2 - r.v1 >= tie) return make_int2(r.bi, r.bj);
+    return rerank64(d, m, T.s, T.i0, T.j0, T.ok, c.x, c.y, W, E[0], E[1], E[2], G[0], G[1], G[2], re, r.v1 + tie,
+                    l.E[0], l.E[1], l.E[2], l.G[0], l.G[1], l.G[2], l.nE64, l.nG64,
+                    make_int2(r.bi, r.bj));
+}
+
+// The same for a whole warp (all 32 lanes call): windows of the common widths ranked from
+// the warp's table, near ties re-ranked by the warp together.  Runs for the exhaustive
+// flag and where no candidate list holds, so it stays out of the pulse loop's
+// instruction stream.
+template <int WT>
+__device__ __noinline__ int2 scan_warp(const DemView d, const MixedCtx m, const Tile T, float2* table_buf, const Leg& l,
+                                       const VoxelStart vs, int W)
+{
+    const int2 c = start_node(d, m, l, vs);
+    const float* E = l.E32;
+    const float* G = l.G32;
+    const float re = __fdividef(l.nE, l.nG);
+    const float tie = kTieM / l.nG;
+    const int ia = max(c.x - W, 0), ib = min(c.x + W, m.nx - 1);
+    const int ja = max(c.y - W, 0), jb = min(c.y + W, m.ny - 1);
+    Rank r{INFINITY, INFINITY, c.x, c.y};
+    bool done = false;
+    if constexpr (WT > 0) {
+        const AirTable AT = build_air_table<TableRows<WT>::v>(m, T, table_buf, c.x, c.y, W, E[0], E[1], E[2], re);
+        if (AT.ok && W == WT && ia == c.x - WT && ib == c.x + WT && ja == c.y - WT && jb == c.y + WT) {
+            scan_table<WT>(m, AT, c.x, c.y, G[0], G[1], G[2], r.v1, r.v2, r.bi, r.bj);
+            done = true;
         }
-    } else if (need) {
-        const int2 b = rerank64(d, m, T.s, T.i0, T.j0, T.ok, is, js, W, E[0], E[1], E[2], G[0], G[1], G[2], re,
-                                v1 + tie, A[0], A[1], A[2], B[0], B[1], B[2], (double)na, (double)nb,
-                                make_int2(bi, bj));
-        bi = b.x;
-        bj = b.y;
     }
-    seed = (bi < 32768 && bj < 65536) ? (bi << 16) | bj : -1;
-    // 3. polish the facets around the best node (FP32); heights from the DEM tile when the
+    if (!done) {
+        const bool in_tile = T.ok && ia >= T.i0 && ib < T.i0 + TI && ja >= T.j0 && jb < T.j0 + TJ;
+        r = scan_generic(m, T.s, T.i0, T.j0, in_tile, ia, ib, ja, jb, E[0], E[1], E[2], G[0], G[1], G[2], re, r);
+    }
+    int2 best = make_int2(r.bi, r.bj);
+    const bool need = !(r.v2 - r.v1 >= tie);
+    if (__any_sync(0xffffffffu, need))
+        best = rerank64_warp(d, m, T.s, T.i0, T.j0, T.ok, need, c.x, c.y, W, E[0], E[1], E[2], G[0], G[1], G[2], re,
+                             r.v1 + tie, l.E[0], l.E[1], l.E[2], l.G[0], l.G[1], l.G[2], l.nE64, l.nG64,
+                             best);
+    return best;
+}
+
+// ------------------------------- candidate lists -------------------------------------
+// The node scan, shared by a warp's 32 voxels and a block of consecutive pulses.  A scan
+// keeps the node with the smallest ranking value L'(N) = re |N - E| + |N - G| in a window
+// around its flat start.  Neighbouring voxels G and consecutive antenna positions E rank
+// the same few nodes best, so the warp ranks the nodes once per block for the block's
+// centre antenna Ec and the warp's centre voxel Gc and lists those that can win for any of
+// its (voxel, pulse) pairs; each solve then ranks the list, with the scan's own
+// arithmetic, instead of the window.
+//
+// With S a node that every window holds, gap(N) = L'(N) - L'(S) moves with E by at most
+// re |u_N - u_S| per metre, u the unit vectors from the nodes to E, and |u_N - u_S| <=
+// 2 |N - S| / (|N - E| + |S - E|); likewise with G.  So a node with
+//     gap(N) at (Ec, Gc) > slack(N) + tie,
+//     slack(N) = 2 |N - S| (re rE / (|N-Ec| + |S-Ec| - 2 rE) + rG / (|N-Gc| + |S-Gc| - 2 rG)),
+// rE and rG the largest distances of the block's antennas and the warp's voxels from the
+// centres, is worse than S by more than the tie band for every pair: it is neither the
+// best node nor within the tie band of it, and the scan's result (best node, tie decision)
+// needs only the others.  A margin far above the FP32 rounding of the gaps is added.
+//
+// Windows.  A start moves with E by at most kappa = nE hG / (nE hG + nG hE) per metre
+// horizontally (hE, hG: the endpoints' heights over the start height; Snell's law gives
+// 0 <= d(dist)/dD <= dist / D <= kappa for nE <= nG), and by at most kappa D / hE per metre
+// of antenna height.  From the lanes' own starts at Ec this bounds every window centre of
+// the block: the warp ranks the union of the windows and requires S in their
+// intersection.  When all listed nodes lie in the intersection the starts themselves are
+// not needed; otherwise each solve makes its start and drops the nodes outside its window.
+//
+// No list (m = -1): antenna on the side of the larger index, start not converged,
+// intersection empty, or more nodes than the list holds; those blocks scan every window
+// node (scan_warp), as the exhaustive flag does.
+constexpr int kListCap = 96;
+constexpr int kBlockPulses = 16;    // longest pulse block
+
+constexpr int kCore = 1, kTables = 2;
+// Lists of at most kTabled nodes carry their FP64 legs (node_tables).
+constexpr int kTabled = 4;
+
+struct LegList {
+    int m;               // listed nodes (i-major order), -1: no list
+    int mode;            // kCore: every listed node lies in every window of the block
+    int i0, j0;          // origin of the entries' packed offsets
+    int si, sj;          // the last block's S (in: a first guess)
+    int pinned;          // kTables: bit k set when node k is its own crossing for the whole block
+    int pad;
+    int2 node[kTabled];  // kTables: the listed nodes
+};
+
+// Entry: x, y, z of the node in the FP32 frame, (i - i0) << 16 | (j - j0).
+__device__ __forceinline__ float4 list_entry(float x, float y, float z, int i, int j)
+{
+    return make_float4(x, y, z, __int_as_float((i << 16) | j));
+}
+
+__device__ __forceinline__ unsigned ordered_bits(float f)   // unsigned order = float order
+{
+    const unsigned u = __float_as_uint(f);
+    return u ^ ((u >> 31) ? 0xffffffffu : 0x80000000u);
+}
+
+// gap(N) - slack(N) of the node offset (x, y, z), and the gap itself.
+struct GapRef {
+    float E[3], G[3];     // block and warp centres
+    float S[3], eS, gS;   // S and its distances |S - Ec|, |S - Gc|
+    float re, cE, cG, rE2, rG2;
+};
+
+__device__ __forceinline__ void gap_set(GapRef& g, float x, float y, float z)
+{
+    g.S[0] = x;
+    g.S[1] = y;
+    g.S[2] = z;
+    float dx = x - g.E[0], dy = y - g.E[1], dz = z - g.E[2];
+    float q = fmaf(dz, dz, fmaf(dx, dx, dy * dy));
+    g.eS = q * rsqrtf(q);
+    dx = x - g.G[0], dy = y - g.G[1], dz = z - g.G[2];
+    q = fmaf(dz, dz, fmaf(dx, dx, dy * dy));
+    g.gS = q * rsqrtf(q);
+}
+
+__device__ __forceinline__ float gap_of(const GapRef& g, float x, float y, float z, float& gap)
+{
+    float dx = x - g.E[0], dy = y - g.E[1], dz = z - g.E[2];
+    float q = fmaf(dz, dz, fmaf(dx, dx, dy * dy));
+    const float e = q * rsqrtf(q);
+    dx = x - g.G[0], dy = y - g.G[1], dz = z - g.G[2];
+    q = fmaf(dz, dz, fmaf(dx, dx, dy * dy));
+    const float v = q * rsqrtf(q);
+    dx = x - g.S[0], dy = y - g.S[1], dz = z - g.S[2];
+    q = fmaf(dz, dz, fmaf(dx, dx, dy * dy));
+    const float nS = q * rsqrtf(fmaxf(q, 1e-30f));
+    gap = fmaf(g.re, e - g.eS, v - g.gS);
+    // denominators at or below zero (a voxel or antenna among the nodes): keep the node
+    const float kE = __fdividef(g.cE, fmaxf(e + g.eS - g.rE2, 1e-6f));
+    const float kG = __fdividef(g.cG, fmaxf(v + g.gS - g.rG2, 1e-6f));
+    return gap - nS * (kE + kG);
+}
+
+// Builds one leg's list for the block (all 32 lanes call).  E: the block's centre antenna,
+// rEh / rEz / rE the antennas' largest horizontal, vertical and 3-D distance from it, dh0
+// the spread of the start height over the block when it lies under the antenna (else 0);
+// G this lane's voxel, Gc / rG the warp's centre and radius; nE <= nG the indices.
+__device__ __forceinline__ void build_list(const MixedCtx& m, const Tile& T, float4* list, LegList* H, int W,
+                                           const float E[3], float rEh, float rEz, float rE, const float G[3],
+                                           float h0, float dh0, bool lp_is_g, const float Gc[3], float rG, float nE,
+                                           float nG)
+{
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int si = H->si, sj = H->sj;
+    __syncwarp();                                  // readers of the previous list are done
+    // window centres of the block
+    const FlatStart f = lp_is_g ? flat_start32(E, G, nE, nG, h0) : flat_start32(G, E, nG, nE, h0);
+    const float hE = fabsf(E[2] - h0), hG = fabsf(G[2] - h0), hEm = hE - rEz - dh0;
+    const float kappa = __fdividef(nE * hG, nE * hG + nG * hEm);
+    const float D = f.D + rEh;
+    const float move = kappa * (rEh + __fdividef(D * rEz, hEm)) + __fdividef(2.0f * D * dh0, hE + hG);
+    const bool ok = nE <= nG && hEm > 0.75f * hE && f.last <= 0.02f * fminf(m.stepx, m.stepy);
+    const float mx = fmaf(move, m.istepx, 0.06f + m.start_band), my = fmaf(move, m.istepy, 0.06f + m.start_band);
+    const float fx = f.sx * m.istepx, fy = f.sy * m.istepy;
+    const int ilo = __reduce_min_sync(full, min(max(__float2int_rn(fx - mx), 0), m.nx - 1));
+    const int ihi = __reduce_max_sync(full, min(max(__float2int_rn(fx + mx), 0), m.nx - 1));
+    const int jlo = __reduce_min_sync(full, min(max(__float2int_rn(fy - my), 0), m.ny - 1));
+    const int jhi = __reduce_max_sync(full, min(max(__float2int_rn(fy + my), 0), m.ny - 1));
+    const int ca = max(ihi - W, 0), cb = min(ilo + W, m.nx - 1);      // intersection of the windows
+    const int da = max(jhi - W, 0), db = min(jlo + W, m.ny - 1);
+    const int ua = max(ilo - W, 0), ub = min(ihi + W, m.nx - 1);      // union
+    const int va = max(jlo - W, 0), vb = min(jhi + W, m.ny - 1);
+    if (!__all_sync(full, ok) || ca > cb || da > db || ub - ua > 32000 || vb - va > 32000) {
+        if (lane == 0) H->m = -1;
+        __syncwarp();
+        return;
+    }
+    const int nj = vb - va + 1, n = (ub - ua + 1) * nj;
+    const bool in_tile = T.ok && ua >= T.i0 && ub < T.i0 + TI && va >= T.j0 && vb < T.j0 + TJ;
+    auto zat = [&](int i, int j) { return in_tile ? T.s[(j - T.j0) * TI + (i - T.i0)] : zf(m, i, j); };
+    if (!(si >= ca && si <= cb && sj >= da && sj <= db)) {
+        si = (ca + cb) >> 1;
+        sj = (da + db) >> 1;
+    }
+    GapRef g;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        g.E[c] = E[c];
+        g.G[c] = Gc[c];
+    }
+    g.re = __fdividef(nE, nG);
+    g.cE = 2.0f * g.re * rE;
+    g.cG = 2.0f * rG;
+    g.rE2 = 2.0f * rE;
+    g.rG2 = 2.0f * rG;
+    gap_set(g, (float)si * m.stepx, (float)sj * m.stepy, zat(si, sj));
+    const unsigned below = (1u << lane) - 1u;
+    int cnt = 0;
+    bool outside = false;
+#pragma unroll 1
+    for (int attempt = 0; attempt < 2; attempt++) {
+        const float thr = kTieM / nG + 1e-4f + 2e-6f * (g.eS + g.gS) + 5e-7f * m.extent;
+        float best = INFINITY;
+        int bij = 0;
+        cnt = 0;
+        outside = false;
+        int i = ua + lane / nj, j = va + lane % nj;
+#pragma unroll 1
+        for (int base = 0; base < n; base += 32) {
+            const bool in = base + lane < n;
+            bool keep = false;
+            float x = 0.f, y = 0.f, z = 0.f;
+            if (in) {
+                x = (float)i * m.stepx;
+                y = (float)j * m.stepy;
+                z = zat(i, j);
+                float gap;
+                keep = gap_of(g, x, y, z, gap) <= thr;
+                const bool core = i >= ca && i <= cb && j >= da && j <= db;
+                outside |= keep && !core;
+                if (core && gap < best) {
+                    best = gap;
+                    bij = ((i - ua) << 16) | (j - va);
+                }
+            }
+            const unsigned bal = __ballot_sync(full, keep);
+            const int pos = cnt + __popc(bal & below);
+            if (keep && pos < kListCap) list[pos] = list_entry(x, y, z, i - ua, j - va);
+            cnt += __popc(bal);
+            j += 32;
+            while (j > vb) {
+                j -= nj;
+                i++;
+            }
+        }
+        __syncwarp();
+        // the best node inside every window becomes S: the tightest list, and the next
+        // block's first guess
+        const unsigned key = ordered_bits(best), kmin = __reduce_min_sync(full, key);
+        const int w = __shfl_sync(full, bij, __ffs(__ballot_sync(full, key == kmin)) - 1);
+        const int ni = ua + (w >> 16), nj2 = va + (w & 0xffff);
+        const bool same = ni == si && nj2 == sj;
+        si = ni;
+        sj = nj2;
+        if (same || cnt <= 1) break;
+        gap_set(g, (float)si * m.stepx, (float)sj * m.stepy, zat(si, sj));
+        if (cnt <= kListCap) {
+            // list against the better S, in place and in order
+            const float thr2 = kTieM / nG + 1e-4f + 2e-6f * (g.eS + g.gS) + 5e-7f * m.extent;
+            const int c0 = cnt;
+            cnt = 0;
+            outside = false;
+#pragma unroll 1
+            for (int base = 0; base < c0; base += 32) {
+                float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                bool keep = false;
+                if (base + lane < c0) {
+                    q = list[base + lane];
+                    float gap;
+                    keep = gap_of(g, q.x, q.y, q.z, gap) <= thr2;
+                    const int pk = __float_as_int(q.w);
+                    const int i2 = ua + (pk >> 16), j2 = va + (pk & 0xffff);
+                    outside |= keep && !(i2 >= ca && i2 <= cb && j2 >= da && j2 <= db);
+                }
+                const unsigned bal = __ballot_sync(full, keep);
+                if (keep) list[cnt + __popc(bal & below)] = q;
+                cnt += __popc(bal);
+            }
+            break;
+        }
+    }
+    const bool any_out = __any_sync(full, outside);
+    if (lane == 0) {
+        H->m = (cnt >= 1 && cnt <= kListCap) ? cnt : -1;
+        H->mode = any_out ? 0 : kCore;
+        H->i0 = ua;
+        H->j0 = va;
+        H->si = si;
+        H->sj = sj;
+    }
+    __syncwarp();
+}
+
+// Whether the listed node (i, j) is the crossing itself for every (antenna, voxel) of the
+// block: the path's one-sided derivatives along the four edges at the node, which point
+// uphill at (Ec, Gc) by more than they can turn over the block.  With t the edge's tangent
+// the derivative is nE u_E.t + nG u_G.t (u: unit vectors from the endpoints), and u turns by
+// at most 2 r / (2 |N - Ec| - r) over a distance r.  Then each of the four facets has its
+// minimum at the node (the corner test of finish_leg), with a margin far above the FP32
+// rounding of the derivatives.  Nodes on the DEM's border have missing facets: never.
+__device__ __forceinline__ bool node_pinned(const MixedCtx& m, int i, int j, const float E[3], const float G[3], float rE,
+                                            float rG, float nE, float nG)
+{
+    if (i < 1 || j < 1 || i > m.nx - 2 || j > m.ny - 2) return false;
+    const float z = zf(m, i, j);
+    const float sxb = (z - zf(m, i - 1, j)) * m.istepx, sxf = (zf(m, i + 1, j) - z) * m.istepx;
+    const float syb = (z - zf(m, i, j - 1)) * m.istepy, syf = (zf(m, i, j + 1) - z) * m.istepy;
+    const float x = (float)i * m.stepx, y = (float)j * m.stepy;
+    const float ex = x - E[0], ey = y - E[1], ez = z - E[2];
+    const float gx = x - G[0], gy = y - G[1], gz = z - G[2];
+    const float qe = ex * ex + ey * ey + ez * ez, qg = gx * gx + gy * gy + gz * gz;
+    const float se = nE * rsqrtf(qe), sg = nG * rsqrtf(qg);
+    const float Fx = se * ex + sg * gx, Fy = se * ey + sg * gy, Fz = se * ez + sg * gz;
+    const float dE = 2.0f * qe * rsqrtf(qe) - rE, dG = 2.0f * qg * rsqrtf(qg) - rG;
+    if (!(dE > rE && dG > rG)) return false;
+    const float turn = 2.0f * (nE * __fdividef(rE, dE) + nG * __fdividef(rG, dG)) + 1e-5f * (nE + nG);
+    auto tangent = [](float sl) { return sqrtf(1.0f + sl * sl); };
+    return fmaf(Fz, sxf, Fx) > turn * tangent(sxf) && -fmaf(Fz, sxb, Fx) > turn * tangent(sxb) &&
+           fmaf(Fz, syf, Fy) > turn * tangent(syf) && -fmaf(Fz, syb, Fy) > turn * tangent(syb);
+}
+
+// Short lists (kTables): nE |N - E| of every listed node and pulse of the block and
+// nG |N - G| of every node and lane, in FP64.  A solve adds two of them per node and keeps
+// the smallest sum, which is the FP64 solver's ranking value, bit for bit; where that node
+// is pinned the sum is the leg's path and the solve is done.
+struct NodeTables {
+    double E[kTabled][kBlockPulses], G[kTabled][32];
+};
+
+// Smallest sum of pulse q (of the block) and this lane over m listed nodes, and its node.
+__device__ __forceinline__ double table_min(const NodeTables& t, int m, int q, int lane, int& c)
+{
+    double v = __dadd_rn(t.E[0][q], t.G[0][lane]);
+    c = 0;
+#pragma unroll 1
+    for (int k = 1; k < m; k++) {
+        const double u = __dadd_rn(t.E[k][q], t.G[k][lane]);
+        if (u < v) {
+            v = u;
+            c = k;
+        }
+    }
+    return v;
+}
+
+// A solve's ranking of a longer list: the best entry.  Near ties are re-ranked in FP64 with the
+// FP64 solver's arithmetic and order (the list is i-major).
+__device__ __noinline__ int rerank_list(const DemView d, const float4* list, int n, int core, int i0, int j0, int is,
+                                        int js, int W, float ex, float ey, float ez, float gx, float gy, float gz,
+                                        float re, float limit, double Ax, double Ay, double Az, double Bx, double By,
+                                        double Bz, double na, double nb, int best_k)
+{
+    const double A[3] = {Ax, Ay, Az}, B[3] = {Bx, By, Bz};
+    double best = INFINITY;
+    for (int k = 0; k < n; k++) {
+        const float4 q = list[k];
+        const int pk = __float_as_int(q.w), i = i0 + (pk >> 16), j = j0 + (pk & 0xffff);
+        if (!core && (abs(i - is) > W || abs(j - js) > W)) continue;
+        const float dxe = q.x - ex, dye = q.y - ey, dze = q.z - ez;
+        const float dxg = q.x - gx, dyg = q.y - gy, dzg = q.z - gz;
+        const float qe = dxe * dxe + dye * dye + dze * dze;
+        const float qg = dxg * dxg + dyg * dyg + dzg * dzg;
+        if (re * sqrtf(qe) + sqrtf(qg) <= limit) {
+            const double L = node_l64(d, i, j, A, B, na, nb);
+            if (L < best) {
+                best = L;
+                best_k = k;
+            }
+        }
+    }
+    return best_k;
+}
+
+__device__ __forceinline__ int2 rank_list(const DemView& d, const MixedCtx& m, const float4* list, const LegList& H,
+                                          const Leg& l, const VoxelStart& vs, int W)
+{
+    int c = 0;
+    if (H.m > 1) {
+        int2 st = make_int2(0, 0);
+        if (!(H.mode & kCore)) st = start_node(d, m, l, vs);
+        const float* E = l.E32;
+        const float* G = l.G32;
+        const float re = __fdividef(l.nE, l.nG);
+        const float tie = kTieM / l.nG;
+        float v1 = INFINITY, v2 = INFINITY;
+#pragma unroll 1
+        for (int k = 0; k < H.m; k++) {
+            const float4 q = list[k];
+            const float dye = q.y - E[1], dxe = q.x - E[0], dze = q.z - E[2];
+            const float qe = fmaf(dze, dze, fmaf(dxe, dxe, dye * dye));
+            const float dxg = q.x - G[0], dyg = q.y - G[1], dzg = q.z - G[2];
+            const float qg = fmaf(dzg, dzg, fmaf(dxg, dxg, dyg * dyg));
+            float L = fmaf(qg, rsqrtf(qg), re * (qe * rsqrtf(qe)));
+            if (!(H.mode & kCore)) {
+                const int pk = __float_as_int(q.w);
+                if (abs(H.i0 + (pk >> 16) - st.x) > W || abs(H.j0 + (pk & 0xffff) - st.y) > W) L = INFINITY;
+            }
+            v2 = fminf(v2, fmaxf(v1, L));
+            const bool p = L < v1;
+            v1 = p ? L : v1;
+            c = p ? k : c;
+        }
+        if (!(v2 - v1 >= tie))
+            c = rerank_list(d, list, H.m, H.mode & kCore, H.i0, H.j0, st.x, st.y, W, E[0], E[1], E[2], G[0], G[1], G[2], re,
+                            v1 + tie, l.E[0], l.E[1], l.E[2], l.G[0], l.G[1], l.G[2], l.nE64, l.nG64, c);
+    }
+    const int pk = __float_as_int(list[c].w);
+    return make_int2(H.i0 + (pk >> 16), H.j0 + (pk & 0xffff));
+}
+
+// From the best node (bi, bj) to the crossing: FP32 polish of the facets around it, FP64
+// final step.  Returns the FP64 optical path; X (optional): the crossing.
+__device__ __forceinline__ double finish_leg(const DemView& d, const MixedCtx& m, const Tile& T, const Leg& l, int bi,
+                                             int bj, double* X = nullptr)
+{
+    const float* A32 = l.E32;
+    const float* B32 = l.G32;
+    const float na = l.nE, nb = l.nG;
+    // polish the facets around the best node (FP32); heights from the DEM tile when the
     //    node's 3 x 3 neighbourhood lies in it.  The nine heights are loaded once (indices
     //    clamped to the DEM; a facet that would need a clamped one is not polished), and the
     //    path's gradient at the node is formed once: with G = na (N - A)/|N - A| +
@@ -828,8 +1071,10 @@ __device__ __forceinline__ double solve_mixed(const DemView& d, const MixedCtx& 
             bool moved = false;
 #pragma unroll 1
             for (int it = 0; it < kPolishIters; it++) {
+                const float u0 = u, v0 = v;
                 if (!facet_step32(F, A32, B32, na, nb, u, v)) break;
                 moved = true;
+                if (fabsf(u - u0) + fabsf(v - v0) < kConverged) break;
             }
             // a facet whose corner is already its minimum keeps the best node's path
             if (moved) L = facet_eval32(F, A32, B32, na, nb, u, v);
@@ -842,9 +1087,7 @@ __device__ __forceinline__ double solve_mixed(const DemView& d, const MixedCtx& 
             bfj = fj;
         }
     }
-    // 4. FP64 final step
-    return final_step64(d, bfi, bfj, A, B, (double)na, (double)nb, (double)bu, (double)bv, dA, dB, X, m.idx64,
-                        m.idy64);
+    return final_step64(d, bfi, bfj, l.E, l.G, l.nE64, l.nG64, (double)bu, (double)bv, X, m.idx64, m.idy64);
 }
 
 // ------------------------------- TMA tile staging -----------------------------------
@@ -913,125 +1156,337 @@ __device__ __forceinline__ MixedCtx req_ctx(const MixedReq& r)
     m.idx64 = r.idx64;
     m.idy64 = r.idy64;
     m.start_band = r.start_band;
-    m.prune = !r.exhaustive;
-    m.zmin = r.zmin;
+    m.lists = !r.exhaustive;
+    m.extent = fmaxf((float)m.nx * m.stepx, (float)m.ny * m.stepy);
     return m;
 }
+
+// The voxel at index k of a request's range: ranges of whole z-planes in the compact order
+// (compact_voxel), others in the reference's flat order (z -> x -> y).
+__device__ __forceinline__ int3 voxel_at(const BpArgs& a, int compact, int64_t k)
+{
+    int x, y, z;
+    if (compact) {
+        const int64_t plane = (int64_t)a.nx * a.ny;
+        compact_voxel(a.nx, a.ny, (int)(a.v_count / plane), k, x, y, z);
+        z += (int)(a.v_begin / plane);
+    } else {
+        const int64_t v = a.v_begin + k;
+        x = (int)((v / a.ny) % a.nx);
+        y = (int)(v % a.ny);
+        z = (int)(v / ((int64_t)a.nx * a.ny));
+    }
+    return make_int3(x, y, z);
+}
+
+__device__ __forceinline__ float warp_max(float v)   // v >= 0
+{
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+
+// Shared memory of one warp.  A pulse block has lists for both legs or none: the lists (or
+// their tables) and the block's paths share their place with the table of the scans that
+// rank every node, which take one pulse at a time and keep its paths in the last row.
+template <int WT> struct WarpShared {
+    union {
+        struct {
+            union {
+                float4 list[2][kListCap];
+                NodeTables tab[2];           // takes the place of a short list's entries
+            };
+            double path[kBlockPulses][32];   // per pulse and lane: the paths of the legs solved one by one
+        } b;
+        float2 table[TableRows<WT>::v * TBJ];
+    } u;
+    double ref_L[kBlockPulses];              // the block's anchors
+    float4 anchor[kBlockPulses];             // fast-time bin fraction, reduced phase, FP16 scale, bin (int)
+    LegList h[2];
+};
+static_assert(sizeof(NodeTables) == sizeof(float4) * kListCap, "one leg's tables take its list's place");
+static_assert(sizeof(float2) * TableRows<12>::v * TBJ + 32 * sizeof(double) <= sizeof(float4) * 2 * kListCap +
+                                                                               32 * sizeof(double) * kBlockPulses,
+              "the last row of paths lies beyond the table");
+
+// Largest antenna movement of a pulse block, from its first pulse: re * distance / |E - G|
+// stays below kBlockSlope (it sets the lists' slack and with it their length), at most
+// kBlockPulses pulses.
+constexpr float kBlockSlope = 0.0125f;
 
 // One voxel of a request over pulses [p0, p1) (k: index in the request's voxel range;
 // k >= v_count repeats the last voxel without storing it, so whole warps stay active).
 // The sum goes to dst at the voxel's image index.
 template <int WT, bool CH>
-__device__ __forceinline__ void voxel_mixed(const BpArgs& a, const MixedCtx& m, const Tile& T, float2* table_buf,
-                                            bool fp16, int64_t kk, int p0, int p1,
+__device__ __forceinline__ void voxel_mixed(const BpArgs& a, const MixedCtx& m, const Tile& T,
+                                            WarpShared<WT>* ws, bool fp16, int compact, int64_t kk, int p0, int p1,
                                             double2* __restrict__ dst)
 {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
     const int np = CH ? p1 : a.np;
     const float k_bin = (float)(a.fs_eff / a.c);
     const float k_phase = (float)(2.0 * 3.14159265358979323846 / a.lambda);
     const float n1f = (float)a.n1, n2f = (float)a.n2;
     const int64_t nr = a.nr;
-    const int64_t k = kk < a.v_count ? kk : a.v_count - 1;
-    const int64_t v = a.v_begin + k;
-    const int yi = (int)(v % a.ny);
-    const int xi = (int)((v / a.ny) % a.nx);
-    const int zi = (int)(v / ((int64_t)a.nx * a.ny));
-    const double P[3] = {__ldg(a.gx + xi), __ldg(a.gy + yi), __ldg(a.gz + zi)};
+    const int3 vx = voxel_at(a, compact, kk < a.v_count ? kk : a.v_count - 1);
+    const double P[3] = {__ldg(a.gx + vx.x), __ldg(a.gy + vx.y), __ldg(a.gz + vx.z)};
     const float P32[3] = {(float)(P[0] - m.ox), (float)(P[1] - m.oy), (float)P[2]};
     const VoxelStart vs{height32(m, P32[0], P32[1]), dem_elevation(a.dem, P[0], P[1])};
-    float accr = 0.f, acci = 0.f, cmpr = 0.f, cmpi = 0.f;
-    int seed0 = -1, seed1 = -1;     // each leg's node at the previous pulse (pruning hint)
-    for (int i = CH ? p0 : 0; i < np; i++) {
-        const double Tx[3] = {__ldg(a.tx + 3 * i), __ldg(a.tx + 3 * i + 1), __ldg(a.tx + 3 * i + 2)};
-        const double Rx[3] = {__ldg(a.rx + 3 * i), __ldg(a.rx + 3 * i + 1), __ldg(a.rx + 3 * i + 2)};
-        const float T32[3] = {(float)(Tx[0] - m.ox), (float)(Tx[1] - m.oy), (float)Tx[2]};
-        const float R32[3] = {(float)(Rx[0] - m.ox), (float)(Rx[1] - m.oy), (float)Rx[2]};
-        // per-pulse legs: n1*r1Tx + n2*r2Tx (Tx -> voxel) + n2*r2Rx + n1*r1Rx (voxel -> Rx);
-        // one solver body serves both legs
-        double L = 0.0;
-#pragma unroll 1
-        for (int leg = 0; leg < 2; leg++) {
-            // endpoints selected element-wise so they stay in registers
-            const double A[3] = {leg ? P[0] : Tx[0], leg ? P[1] : Tx[1], leg ? P[2] : Tx[2]};
-            const double B[3] = {leg ? Rx[0] : P[0], leg ? Rx[1] : P[1], leg ? Rx[2] : P[2]};
-            const float A32[3] = {leg ? P32[0] : T32[0], leg ? P32[1] : T32[1], leg ? P32[2] : T32[2]};
-            const float B32[3] = {leg ? R32[0] : P32[0], leg ? R32[1] : P32[1], leg ? R32[2] : P32[2]};
-            double dA, dB;
-            int seed = leg ? seed1 : seed0;
-            L += solve_mixed<WT, true>(a.dem, m, T, table_buf, A, B, A32, B32, leg ? n2f : n1f,
-                                       leg ? n1f : n2f, leg == 0, a.W, vs, seed, dA, dB);
-            seed1 = leg ? seed : seed1;
-            seed0 = leg ? seed0 : seed;
+    // centre and radius of the warp's voxels
+    float Gc[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        float lo = P32[c], hi = P32[c];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(full, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(full, hi, o));
         }
-        const float dL = (float)(L - __ldg(a.ref_L + i));
-        // fast-time bin: integer anchor + FP32 offset
-        const float t = __ldg(a.ref_bin_f + i) + dL * k_bin;
-        const float fl = floorf(t);
-        const int64_t lo = (int64_t)__ldg(a.ref_bin_i + i) + (int64_t)fl;
-        const float q = t - fl;
-        const bool exact = (q == 0.0f);
-        if (lo >= 0 && (lo < nr - 1 || (lo == nr - 1 && exact))) {
-            float s0r, s0i, s1r = 0.f, s1i = 0.f;
-            const int64_t base = (int64_t)i * nr + lo;
-            if (fp16) {
-                const float sc = __ldg(a.scale16 + i);
-                float2 f0 = __half22float2(a.rc16[base]);
-                s0r = f0.x * sc;
-                s0i = f0.y * sc;
-                if (!exact) {
-                    float2 f1 = __half22float2(a.rc16[base + 1]);
-                    s1r = f1.x * sc;
-                    s1i = f1.y * sc;
+        Gc[c] = 0.5f * (lo + hi);
+    }
+    float rG;
+    {
+        const float dx = P32[0] - Gc[0], dy = P32[1] - Gc[1], dz = P32[2] - Gc[2];
+        rG = warp_max(sqrtf(dx * dx + dy * dy + dz * dz)) * 1.0001f + 1e-5f;
+    }
+    if (lane < 2) ws->h[lane].si = ws->h[lane].sj = -1;
+    __syncwarp();
+    float accr = 0.f, acci = 0.f, cmpr = 0.f, cmpi = 0.f;
+    int block_end;
+    for (int i = CH ? p0 : 0; i < np; i = block_end) {
+        {
+            // the next pulse block: as many pulses as keep both antennas close together
+            const int pl = min(i + lane, np - 1);
+            float e[2][3], far = 0.f;
+#pragma unroll
+            for (int leg = 0; leg < 2; leg++) {
+                const double* tr = leg ? a.rx : a.tx;
+                e[leg][0] = (float)(__ldg(tr + 3 * pl) - m.ox);
+                e[leg][1] = (float)(__ldg(tr + 3 * pl + 1) - m.oy);
+                e[leg][2] = (float)__ldg(tr + 3 * pl + 2);
+                const float dx = e[leg][0] - __shfl_sync(full, e[leg][0], 0);
+                const float dy = e[leg][1] - __shfl_sync(full, e[leg][1], 0);
+                const float dz = e[leg][2] - __shfl_sync(full, e[leg][2], 0);
+                const float gx = e[leg][0] - Gc[0], gy = e[leg][1] - Gc[1], gz = e[leg][2] - Gc[2];
+                // movement against the antenna's distance from the voxels
+                far = fmaxf(far, __fdividef(dx * dx + dy * dy + dz * dz, gx * gx + gy * gy + gz * gz));
+            }
+            const float re = fminf(__fdividef(n1f, n2f), 1.0f);
+            const unsigned stop = __ballot_sync(full, !(far * re * re <= 4.0f * kBlockSlope * kBlockSlope) && lane > 0);
+            const int n = min(min(stop ? __ffs(stop) - 1 : 32, kBlockPulses), np - i);
+            block_end = i + n;
+            if (lane < n) {
+                ws->ref_L[lane] = __ldg(a.ref_L + pl);
+                ws->anchor[lane] = make_float4(__ldg(a.ref_bin_f + pl), __ldg(a.ref_phase + pl),
+                                               fp16 ? __ldg(a.scale16 + pl) : 1.0f,
+                                               __int_as_float(__ldg(a.ref_bin_i + pl)));
+            }
+#pragma unroll 1
+            for (int leg = 0; leg < 2; leg++) {
+                const float x = leg ? e[1][0] : e[0][0], y = leg ? e[1][1] : e[0][1], z = leg ? e[1][2] : e[0][2];
+                const int mid = (n - 1) >> 1;
+                const float E[3] = {__shfl_sync(full, x, mid), __shfl_sync(full, y, mid), __shfl_sync(full, z, mid)};
+                const float dx = x - E[0], dy = y - E[1], dz = fabsf(z - E[2]);
+                const bool in = lane < n;
+                const float h2 = dx * dx + dy * dy;
+                const float rEh = warp_max(in ? sqrtf(h2) : 0.f) * 1.0001f + 1e-5f;
+                const float rEz = warp_max(in ? dz : 0.f) * 1.0001f + 1e-5f;
+                const float rE = warp_max(in ? sqrtf(h2 + dz * dz) : 0.f) * 1.0001f + 1e-5f;
+                // start height: under the voxel, or under the antenna where the antenna is
+                // the path's lower endpoint (equal indices, second leg)
+                const bool lp_is_g = lower_is_voxel(n1f, n2f, leg == 0);
+                float h0 = vs.h32, dh0 = 0.f;
+                if (!lp_is_g) {
+                    const float h = height32(m, x, y);
+                    h0 = __shfl_sync(full, h, mid);
+                    dh0 = warp_max(in ? fabsf(h - h0) : 0.f) * 1.0001f + 1e-5f;
                 }
-            } else {
-                float2 f0 = __ldg(a.rc32 + base);
-                s0r = f0.x;
-                s0i = f0.y;
-                if (!exact) {
-                    float2 f1 = __ldg(a.rc32 + base + 1);
-                    s1r = f1.x;
-                    s1i = f1.y;
+                if (m.lists) {
+                    build_list(m, T, ws->u.b.list[leg], &ws->h[leg], a.W, E, rEh, rEz, rE, P32, h0, dh0, lp_is_g, Gc, rG,
+                               n1f, n2f);
+                    const int cnt = ws->h[leg].m;
+                    if (cnt > 0 && cnt <= kTabled) {
+                        LegList* H = &ws->h[leg];
+                        const float4 q = ws->u.b.list[leg][min(lane, cnt - 1)];     // lane k: node k
+                        const int pk = __float_as_int(q.w);
+                        const int ni = H->i0 + (pk >> 16), nj = H->j0 + (pk & 0xffff);
+                        const bool pin = node_pinned(m, ni, nj, E, Gc, rE, rG, n1f, n2f);
+                        const unsigned pinned = __ballot_sync(full, pin && lane < cnt);
+                        if (lane < cnt) H->node[lane] = make_int2(ni, nj);
+                        if (lane == 0) {
+                            H->mode |= kTables;
+                            H->pinned = (int)pinned;
+                        }
+                        const double* tr = (leg ? a.rx : a.tx) + 3 * pl;
+                        const double El[3] = {__ldg(tr), __ldg(tr + 1), __ldg(tr + 2)};
+                        __syncwarp();                    // the entries are read: their place is free
+#pragma unroll 1
+                        for (int k = 0; k < cnt; k++) {
+                            const int2 nd = H->node[k];
+                            const double x = __ldg(a.dem.xv + nd.x), y = __ldg(a.dem.yv + nd.y);
+                            const double z = __ldg(a.dem.z + (int64_t)nd.y * a.dem.nx + nd.x);
+                            const double e = __dmul_rn(a.n1, leg_len64(x, y, z, El));
+                            if (lane < kBlockPulses) ws->u.b.tab[leg].E[k][lane] = e;
+                            ws->u.b.tab[leg].G[k][lane] = __dmul_rn(a.n2, leg_len64(x, y, z, P));
+                        }
+                    }
                 }
             }
-            const float w0 = 1.0f - q;
-            const float vr = exact ? s0r : fmaf(w0, s0r, q * s1r);
-            const float vi = exact ? s0i : fmaf(w0, s0i, q * s1i);
-            // carrier phase: FP64-reduced anchor + FP32 offset, reduced again to [-pi, pi]
-            float ph = __ldg(a.ref_phase + i) + dL * k_phase;
-            const float kr = rintf(ph * 0.15915494309189535f);
-            ph = fmaf(-kr, 6.28318548202514648f, ph);
-            ph = fmaf(-kr, -1.7484555e-7f, ph);
-            float sn, cs;
-            __sincosf(ph, &sn, &cs);
-            const float cr = vr * cs - vi * sn;
-            const float ci = vr * sn + vi * cs;
-            // Kahan-compensated sums
-            float y = cr - cmpr;
-            float tt = accr + y;
-            cmpr = (tt - accr) - y;
-            accr = tt;
-            y = ci - cmpi;
-            tt = acci + y;
-            cmpi = (tt - acci) - y;
-            acci = tt;
+            __syncwarp();
+            if (!m.lists || ws->h[0].m < 0 || ws->h[1].m < 0) {
+                __syncwarp();
+                if (lane < 2) ws->h[lane].m = -1;
+            }
+            __syncwarp();
+        }
+        const int hm0 = ws->h[0].m, hm1 = ws->h[1].m;
+        // legs whose listed nodes are all pinned: the paths come from the tables alone
+        auto all_pinned = [&](int leg, int hm) {
+            return hm > 0 && ws->h[leg].mode == (kCore | kTables) && ws->h[leg].pinned == (1 << hm) - 1;
+        };
+        const int m0 = all_pinned(0, hm0) ? hm0 : 0, m1 = all_pinned(1, hm1) ? hm1 : 0;
+        const int step = hm0 < 0 ? 1 : block_end - i;      // no lists: one pulse at a time
+        for (int b = i; b < block_end; b += step) {
+            double* path = hm0 < 0 ? ws->u.b.path[kBlockPulses - 1] : ws->u.b.path[0];
+            // per-pulse legs: n1*r1Tx + n2*r2Tx (Tx -> voxel) + n2*r2Rx + n1*r1Rx (voxel -> Rx);
+            // the legs to solve, one after the other over the block's pulses
+#pragma unroll 1
+            for (int leg = m0 ? 1 : 0; leg < (m1 ? 1 : 2); leg++) {
+                const LegList* H = &ws->h[leg];
+                const int hm = H->m, mode = H->mode;
+                Leg l;
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    l.G[c] = P[c];
+                    l.G32[c] = P32[c];
+                }
+                l.nE = n1f;
+                l.nG = n2f;
+                l.nE64 = a.n1;
+                l.nG64 = a.n2;
+                l.g_lower = lower_is_voxel(n1f, n2f, leg == 0);
+#pragma unroll 1
+                for (int p = b; p < b + step; p++) {
+                    double L = 0.0;
+                    int2 node = make_int2(0, 0);
+                    bool solved = false;
+                    if (hm > 0 && mode == (kCore | kTables)) {
+                        int c;
+                        L = table_min(ws->u.b.tab[leg], hm, p - i, lane, c);
+                        solved = (H->pinned >> c) & 1;
+                        node = H->node[c];
+                    }
+                    if (!solved) {
+                        const double* tr = (leg ? a.rx : a.tx) + 3 * p;
+#pragma unroll
+                        for (int c = 0; c < 3; c++) l.E[c] = __ldg(tr + c);
+                        l.E32[0] = (float)(l.E[0] - m.ox);
+                        l.E32[1] = (float)(l.E[1] - m.oy);
+                        l.E32[2] = (float)l.E[2];
+                        if (hm < 0) {
+                            const Leg lc = l;
+                            node = scan_warp<WT>(a.dem, m, T, ws->u.table, lc, vs, a.W);
+                        } else if (!(mode & kTables)) {
+                            node = rank_list(a.dem, m, ws->u.b.list[leg], *H, l, vs, a.W);
+                        } else if (!(mode & kCore)) {
+                            // a listed node may lie outside this solve's window
+                            const int2 st = start_node(a.dem, m, l, vs);
+                            const NodeTables* t = &ws->u.b.tab[leg];
+                            double v = INFINITY;
+                            int c = 0;
+#pragma unroll 1
+                            for (int k = 0; k < hm; k++) {
+                                const int2 nd = H->node[k];
+                                const double u = __dadd_rn(t->E[k][p - i], t->G[k][lane]);
+                                if (u < v && abs(nd.x - st.x) <= a.W && abs(nd.y - st.y) <= a.W) {
+                                    v = u;
+                                    c = k;
+                                }
+                            }
+                            node = H->node[c];
+                        }
+                        L = finish_leg(a.dem, m, T, l, node.x, node.y);
+                    }
+                    double* d = path + (p - b) * 32 + lane;
+                    *d = (leg && !m0) ? __dadd_rn(*d, L) : L;
+                }
+            }
+            // delays, gathers and sums of the block's pulses
+#pragma unroll 1
+            for (int p = b; p < b + step; p++) {
+                const int q0 = p - i;
+                double L = (m0 && m1) ? 0.0 : path[(p - b) * 32 + lane];
+                int c;
+                if (m0) L = __dadd_rn(L, table_min(ws->u.b.tab[0], m0, q0, lane, c));
+                if (m1) L = __dadd_rn(L, table_min(ws->u.b.tab[1], m1, q0, lane, c));
+                const float dL = (float)(L - ws->ref_L[q0]);
+                const float4 an = ws->anchor[q0];
+                // fast-time bin: integer anchor + FP32 offset
+                const float t = an.x + dL * k_bin;
+                const float fl = floorf(t);
+                const int64_t lo = (int64_t)__float_as_int(an.w) + (int)fl;
+                const float q = t - fl;
+                const bool exact = (q == 0.0f);
+                // |fl| < 2^31 also drops a path that is not a number
+                if (fabsf(fl) < 2.0e9f && lo >= 0 && (lo < nr - 1 || (lo == nr - 1 && exact))) {
+                    float s0r, s0i, s1r = 0.f, s1i = 0.f;
+                    const int64_t base = (int64_t)p * nr + lo;
+                    if (fp16) {
+                        float2 f0 = __half22float2(a.rc16[base]);
+                        s0r = f0.x * an.z;
+                        s0i = f0.y * an.z;
+                        if (!exact) {
+                            float2 f1 = __half22float2(a.rc16[base + 1]);
+                            s1r = f1.x * an.z;
+                            s1i = f1.y * an.z;
+                        }
+                    } else {
+                        float2 f0 = __ldg(a.rc32 + base);
+                        s0r = f0.x;
+                        s0i = f0.y;
+                        if (!exact) {
+                            float2 f1 = __ldg(a.rc32 + base + 1);
+                            s1r = f1.x;
+                            s1i = f1.y;
+                        }
+                    }
+                    const float w0 = 1.0f - q;
+                    const float vr = exact ? s0r : fmaf(w0, s0r, q * s1r);
+                    const float vi = exact ? s0i : fmaf(w0, s0i, q * s1i);
+                    // carrier phase: FP64-reduced anchor + FP32 offset, reduced again to [-pi, pi]
+                    float ph = an.y + dL * k_phase;
+                    const float kr = rintf(ph * 0.15915494309189535f);
+                    ph = fmaf(-kr, 6.28318548202514648f, ph);
+                    ph = fmaf(-kr, -1.7484555e-7f, ph);
+                    float sn, cs;
+                    __sincosf(ph, &sn, &cs);
+                    const float cr = vr * cs - vi * sn;
+                    const float ci = vr * sn + vi * cs;
+                    // Kahan-compensated sums
+                    float y = cr - cmpr;
+                    float tt = accr + y;
+                    cmpr = (tt - accr) - y;
+                    accr = tt;
+                    y = ci - cmpi;
+                    tt = acci + y;
+                    cmpi = (tt - acci) - y;
+                    acci = tt;
+                }
+            }
         }
     }
     if (kk < a.v_count)
-        (CH ? dst : a.out)[((int64_t)xi * a.ny + yi) * a.nz + zi] =
+        (CH ? dst : a.out)[((int64_t)vx.x * a.ny + vx.y) * a.nz + vx.z] =
             make_double2((double)accr - (double)cmpr, (double)acci - (double)cmpi);
 }
 
 // The last of a tile's pulse chunks to finish adds the chunks' sums, in chunk order, into
 // the image (partial sums of the other CTAs are read from L2).
-__device__ __forceinline__ void reduce_chunks(const BpArgs& a, const double2* __restrict__ partial, int K,
+__device__ __forceinline__ void reduce_chunks(const BpArgs& a, const double2* __restrict__ partial, int compact, int K,
                                               int64_t kk)
 {
     if (kk >= a.v_count) return;
-    const int64_t v = a.v_begin + kk;
-    const int yi = (int)(v % a.ny);
-    const int xi = (int)((v / a.ny) % a.nx);
-    const int zi = (int)(v / ((int64_t)a.nx * a.ny));
-    const int64_t idx = ((int64_t)xi * a.ny + yi) * a.nz + zi;
+    const int3 vx = voxel_at(a, compact, kk);
+    const int64_t idx = ((int64_t)vx.x * a.ny + vx.y) * a.nz + vx.z;
     const int64_t nvox = (int64_t)a.nx * a.ny * a.nz;
     double sr = 0.0, si = 0.0;
     for (int c = 0; c < K; c++) {
@@ -1056,7 +1511,8 @@ __device__ __forceinline__ void reduce_chunks(const BpArgs& a, const double2* __
 // 25 x 25 scan builds 30-row warp tables every pulse and reads them from the tile faster
 // than through L1.  For 7 x 7 and 13 x 13 scans the tile's bookkeeping costs registers
 // (twice the spills) and its 17 KB per CTA shrinks L1, and the kernel runs faster with the
-// heights read from global memory -- the same FP32 values, so the same image.
+// heights read from global memory -- the same FP32 values, so the same image.  (Measured with
+// the scans that rank every node, which the exhaustive flag still runs.)
 template <int WT> struct StagesTile { static constexpr bool v = WT == 0 || WT >= 12; };
 
 template <int WT, bool CH>
@@ -1064,11 +1520,11 @@ __global__ void __launch_bounds__(128, 4) k_bp_mixed(MixedBatch b)
 {
     constexpr bool kTile = StagesTile<WT>::v;
     __shared__ alignas(128) float tile_s[kTile ? TI * TJ : 32];
-    __shared__ alignas(16) float2 air_s[4][TableRows<WT>::v * TBJ];   // one (z, E-leg) table per warp
+    __shared__ alignas(16) WarpShared<WT> warp_s[4];
     __shared__ alignas(8) uint64_t mbar;
     __shared__ int2 work;
     __shared__ int last_chunk;
-    float2* table_buf = air_s[threadIdx.x >> 5];
+    WarpShared<WT>* ws = &warp_s[threadIdx.x >> 5];
     const int ntiles = b.ntiles_dev ? *b.ntiles_dev : b.ntiles;
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar)) : "memory");
@@ -1096,11 +1552,10 @@ __global__ void __launch_bounds__(128, 4) k_bp_mixed(MixedBatch b)
         Tile T{tile_s, 0, 0, false};
         if (kTile && R.use_tile && !copy_pending) {
             // DEM tile centred on this work item's voxels plus the mean crossing offset
-            const int64_t v0 = a.v_begin + (int64_t)tile * 128;
-            const int64_t vl = min(v0 + 128, a.v_begin + a.v_count) - 1;
-            const int64_t vm = (v0 + vl) / 2;
-            const double cx = __ldg(a.gx + (int)((vm / a.ny) % a.nx)) + R.off_x;
-            const double cy = __ldg(a.gy + (int)(vm % a.ny)) + R.off_y;
+            const int64_t k0 = (int64_t)tile * 128;
+            const int3 vm = voxel_at(a, R.compact, (k0 + min(k0 + 128, a.v_count) - 1) / 2);
+            const double cx = __ldg(a.gx + vm.x) + R.off_x;
+            const double cy = __ldg(a.gy + vm.y) + R.off_y;
             const int ci = (int)floor((cx - m.ox) / m.stepx), cj = (int)floor((cy - m.oy) / m.stepy);
             T.i0 = ((ci - TI / 2) >> 2) << 2;      // TMA: x offset a multiple of 4 floats (16 B)
             T.j0 = cj - TJ / 2;
@@ -1112,13 +1567,13 @@ __global__ void __launch_bounds__(128, 4) k_bp_mixed(MixedBatch b)
             copy_pending = __syncthreads_or(threadIdx.x == 0 && !seen);
         }
         if constexpr (!CH) {
-            voxel_mixed<WT, false>(a, m, T, table_buf, R.fp16 != 0, (int64_t)w.y * 128 + threadIdx.x, 0, 0,
-                                   nullptr);
+            voxel_mixed<WT, false>(a, m, T, ws, R.fp16 != 0, R.compact, (int64_t)w.y * 128 + threadIdx.x, 0,
+                                   0, nullptr);
         } else {
             const int p0 = (int)((int64_t)chunk * a.np / K), p1 = (int)((int64_t)(chunk + 1) * a.np / K);
             double2* dst = K == 1 ? a.out : b.chunks[w.x].partial + chunk * ((int64_t)a.nx * a.ny * a.nz);
-            voxel_mixed<WT, true>(a, m, T, table_buf, R.fp16 != 0, (int64_t)tile * 128 + threadIdx.x, p0, p1,
-                                  dst);
+            voxel_mixed<WT, true>(a, m, T, ws, R.fp16 != 0, R.compact, (int64_t)tile * 128 + threadIdx.x,
+                                  p0, p1, dst);
             // the work item again from shared memory, so none of it stays live over the pulses
             const volatile int* wv = reinterpret_cast<volatile int*>(&work);
             const int2 w2 = make_int2(wv[0], wv[1]);
@@ -1131,7 +1586,8 @@ __global__ void __launch_bounds__(128, 4) k_bp_mixed(MixedBatch b)
                 __syncthreads();
                 if (last_chunk) {
                     __threadfence();
-                    reduce_chunks(b.reqs[w2.x].a, C.partial, C.nchunk, (int64_t)tile2 * 128 + threadIdx.x);
+                    reduce_chunks(b.reqs[w2.x].a, C.partial, b.reqs[w2.x].compact, C.nchunk,
+                                  (int64_t)tile2 * 128 + threadIdx.x);
                 }
             }
         }
@@ -1155,26 +1611,35 @@ static MixedCtx mixed_ctx(const DemView& d, int pitch)
     m.idx64 = 1.0 / d.stepx;
     m.idy64 = 1.0 / d.stepy;
     m.start_band = mixed_start_band(d);
-    m.prune = 0;
-    m.zmin = -INFINITY;
+    m.lists = 0;
+    m.extent = 0.0f;
     return m;
 }
 
 // Crossing points of the mixed solver (FP32 scan and polish, FP64 final step) for n
 // (start, end) pairs: the data behind the mixed form's crossing-point error.
 __global__ void k_refraction_mixed(DemView d, MixedCtx m, const double* __restrict__ p1, const double* __restrict__ p2,
-                                   int64_t n, float na, float nb, int W, double* __restrict__ out)
+                                   int64_t n, double na, double nb, int W, double* __restrict__ out)
 {
     const Tile T{nullptr, 0, 0, false};
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
-        const double A[3] = {p1[3 * k], p1[3 * k + 1], p1[3 * k + 2]};
-        const double B[3] = {p2[3 * k], p2[3 * k + 1], p2[3 * k + 2]};
-        const float A32[3] = {(float)(A[0] - m.ox), (float)(A[1] - m.oy), (float)A[2]};
-        const float B32[3] = {(float)(B[0] - m.ox), (float)(B[1] - m.oy), (float)B[2]};
-        double dA, dB, X[3];
-        const VoxelStart vs{height32(m, B32[0], B32[1]), dem_elevation(d, B[0], B[1])};
-        int seed = -1;
-        solve_mixed<0, false>(d, m, T, nullptr, A, B, A32, B32, na, nb, true, W, vs, seed, dA, dB, X);
+        Leg l;
+        for (int c = 0; c < 3; c++) {
+            const double o = c == 0 ? m.ox : (c == 1 ? m.oy : 0.0);
+            l.E[c] = p1[3 * k + c];
+            l.G[c] = p2[3 * k + c];
+            l.E32[c] = (float)(l.E[c] - o);
+            l.G32[c] = (float)(l.G[c] - o);
+        }
+        l.nE = (float)na;
+        l.nG = (float)nb;
+        l.nE64 = na;
+        l.nG64 = nb;
+        l.g_lower = lower_is_voxel(l.nE, l.nG, true);
+        double X[3];
+        const VoxelStart vs{height32(m, l.G32[0], l.G32[1]), dem_elevation(d, l.G[0], l.G[1])};
+        const int2 node = scan_lane(d, m, T, l, vs, W);
+        finish_leg(d, m, T, l, node.x, node.y, X);
         out[3 * k] = X[0];
         out[3 * k + 1] = X[1];
         out[3 * k + 2] = X[2];
@@ -1186,7 +1651,7 @@ cudaError_t launch_refraction_mixed(const DemView& d, int pitch, const double* p
 {
     int64_t b = (n + 127) / 128;
     int blocks = (int)(b < 1 ? 1 : (b > 148 * 64 ? 148 * 64 : b));
-    k_refraction_mixed<<<blocks, 128, 0, st>>>(d, mixed_ctx(d, pitch), p1, p2, n, (float)n1, (float)n2, W, out);
+    k_refraction_mixed<<<blocks, 128, 0, st>>>(d, mixed_ctx(d, pitch), p1, p2, n, n1, n2, W, out);
     return cudaGetLastError();
 }
 
@@ -1222,14 +1687,13 @@ static void mixed_setup_device()
 
 int mixed_chunks(int64_t voxels, int pulses)
 {
-    constexpr int kMinChunkPulses = 128;   // below this a chunk's fixed cost (DEM tile, start heights) shows
+    constexpr int kMinChunkPulses = 32;    // below this a chunk's fixed cost (start heights, first block) shows
+    constexpr int64_t kItemsPerCta = 4;    // work items per resident CTA that even out their unequal costs
     const int64_t tiles = (voxels + 127) / 128;
-    const int64_t ctas = mixed_grid_ctas();
-    if (tiles <= 0 || pulses < 2 * kMinChunkPulses || tiles * 2 > ctas) return 1;
-    int64_t k = ctas / tiles;
-    if (k > 8) k = 8;
-    if (k > pulses / kMinChunkPulses) k = pulses / kMinChunkPulses;
-    return (int)k;
+    const int64_t want = std::min<int64_t>(kItemsPerCta * mixed_grid_ctas(), kMaxChunkedTiles);
+    if (tiles <= 0 || tiles >= want) return 1;
+    const int64_t k = std::min<int64_t>({(want + tiles - 1) / tiles, kMaxChunks, pulses / kMinChunkPulses});
+    return k < 1 ? 1 : (int)k;
 }
 
 // Resident CTAs of the current device, looked up once per device: the pulse-chunk count

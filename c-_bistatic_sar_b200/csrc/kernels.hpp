@@ -110,6 +110,32 @@ struct BpArgs {
     const float* ref_bin_f; // np, ref_L * fs_eff / c - ref_bin_i
 };
 
+// Order in which the mixed kernel takes the voxels of nz whole z-planes: the voxel at
+// position k.  It keeps the 32 voxels of a warp close together, which keeps their candidate
+// lists short and their gathers on few cache lines: pairs of z-planes, in them strips of
+// four x, in them y, and per y the strip's 4 x 2 voxels, so a warp is a 4 x 4 x 2 block.
+// Strips run back and forth in y and layers back and forth in x, so the voxels on both
+// sides of a strip's end are neighbours too and no lane is spent on padding.
+inline __host__ __device__ void compact_voxel(int nx, int ny, int nz, int64_t k, int& x, int& y, int& z)
+{
+    const int64_t layer = (int64_t)2 * nx * ny;
+    const int zl = (int)(k / layer);
+    int64_t r = k - layer * zl;
+    const int hz = nz - 2 * zl < 2 ? nz - 2 * zl : 2;
+    const int64_t strip = (int64_t)4 * ny * hz;
+    const int xs = (int)(r / strip);
+    r -= strip * xs;
+    const int hx = nx - 4 * xs < 4 ? nx - 4 * xs : 4;
+    const int block = hx * hz;                 // voxels of the strip per y
+    y = (int)(r / block);
+    const int q = (int)(r - (int64_t)y * block);
+    x = 4 * xs + q % hx;
+    z = 2 * zl + q / hx;
+    const int64_t strips = (nx + 3) / 4;
+    if ((zl * strips + xs) & 1) y = ny - 1 - y;
+    if (zl & 1) x = nx - 1 - x;
+}
+
 // DEM tile of the mixed kernel (nodes): TMA box dims.  The x extent is a multiple of
 // 4 floats so every tiled copy row is a multiple of 16 bytes.
 constexpr int kMixedTileI = 68;
@@ -124,13 +150,13 @@ struct alignas(64) MixedReq {
     int pitch;            // row pitch (floats), a multiple of 4
     int use_tile;         // tmap valid: stage DEM tiles with TMA
     int fp16;             // samples stored FP16 complex + scale (else complex64)
-    int exhaustive;       // 1: node scans rank every node (no pruning); the image is the same
+    int exhaustive;       // 1: node scans rank every node (no candidate lists); the image is the same
+    int compact;          // the voxel range is whole z-planes: warps take compact blocks of voxels
     float stepx, stepy, istepx, istepy;
     double ox, oy;        // origin of the FP32 frame (first DEM node)
     double idx64, idy64;  // 1 / spacing
     float off_x, off_y;   // mean crossing offset from the voxel, metres (tile centring)
     float start_band;     // node units: FP32 flat starts this close to a cell boundary are redone in FP64
-    float zmin;           // lowest FP32 height of the DEM (bounds of the pruned node scan)
 };
 
 // Pulse chunks of a request (kept beside MixedReq, read only by the chunked kernel).
@@ -170,9 +196,15 @@ cudaError_t launch_transpose_c128(const double2* in, double2* out, int64_t R, in
 cudaError_t launch_real_to_c128(const double* in, double2* out, int64_t n, cudaStream_t st);
 int mixed_grid_ctas();   // persistent grid size (SMs x resident CTAs)
 // Pulse chunks per 128-voxel tile for a request of `voxels` voxels and `pulses` pulses:
-// as many as keep the request's work items within one wave of resident CTAs, at most 8
-// and with at least 128 pulses each; 1 for grids that already fill the GPU.  A property of the
-// request and the device only, so every path gives the same request the same image.
+// enough work items for four per resident CTA, at most kMaxChunks per tile and with at
+// least 32 pulses each; 1 for grids whose tiles alone are that many.  Items differ in cost
+// (list lengths, polished facets), so one wave of them leaves SMs idle: four items per CTA
+// against one wave of 128-pulse chunks measured 2.60 against 3.95 ms on a 161 x 161 x 1
+// slice of 1024 pulses and 4.4 against 8.3 ms on 97 x 83 x 11 voxels of 701 pulses.  A
+// property of the request and the device only, so every path gives the same request the
+// same image.
+constexpr int kMaxChunks = 8;
+constexpr int kMaxChunkedTiles = 4095;
 int mixed_chunks(int64_t voxels, int pulses);
 cudaError_t launch_ref_ranges(const DemView& d, const double* tx, const double* rx, int np, const double* center,
                               double n1, double n2, int W, double lambda, double bin_per_m, double* ref_L,

@@ -1,0 +1,56 @@
+"""The mixed kernel's candidate lists (a node scan shared by a warp's voxels and a block of
+pulses) against the scan that ranks every node of every window (exhaustive=True): the image
+must be the same bit for bit, over the geometries where the lists take other branches:
+long lists and no list (coarse voxels, fine DEMs), windows cut by the DEM's border or moving
+over the block (nodes outside some window), equal indices (the antenna is the lower endpoint
+of one leg), a lower index below ground, exact ties (a flat DEM), pulses far apart, low
+antennas, voxels at the surface, and grids with remainders in every axis."""
+import numpy as np
+import pytest
+
+import bsar
+from bsar import scene as S
+
+pytestmark = pytest.mark.gpu
+
+# name: (scene fields, antenna shift in z, z axis or None, search radius)
+CASES = {
+    "coarse voxels": (dict(nx=9, ny=17, nz=3, dxy=0.5, dz=0.4), 0.0, None, 0.0),
+    "fine dem": (dict(nx=10, ny=13, nz=3, dem_d=0.06, dem_n=400), 0.0, None, 0.0),
+    "wide window": (dict(nx=6, ny=9, nz=2, dem_d=0.125, dem_n=300), 0.0, None, 4.0),
+    "one-node window": (dict(nx=8, ny=9, nz=2, dem_d=2.0, dem_n=40), 0.0, None, 0.0),
+    "dem border": (dict(nx=12, ny=11, nz=3, dxy=0.2, dem_n=14), 0.0, None, 0.0),
+    "border, wide": (dict(nx=12, ny=11, nz=3, dxy=0.2, dem_d=0.125, dem_n=30), 0.0, None, 0.0),
+    "equal indices": (dict(nx=9, ny=10, nz=3, eps_r=1.0), 0.0, None, 0.0),
+    "lower index": (dict(nx=9, ny=10, nz=3, eps_r=0.5), 0.0, None, 0.0),
+    "flat dem": (dict(nx=9, ny=9, nz=3, dxy=0.25, dem_sigma=0.0, dem_kind="plane"), 0.0, None, 0.0),
+    "smooth dem": (dict(nx=13, ny=14, nz=3, dem_sigma=0.002, dem_kind="plane"), 0.0, None, 0.0),
+    "pulses apart": (dict(nx=9, ny=10, nz=3, n_pulses=9), 0.0, None, 0.0),
+    "low antennas": (dict(nx=9, ny=10, nz=3, n_pulses=60), -27.5, None, 0.0),
+    "surface voxels": (dict(nx=13, ny=10, nz=4), 0.0, np.array([-0.5, -0.2, 0.0, 0.3]), 0.0),
+    "single voxel": (dict(nx=1, ny=1, nz=1, n_scatterers=1), 0.0, None, 0.0),
+    "rows": (dict(nx=3, ny=45, nz=1), 0.0, None, 0.0),
+    "columns": (dict(nx=45, ny=1, nz=3), 0.0, None, 0.0),
+}
+
+
+@pytest.mark.parametrize("precision", ["mixed", "mixed_fp16"])
+@pytest.mark.parametrize("name", CASES)
+def test_lists_give_the_exhaustive_image(ctx, name, precision):
+    kw, dz, gz, radius = CASES[name]
+    sc = S.make_scene(S.scaled(S.config_spec(2), **{**dict(n_pulses=70, n_samples=4096, n_scatterers=3), **kw}),
+                      with_raw=False)
+    sc.tx = sc.tx + np.array([0.0, 0.0, dz])
+    sc.rx = sc.rx + np.array([0.0, 0.0, dz])
+    rng = np.random.default_rng(11)
+    sc.raw = rng.normal(size=(len(sc.tx), 4096)) + 1j * rng.normal(size=(len(sc.tx), 4096))
+    z = sc.gz if gz is None else gz
+    how = dict(solver="newton", legs="per_pulse", precision=precision, search_radius_m=radius)
+    sid = bsar.upload_scene(ctx, sc)
+    try:
+        full = ctx.backproject(sid, sc.gx, sc.gy, z, exhaustive=True, **how)
+        lists = ctx.backproject(sid, sc.gx, sc.gy, z, **how)
+    finally:
+        ctx.scene_release(sid)
+    assert np.abs(full).max() > 0
+    assert np.array_equal(lists, full)
