@@ -1,0 +1,327 @@
+// k_newton.cu -- FP64 back-projection with the Newton solver and per-pulse legs.
+//
+// The layout of the mixed kernel (k_mixed.cu): one thread per voxel, a warp's 32 voxels a
+// compact block of the grid, pulses in blocks of up to 16 whose antennas lie close together,
+// and per block and leg one candidate list of the DEM nodes that can win the node scan of
+// any of its (voxel, pulse) pairs (node_lists.cuh; the lists' bounds are FP32 with margins,
+// every path, ranking, Newton step, delay, phase and sum here is FP64).  Lists of up to four
+// nodes carry the nodes' path legs; where every listed node is itself the crossing for the
+// whole block, a solve is two table reads per node.  The other solves rank the list and polish
+// the facets around the best node (active-set Newton, one final step on the winning facet).
+//
+// A CTA's warps share 32 voxels and split the pulses into consecutive parts; the parts'
+// sums are added in pulse order.  The split follows the whole grid's size, so a range of
+// the grid has the image's bits.
+//
+// What bounds it: FP64 issue (list tables, sincospi, the polish of about a quarter of the
+// solves).  81 x 77 x 13 voxels x 512 pulses on a 0.25 m DEM, with pulse compression: 4.9 ms
+// on one B200; one warp per voxel with every pulse's own scan of (2W+1)^2 nodes, two FP64
+// square roots each, took 82 ms.  Three CTAs per SM (168 registers, no spills) against four:
+// 7.10 and 7.24 ms.
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "dev_common.cuh"
+#include "kernels.hpp"
+#include "node_lists.cuh"
+
+namespace bsar {
+
+namespace {
+
+// Heights for the candidate lists from the FP64 DEM.
+struct Heights64 {
+    const DemView& d;
+    __device__ __forceinline__ explicit Heights64(const DemView& d_) : d(d_) {}
+    __device__ __forceinline__ void cover(int, int, int, int) {}
+    __device__ __forceinline__ float operator()(int i, int j) const { return (float)__ldg(d.z + (int64_t)j * d.nx + i); }
+    __device__ __forceinline__ float ground(float x, float y) const
+    {
+        return (float)dem_elevation(d, (double)x + d.x0, (double)y + d.y0);
+    }
+};
+
+struct Leg64 {
+    double E[3], G[3], nE, nG;
+    bool g_lower;
+};
+
+// Window centre of a leg's node scan; h64: the height under the voxel.
+__device__ __noinline__ int2 start_node64(const DemView d, const Leg64 l, double h64)
+{
+    const double* Lp = l.g_lower ? l.G : l.E;
+    const double* Up = l.g_lower ? l.E : l.G;
+    const double h0 = l.g_lower ? h64 : dem_elevation(d, Lp[0], Lp[1]);
+    double sx, sy;
+    flat_start(Up, Lp, l.g_lower ? l.nE : l.nG, l.g_lower ? l.nG : l.nE, h0, kFlatIters, sx, sy);
+    return make_int2(nearest_node(d.x0, d.stepx, d.nx, sx), nearest_node(d.y0, d.stepy, d.ny, sy));
+}
+
+// Every node of one lane's window, in the solver's order (no list for the block).
+__device__ __noinline__ int2 scan_all64(const DemView d, const Leg64 l, double h64, int W)
+{
+    int2 best = start_node64(d, l, h64);
+    const int ia = max(best.x - W, 0), ib = min(best.x + W, d.nx - 1);
+    const int ja = max(best.y - W, 0), jb = min(best.y + W, d.ny - 1);
+    double v = INFINITY;
+    for (int i = ia; i <= ib; i++)
+        for (int j = ja; j <= jb; j++) {
+            const double u = node_l64(d, i, j, l.E, l.G, l.nE, l.nG);
+            if (u < v) {
+                v = u;
+                best = make_int2(i, j);
+            }
+        }
+    return best;
+}
+
+// A longer list, ranked in FP64 (it is in the solver's order).
+__device__ __forceinline__ int2 rank_list64(const DemView& d, const float4* list, const LegList& H, const Leg64& l,
+                                            double h64, int W)
+{
+    int2 st = make_int2(0, 0), best = make_int2(H.si, H.sj);
+    const bool core = H.mode & kCore;
+    if (!core) st = start_node64(d, l, h64);
+    double v = INFINITY;
+#pragma unroll 1
+    for (int k = 0; k < H.m; k++) {
+        const int pk = __float_as_int(list[k].w), i = H.i0 + (pk >> 16), j = H.j0 + (pk & 0xffff);
+        if (!core && (abs(i - st.x) > W || abs(j - st.y) > W)) continue;
+        const double u = node_l64(d, i, j, l.E, l.G, l.nE, l.nG);
+        if (u < v) {
+            v = u;
+            best = make_int2(i, j);
+        }
+    }
+    return best;
+}
+
+// From the best node (bi, bj) to the path: each of the four facets that have the node as
+// a corner, unless that corner is its minimum (the path's one-sided derivatives at the
+// node), is polished; one more step on the best facet.
+__device__ __forceinline__ double polish64(const DemView& d, const Leg64& l, double istepx, double istepy, int bi, int bj)
+{
+    const double x = __ldg(d.xv + bi), y = __ldg(d.yv + bj);
+    const int im = max(bi - 1, 0), ip = min(bi + 1, d.nx - 1), jm = max(bj - 1, 0), jp = min(bj + 1, d.ny - 1);
+    const int64_t row = (int64_t)bj * d.nx;
+    const double z = __ldg(d.z + row + bi);
+    double gxb, gxf, gyb, gyf, best;
+    {
+        const double ex = x - l.E[0], ey = y - l.E[1], ez = z - l.E[2];
+        const double gx = x - l.G[0], gy = y - l.G[1], gz = z - l.G[2];
+        const double qe = ex * ex + ey * ey + ez * ez, qg = gx * gx + gy * gy + gz * gz;
+        const double se = l.nE * rsqrt(qe), sg = l.nG * rsqrt(qg);
+        best = path64(leg_len64(x, y, z, l.E), leg_len64(x, y, z, l.G), l.nE, l.nG);
+        const double Fx = se * ex + sg * gx, Fy = se * ey + sg * gy, Fz = se * ez + sg * gz;
+        gxb = Fx + Fz * (z - __ldg(d.z + row + im)) * istepx;
+        gxf = Fx + Fz * (__ldg(d.z + row + ip) - z) * istepx;
+        gyb = Fy + Fz * (z - __ldg(d.z + (int64_t)jm * d.nx + bi)) * istepy;
+        gyf = Fy + Fz * (__ldg(d.z + (int64_t)jp * d.nx + bi) - z) * istepy;
+    }
+    bool moved = false;
+    double bu = 0.0, bv = 0.0;
+    int bfi = 0, bfj = 0;
+    auto at = [&](const Facet64& F, double u, double v) {
+        const double px = F.x0 + u * F.dx, py = F.y0 + v * F.dy, pz = F.z00 + F.b * u + F.c * v + F.e * u * v;
+        return path64(leg_len64(px, py, pz, l.E), leg_len64(px, py, pz, l.G), l.nE, l.nG);
+    };
+#pragma unroll 1
+    for (int k = 0; k < 4; k++) {
+        const bool kx = k >> 1, ky = k & 1;
+        const int fi = bi - 1 + kx, fj = bj - 1 + ky;
+        if (fi < 0 || fj < 0 || fi > d.nx - 2 || fj > d.ny - 2) continue;
+        if ((kx ? gxf > 0.0 : gxb < 0.0) && (ky ? gyf > 0.0 : gyb < 0.0)) continue;
+        Facet64 F;
+        facet_load(d, fi, fj, F);
+        const double idx = 1.0 / F.dx, idy = 1.0 / F.dy;
+        double u = kx ? 0.0 : 1.0, v = ky ? 0.0 : 1.0;
+        bool m = false;
+#pragma unroll 1
+        for (int it = 0; it < kPolishIters; it++) {
+            if (!facet_newton64(F, l.E, l.G, l.nE, l.nG, idx, idy, u, v)) break;
+            m = true;
+        }
+        const double L = m ? at(F, u, v) : best;
+        if (L < best) {
+            best = L;
+            moved = true;
+            bu = u;
+            bv = v;
+            bfi = fi;
+            bfj = fj;
+        }
+    }
+    if (moved) {
+        Facet64 F;
+        facet_load(d, bfi, bfj, F);
+        facet_newton64(F, l.E, l.G, l.nE, l.nG, 1.0 / F.dx, 1.0 / F.dy, bu, bv);
+        best = at(F, bu, bv);
+    }
+    return best;
+}
+
+struct NewtonWarp {
+    BlockLists l;
+    double path[kBlockPulses][32];
+    LegList h[2];
+};
+
+}  // namespace
+
+template <int WPC>
+__global__ void __launch_bounds__(32 * WPC, WPC == 4 ? 3 : 16 / WPC) k_bp_newton(BpArgs a, float start_band, int compact)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    NewtonWarp* ws = reinterpret_cast<NewtonWarp*>(smem_raw) + (threadIdx.x >> 5);
+    __shared__ double2 part[WPC][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const DemView& d = a.dem;
+    ListGrid m;
+    m.nx = d.nx;
+    m.ny = d.ny;
+    m.stepx = (float)d.stepx;
+    m.stepy = (float)d.stepy;
+    m.istepx = (float)(1.0 / d.stepx);
+    m.istepy = (float)(1.0 / d.stepy);
+    m.start_band = start_band;
+    m.extent = fmaxf((float)d.nx * m.stepx, (float)d.ny * m.stepy);
+    const double istepx = 1.0 / d.stepx, istepy = 1.0 / d.stepy;
+    const int64_t kk = (int64_t)blockIdx.x * 32 + lane;
+    const int3 vx = voxel_at(a, compact, kk < a.v_count ? kk : a.v_count - 1);
+    const double P[3] = {__ldg(a.gx + vx.x), __ldg(a.gy + vx.y), __ldg(a.gz + vx.z)};
+    const float P32[3] = {(float)(P[0] - d.x0), (float)(P[1] - d.y0), (float)P[2]};
+    const double h64 = dem_elevation(d, P[0], P[1]);
+    const WarpVoxels wv = warp_voxels(P32);
+    if (lane < 2) ws->h[lane].si = ws->h[lane].sj = -1;
+    __syncwarp();
+    const double inv_c = 1.0 / a.c, inv_lambda = 1.0 / a.lambda;
+    const Heights64 zat(d);
+    const int p0 = (int)((int64_t)w * a.np / WPC), p1 = (int)((int64_t)(w + 1) * a.np / WPC);
+    double accr = 0.0, acci = 0.0;
+    int n;
+    for (int i = p0; i < p1; i += n) {
+        n = pulse_block(m, zat, d, ws->l, ws->h, a.tx, a.rx, i, p1, d.x0, d.y0, P, P32, (float)h64, wv, a.n1, a.n2, a.W,
+                        true);
+        const int m0 = all_pinned(ws->h[0]) ? ws->h[0].m : 0, m1 = all_pinned(ws->h[1]) ? ws->h[1].m : 0;
+        // the legs to solve, one after the other over the block's pulses
+#pragma unroll 1
+        for (int leg = m0 ? 1 : 0; leg < (m1 ? 1 : 2); leg++) {
+            const LegList* H = &ws->h[leg];
+            const int hm = H->m, mode = H->mode;
+            Leg64 l;
+#pragma unroll
+            for (int c = 0; c < 3; c++) l.G[c] = P[c];
+            l.nE = a.n1;
+            l.nG = a.n2;
+            l.g_lower = lower_is_voxel((float)a.n1, (float)a.n2, leg == 0);
+#pragma unroll 1
+            for (int q = 0; q < n; q++) {
+                double L = 0.0;
+                int2 node = make_int2(0, 0);
+                bool solved = false;
+                if (hm > 0 && mode == (kCore | kTables)) {
+                    int c;
+                    L = table_min(ws->l.tab[leg], hm, q, lane, c);
+                    solved = (H->pinned >> c) & 1;
+                    node = H->node[c];
+                }
+                if (!solved) {
+                    const double* tr = (leg ? a.rx : a.tx) + 3 * (i + q);
+#pragma unroll
+                    for (int c = 0; c < 3; c++) l.E[c] = __ldg(tr + c);
+                    if (hm < 0) {
+                        node = scan_all64(d, l, h64, a.W);
+                    } else if (!(mode & kTables)) {
+                        node = rank_list64(d, ws->l.list[leg], *H, l, h64, a.W);
+                    } else if (!(mode & kCore)) {
+                        // a listed node may lie outside this solve's window
+                        const int2 st = start_node64(d, l, h64);
+                        const NodeTables* t = &ws->l.tab[leg];
+                        double v = INFINITY;
+                        int c = 0;
+#pragma unroll 1
+                        for (int k = 0; k < hm; k++) {
+                            const int2 nd = H->node[k];
+                            const double u = __dadd_rn(t->E[k][q], t->G[k][lane]);
+                            if (u < v && abs(nd.x - st.x) <= a.W && abs(nd.y - st.y) <= a.W) {
+                                v = u;
+                                c = k;
+                            }
+                        }
+                        node = H->node[c];
+                    }
+                    L = polish64(d, l, istepx, istepy, node.x, node.y);
+                }
+                double* path = &ws->path[q][lane];
+                *path = (leg && !m0) ? *path + L : L;
+            }
+        }
+        // delays, gathers and sums of the block's pulses
+#pragma unroll 1
+        for (int q = 0; q < n; q++) {
+            double L = (m0 && m1) ? 0.0 : ws->path[q][lane];
+            int c;
+            if (m0) L += table_min(ws->l.tab[0], m0, q, lane, c);
+            if (m1) L += table_min(ws->l.tab[1], m1, q, lane, c);
+            const double t_val = inv_c * L;                          // proc_test_script.cpp:565
+            const double b = (1.0 + t_val * a.fs_eff) - 1.0;         // :569, :593
+            // (int)floor(b) >= 0 && (int)ceil(b) < nr  <=>  0 <= b <= nr - 1 (NaN fails both)
+            if (b >= 0.0 && b <= (double)(a.nr - 1)) {
+                const double lo_d = floor(b);
+                const int lo = (int)lo_d;                            // nr <= 2^30
+                const double qf = b - lo_d;
+                const double2* row = a.rc64 + (int64_t)(i + q) * a.nr + lo;
+                const double2 s0 = __ldg(row);
+                double vr = s0.x, vi = s0.y;
+                if (qf != 0.0) {
+                    const double2 s1 = __ldg(row + 1);
+                    vr = (1.0 - qf) * s0.x + qf * s1.x;              // :635
+                    vi = (1.0 - qf) * s0.y + qf * s1.y;
+                }
+                // carrier phase (:573, :638) in turns, reduced before the sine
+                const double turns = rint(L * inv_lambda);
+                double sn, cs;
+                sincospi(2.0 * (fma(-turns, a.lambda, L) * inv_lambda), &sn, &cs);
+                accr += vr * cs - vi * sn;
+                acci += vr * sn + vi * cs;
+            }
+        }
+    }
+    part[w][lane] = make_double2(accr, acci);
+    __syncthreads();
+    if (w == 0 && kk < a.v_count) {
+#pragma unroll
+        for (int q = 1; q < WPC; q++) {
+            accr += part[q][lane].x;
+            acci += part[q][lane].y;
+        }
+        a.out[((int64_t)vx.x * a.ny + vx.y) * a.nz + vx.z] = make_double2(accr, acci);
+    }
+}
+
+template <int WPC> static cudaError_t launch_wpc(const BpArgs& a, float band, int compact, cudaStream_t st)
+{
+    const size_t sm = sizeof(NewtonWarp) * WPC;
+    cudaError_t e = cudaFuncSetAttribute(k_bp_newton<WPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    k_bp_newton<WPC><<<(unsigned)((a.v_count + 31) / 32), 32 * WPC, sm, st>>>(a, band, compact);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_bp_newton(const BpArgs& a, cudaStream_t st)
+{
+    const int64_t plane = (int64_t)a.nx * a.ny;
+    const int compact = a.v_begin % plane == 0 && a.v_count % plane == 0;
+    const float band = list_start_band(a.dem);
+    // warps per 32 voxels: enough for about three waves of 16 warps per SM, with at least a
+    // pulse block each
+    const int64_t tiles = (plane * a.nz + 31) / 32;
+    int wpc = 4;
+    while (wpc < 16 && tiles * wpc < (int64_t)148 * 48 && a.np >= 2 * wpc * kBlockPulses) wpc *= 2;
+    if (wpc == 16) return launch_wpc<16>(a, band, compact, st);
+    if (wpc == 8) return launch_wpc<8>(a, band, compact, st);
+    return launch_wpc<4>(a, band, compact, st);
+}
+
+}  // namespace bsar

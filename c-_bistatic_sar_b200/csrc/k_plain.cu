@@ -6,7 +6,9 @@
 // Each lane solves its pulse's two crossing points and forms the pulse's contribution;
 // the warp then adds the 32 contributions to the voxel sum in pulse order through
 // shuffles, so the FP64 sum has exactly the reference's order (pulse 0, 1, 2, ...,
-// proc_test_script.cpp:589-641) while 32 pulses are solved in parallel.
+// proc_test_script.cpp:589-641) while 32 pulses are solved in parallel.  The Newton solver
+// with per-pulse legs runs in k_newton.cu (16x faster); here it serves DEMs without a facet,
+// which have no node lists, and the mean legs.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -284,6 +286,7 @@ cudaError_t launch_slant_range(const DemView& d, const double* tx, const double*
 
 cudaError_t launch_bp_plain(const BpArgs& a, int solver, int legs, cudaStream_t st)
 {
+    if (solver != 0 && legs != 0 && !a.dem.empty && a.dem.nx >= 2 && a.dem.ny >= 2) return launch_bp_newton(a, st);
     // one warp per voxel; 4 warps per CTA; enough CTAs to cover the voxel range
     int64_t ctas = (a.v_count + 3) / 4;
     int blocks = (int)(ctas > (int64_t)148 * 512 ? (int64_t)148 * 512 : (ctas < 1 ? 1 : ctas));

@@ -185,6 +185,8 @@ struct MixedBatch {
 };
 
 cudaError_t launch_bp_plain(const BpArgs& a, int solver, int legs, cudaStream_t st);
+// FP64 Newton, per-pulse legs, a DEM of at least 2 x 2 nodes
+cudaError_t launch_bp_newton(const BpArgs& a, cudaStream_t st);
 cudaError_t launch_refraction_mixed(const DemView& d, int pitch, const double* p1, const double* p2, int64_t n,
                                     double n1, double n2, int W, double* out, cudaStream_t st);
 // chunked: some request of the batch has nchunk > 1 (the kernel with the chunk sums)

@@ -1,0 +1,49 @@
+"""The FP64 Newton back-projection on candidate lists (k_newton.cu) against the oracle's FP64
+Newton image, rel-L2 <= 1e-9, where its branches differ: short and long lists, no list,
+windows cut by the DEM's border, equal indices and a lower one below ground, an exactly flat
+DEM, few pulses far apart, and the warps-per-voxel splits (few and many pulses, grids with
+remainders)."""
+import numpy as np
+import pytest
+
+import bsar
+from bsar import scene as S
+import oracle as O
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    "rough": dict(nx=7, ny=9, nz=3),
+    "coarse voxels": dict(nx=5, ny=9, nz=2, dxy=0.5, dz=0.4),
+    "fine dem": dict(nx=4, ny=5, nz=2, dem_d=0.08, dem_n=300),
+    "dem border": dict(nx=6, ny=7, nz=2, dxy=0.3, dem_n=14),
+    "equal indices": dict(nx=5, ny=6, nz=2, eps_r=1.0),
+    "lower index": dict(nx=5, ny=6, nz=2, eps_r=0.5),
+    "flat dem": dict(nx=5, ny=5, nz=3, dxy=0.27, dem_sigma=0.0, dem_kind="plane"),
+    "smooth dem": dict(nx=5, ny=6, nz=3, dem_sigma=0.002, dem_kind="plane"),
+    "pulses apart": dict(nx=5, ny=6, nz=2, n_pulses=9),
+    "many pulses": dict(nx=3, ny=3, nz=1, n_pulses=1100),
+    "eight warps": dict(nx=3, ny=5, nz=1, n_pulses=300),
+    "one pulse": dict(nx=3, ny=5, nz=1, n_pulses=1),
+}
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_newton_image_matches_the_oracle(ctx, oracle, name):
+    spec = S.scaled(S.config_spec(2), **{**dict(n_pulses=50, n_samples=4096, n_scatterers=2), **CASES[name]})
+    sc = S.make_scene(spec, with_raw=False)
+    rng = np.random.default_rng(5)
+    sc.raw = rng.normal(size=(spec.n_pulses, 4096)) + 1j * rng.normal(size=(spec.n_pulses, 4096))
+    sid = bsar.upload_scene(ctx, sc)
+    try:
+        img = ctx.backproject(sid, sc.gx, sc.gy, sc.gz, solver="newton", legs="per_pulse", precision="fp64")
+    finally:
+        ctx.scene_release(sid)
+    rc = oracle.spline_upsample(oracle.fft_correlate(sc.raw, sc.reference), spec.upsample)
+    want = oracle.backproject(O.Dem(sc.x_vec, sc.y_vec, sc.z), sc.tx, sc.rx, rc, sc.gx, sc.gy, sc.gz, spec.n1, spec.n2,
+                              3e8, sc.fs_eff, sc.lam, legs="per", solver="newton",
+                              search_nodes=S.search_nodes_for(sc.x_vec, sc.y_vec))
+    assert np.abs(want).max() > 0
+    assert rel_l2(img, want) <= 1e-9
