@@ -479,6 +479,8 @@ static void backproject(bsar_ctx* ctx, bsar_scene_id id, const bsar_grid* g, con
     a.v_begin = v_begin;
     a.v_count = v_count;
     a.out = d_out;
+    a.zlo = s->dem.zlo;
+    a.zhi = s->dem.zhi;
     if (o->precision == BSAR_FP64) {
         launched(ctx, launch_bp_plain(a, o->solver, o->legs, ctx->stream), "back-projection (FP64)");
         return;

@@ -30,14 +30,35 @@ template <int SOLVER>
 __global__ void __launch_bounds__(64) k_refraction_points(DemView d, const double* __restrict__ p1, const double* __restrict__ p2,
                                     int64_t n, double n1, double n2, int W, double* __restrict__ out)
 {
+    __shared__ SolverShared<SOLVER, 64> sh;
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
         double A[3] = {p1[3 * k], p1[3 * k + 1], p1[3 * k + 2]};
         double B[3] = {p2[3 * k], p2[3 * k + 1], p2[3 * k + 2]};
         double o[3];
-        refraction_point<SOLVER, 64>(d, A, B, n1, n2, W, o);
+        refraction_point<SOLVER, 64>(d, A, B, n1, n2, W, &sh, o);
         out[3 * k] = o[0];
         out[3 * k + 1] = o[1];
         out[3 * k + 2] = o[2];
+    }
+}
+
+// The same with a warp per point, for batches that do not fill the GPU with threads.
+template <int SOLVER>
+__global__ void __launch_bounds__(64) k_refraction_points_warp(DemView d, const double* __restrict__ p1,
+                                                               const double* __restrict__ p2, int64_t n, double n1,
+                                                               double n2, int W, double* __restrict__ out)
+{
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t k = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); k < n; k += warps) {
+        const double A[3] = {p1[3 * k], p1[3 * k + 1], p1[3 * k + 2]};
+        const double B[3] = {p2[3 * k], p2[3 * k + 1], p2[3 * k + 2]};
+        double o[3];
+        refraction_point_warp<SOLVER>(d, A, B, n1, n2, W, o);
+        if ((threadIdx.x & 31) == 0) {
+            out[3 * k] = o[0];
+            out[3 * k + 1] = o[1];
+            out[3 * k + 2] = o[2];
+        }
     }
 }
 
@@ -84,13 +105,14 @@ __global__ void __launch_bounds__(64) k_slant_range(DemView d, const double* __r
                               double* __restrict__ ranges, double* __restrict__ ida, double* __restrict__ volta,
                               double* __restrict__ refl)
 {
+    __shared__ SolverShared<SOLVER, 64> sh;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
         double T[3] = {tx[3 * i], tx[3 * i + 1], tx[3 * i + 2]};
         double R[3] = {rx[3 * i], rx[3 * i + 1], rx[3 * i + 2]};
         double P[3] = {Px, Py, Pz};
         double a[3], b[3];
-        refraction_point<SOLVER, 64>(d, T, P, n1, n2, W, a);   // :166-172
-        refraction_point<SOLVER, 64>(d, P, R, n2, n1, W, b);   // :175-181
+        refraction_point<SOLVER, 64>(d, T, P, n1, n2, W, &sh, a);   // :166-172
+        refraction_point<SOLVER, 64>(d, P, R, n2, n1, W, &sh, b);   // :175-181
         for (int c = 0; c < 3; c++) {
             ida[3 * i + c] = a[c];
             volta[3 * i + c] = b[c];
@@ -107,12 +129,54 @@ __global__ void __launch_bounds__(64) k_slant_range(DemView d, const double* __r
     }
 }
 
+// The same with a warp per pulse and leg.
+template <int SOLVER>
+__global__ void __launch_bounds__(64) k_slant_range_warp(DemView d, const double* __restrict__ tx,
+                                                         const double* __restrict__ rx, int64_t np, double Px, double Py,
+                                                         double Pz, double n1, double n2, int W,
+                                                         double* __restrict__ ranges, double* __restrict__ ida,
+                                                         double* __restrict__ volta, double* __restrict__ refl)
+{
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const double P[3] = {Px, Py, Pz};
+    for (int64_t k = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); k < 2 * np; k += warps) {
+        const int64_t i = k >> 1;
+        const bool back = k & 1;
+        const double* tr = (back ? rx : tx) + 3 * i;
+        const double E[3] = {tr[0], tr[1], tr[2]};
+        double a[3];
+        // one call serves both legs: Tx -> P (:166-172) and P -> Rx (:175-181)
+        const double A[3] = {back ? P[0] : E[0], back ? P[1] : E[1], back ? P[2] : E[2]};
+        const double B[3] = {back ? E[0] : P[0], back ? E[1] : P[1], back ? E[2] : P[2]};
+        refraction_point_warp<SOLVER>(d, A, B, back ? n2 : n1, back ? n1 : n2, W, a);
+        if ((threadIdx.x & 31) == 0) {
+            double* o = (back ? volta : ida) + 3 * i;
+            for (int c = 0; c < 3; c++) o[c] = a[c];
+            double* r = ranges + (back ? 2 * np : 0) + i;
+            r[0] = sqrt((E[0] - a[0]) * (E[0] - a[0]) + (E[1] - a[1]) * (E[1] - a[1]) + (E[2] - a[2]) * (E[2] - a[2]));
+            r[np] = sqrt((P[0] - a[0]) * (P[0] - a[0]) + (P[1] - a[1]) * (P[1] - a[1]) + (P[2] - a[2]) * (P[2] - a[2]));
+            if (refl && !back) {
+                double q[3];
+                reflection_point(d, E[0], E[1], rx[3 * i], rx[3 * i + 1], q);
+                for (int c = 0; c < 3; c++) refl[3 * i + c] = q[c];
+            }
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------------
 // Back-projection, FP64: proc_test_script.cpp:491-669 for every voxel.
 // ---------------------------------------------------------------------------------
+template <int SOLVER> struct BpShared { using T = SolverShared<SOLVER, 128>; };
+template <> struct BpShared<2> { using T = FilterCols<128>; };
+
+// SOLVER: 0 grid search, 1 Newton, 2 grid search behind the FP32 filter (the same image;
+// zlo, zhi: the DEM's range of heights).
 template <int SOLVER, int LEGS>
-__global__ void __launch_bounds__(128) k_bp_plain(BpArgs a)
+__global__ void __launch_bounds__(128) k_bp_plain(BpArgs a, float zlo, float zhi)
 {
+    __shared__ typename BpShared<SOLVER>::T sh;
+    const int pitch = (a.dem.nx + 3) & ~3;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -131,15 +195,23 @@ __global__ void __launch_bounds__(128) k_bp_plain(BpArgs a)
         const double P[3] = {__ldg(a.gx + xi), __ldg(a.gy + yi), __ldg(a.gz + zi)};
         double accr = 0.0, acci = 0.0;
         for (int c0 = 0; c0 < np; c0 += 32) {
-            const int i = c0 + lane;
+            // lanes beyond the last pulse repeat it (a search may take the whole warp)
+            const int i = min(c0 + lane, np - 1);
             double cr = 0.0, ci = 0.0;
             int valid = 0;
-            if (i < np) {
+            {
                 const double T[3] = {__ldg(tx + 3 * i), __ldg(tx + 3 * i + 1), __ldg(tx + 3 * i + 2)};
                 const double R[3] = {__ldg(rx + 3 * i), __ldg(rx + 3 * i + 1), __ldg(rx + 3 * i + 2)};
                 double ia[3], vb[3];
-                refraction_point<SOLVER, 128>(a.dem, T, P, a.n1, a.n2, a.W, ia);   // ida
-                refraction_point<SOLVER, 128>(a.dem, P, R, a.n2, a.n1, a.W, vb);   // volta
+                if constexpr (SOLVER == 2) {
+                    refraction_grid_filter<128>(a.dem, pitch, zlo, zhi, T[0], T[1], T[2], P[0], P[1], P[2], a.n1, a.n2,
+                                                &sh, ia);                                  // ida
+                    refraction_grid_filter<128>(a.dem, pitch, zlo, zhi, P[0], P[1], P[2], R[0], R[1], R[2], a.n2, a.n1,
+                                                &sh, vb);                                  // volta
+                } else {
+                    refraction_point<SOLVER, 128>(a.dem, T, P, a.n1, a.n2, a.W, &sh, ia);   // ida
+                    refraction_point<SOLVER, 128>(a.dem, P, R, a.n2, a.n1, a.W, &sh, vb);   // volta
+                }
                 double dx = P[0] - ia[0], dy = P[1] - ia[1], dz = P[2] - ia[2];
                 const double R2t = sqrt(dx * dx + dy * dy + dz * dz);          // :497-505
                 dx = P[0] - vb[0];
@@ -214,18 +286,27 @@ __global__ void __launch_bounds__(128) k_bp_plain(BpArgs a)
 
 // Per-pulse reference optical path to the grid centre (FP64, Newton, per-pulse legs)
 // and its carrier phase reduced to [-pi, pi) in FP64: the mixed form's anchors.
-__global__ void k_ref_ranges(DemView d, const double* __restrict__ tx, const double* __restrict__ rx, int np,
+// WARP: a warp per pulse, else a thread.
+template <bool WARP>
+__global__ void __launch_bounds__(64) k_ref_ranges(DemView d, const double* __restrict__ tx, const double* __restrict__ rx, int np,
                              double cx, double cy, double cz, double n1, double n2, int W, double lambda,
                              double bin_per_m, double* __restrict__ ref_L, float* __restrict__ ref_phase,
                              int* __restrict__ ref_bin_i, float* __restrict__ ref_bin_f, double* __restrict__ offsets)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
+    const int per = WARP ? blockDim.x >> 5 : blockDim.x, t = WARP ? threadIdx.x >> 5 : threadIdx.x;
+    for (int i = blockIdx.x * per + t; i < np; i += gridDim.x * per) {
         const double T[3] = {tx[3 * i], tx[3 * i + 1], tx[3 * i + 2]};
         const double R[3] = {rx[3 * i], rx[3 * i + 1], rx[3 * i + 2]};
         const double P[3] = {cx, cy, cz};
         double ia[3], vb[3];
-        refraction_newton(d, T, P, n1, n2, W, ia);
-        refraction_newton(d, P, R, n2, n1, W, vb);
+        if constexpr (WARP) {
+            refraction_newton_warp(d, T, P, n1, n2, W, ia);
+            refraction_newton_warp(d, P, R, n2, n1, W, vb);
+            if ((threadIdx.x & 31) != 0) continue;
+        } else {
+            refraction_newton(d, T, P, n1, n2, W, ia);
+            refraction_newton(d, P, R, n2, n1, W, vb);
+        }
         auto dist = [](const double* u, const double* w) {
             double x = u[0] - w[0], y = u[1] - w[1], z = u[2] - w[2];
             return sqrt(x * x + y * y + z * z);
@@ -255,6 +336,14 @@ static int grid_for(int64_t n, int threads)
     return (int)(b < 1 ? 1 : b);
 }
 
+// Up to this many solves a warp takes one each (the search's points or the scan's nodes over
+// its lanes), beyond it a thread does.  A thread's search or scan is one serial chain, so
+// batches that do not fill the GPU wait for it; a warp repeats the starts and reductions in
+// every lane.  Whole call on a 256 x 256 DEM at 0.25 m, one B200, warp / thread: grid 256
+// points 121 / 451 us, 8192 236 / 483, 16384 383 / 519, 32768 739 / 613; Newton 256 points
+// 97 / 133 us, 8192 157 / 166, 16384 225 / 194.
+static int64_t warp_solves(int solver) { return solver == 0 ? 16384 : 8192; }
+
 cudaError_t launch_dem_elevation(const DemView& d, const double* xy, int64_t n, double* z, cudaStream_t st)
 {
     k_dem_elevation<<<grid_for(n, 128), 128, 0, st>>>(d, (const double2*)xy, n, z);
@@ -264,7 +353,12 @@ cudaError_t launch_dem_elevation(const DemView& d, const double* xy, int64_t n, 
 cudaError_t launch_refraction_points(const DemView& d, const double* p1, const double* p2, int64_t n, double n1,
                                      double n2, int solver, int W, double* out, cudaStream_t st)
 {
-    if (solver == 0)
+    if (n <= warp_solves(solver)) {
+        if (solver == 0)
+            k_refraction_points_warp<0><<<grid_for(n, 2), 64, 0, st>>>(d, p1, p2, n, n1, n2, W, out);
+        else
+            k_refraction_points_warp<1><<<grid_for(n, 2), 64, 0, st>>>(d, p1, p2, n, n1, n2, W, out);
+    } else if (solver == 0)
         k_refraction_points<0><<<grid_for(n, 64), 64, 0, st>>>(d, p1, p2, n, n1, n2, W, out);
     else
         k_refraction_points<1><<<grid_for(n, 64), 64, 0, st>>>(d, p1, p2, n, n1, n2, W, out);
@@ -275,7 +369,14 @@ cudaError_t launch_slant_range(const DemView& d, const double* tx, const double*
                                const double* target, double n1, double n2, int solver, int W, double* ranges,
                                double* ida, double* volta, double* refl, cudaStream_t st)
 {
-    if (solver == 0)
+    if (2 * np <= warp_solves(solver)) {
+        if (solver == 0)
+            k_slant_range_warp<0><<<grid_for(2 * np, 2), 64, 0, st>>>(d, tx, rx, np, target[0], target[1], target[2], n1,
+                                                                     n2, W, ranges, ida, volta, refl);
+        else
+            k_slant_range_warp<1><<<grid_for(2 * np, 2), 64, 0, st>>>(d, tx, rx, np, target[0], target[1], target[2], n1,
+                                                                     n2, W, ranges, ida, volta, refl);
+    } else if (solver == 0)
         k_slant_range<0><<<grid_for(np, 64), 64, 0, st>>>(d, tx, rx, np, target[0], target[1], target[2], n1, n2, W,
                                                           ranges, ida, volta, refl);
     else
@@ -290,10 +391,15 @@ cudaError_t launch_bp_plain(const BpArgs& a, int solver, int legs, cudaStream_t 
     // one warp per voxel; 4 warps per CTA; enough CTAs to cover the voxel range
     int64_t ctas = (a.v_count + 3) / 4;
     int blocks = (int)(ctas > (int64_t)148 * 512 ? (int64_t)148 * 512 : (ctas < 1 ? 1 : ctas));
-    if (solver == 0 && legs == 0) k_bp_plain<0, 0><<<blocks, 128, 0, st>>>(a);
-    else if (solver == 0) k_bp_plain<0, 1><<<blocks, 128, 0, st>>>(a);
-    else if (legs == 0) k_bp_plain<1, 0><<<blocks, 128, 0, st>>>(a);
-    else k_bp_plain<1, 1><<<blocks, 128, 0, st>>>(a);
+    const DemView& d = a.dem;
+    const bool filter = solver == 0 && !d.empty && d.uniform && d.nx >= 2 && d.ny >= 2 && d.z32 && a.n1 > 0 && a.n2 > 0;
+    const float zlo = a.zlo, zhi = a.zhi;
+    if (filter && legs == 0) k_bp_plain<2, 0><<<blocks, 128, 0, st>>>(a, zlo, zhi);
+    else if (filter) k_bp_plain<2, 1><<<blocks, 128, 0, st>>>(a, zlo, zhi);
+    else if (solver == 0 && legs == 0) k_bp_plain<0, 0><<<blocks, 128, 0, st>>>(a, zlo, zhi);
+    else if (solver == 0) k_bp_plain<0, 1><<<blocks, 128, 0, st>>>(a, zlo, zhi);
+    else if (legs == 0) k_bp_plain<1, 0><<<blocks, 128, 0, st>>>(a, zlo, zhi);
+    else k_bp_plain<1, 1><<<blocks, 128, 0, st>>>(a, zlo, zhi);
     return cudaGetLastError();
 }
 
@@ -301,8 +407,14 @@ cudaError_t launch_ref_ranges(const DemView& d, const double* tx, const double* 
                               double n1, double n2, int W, double lambda, double bin_per_m, double* ref_L,
                               float* ref_phase, int* ref_bin_i, float* ref_bin_f, double* offsets, cudaStream_t st)
 {
-    k_ref_ranges<<<grid_for(np, 64), 64, 0, st>>>(d, tx, rx, np, center[0], center[1], center[2], n1, n2, W, lambda,
-                                                  bin_per_m, ref_L, ref_phase, ref_bin_i, ref_bin_f, offsets);
+    if (2 * (int64_t)np <= warp_solves(1))
+        k_ref_ranges<true><<<grid_for(np, 2), 64, 0, st>>>(d, tx, rx, np, center[0], center[1], center[2], n1, n2, W,
+                                                           lambda, bin_per_m, ref_L, ref_phase, ref_bin_i, ref_bin_f,
+                                                           offsets);
+    else
+        k_ref_ranges<false><<<grid_for(np, 64), 64, 0, st>>>(d, tx, rx, np, center[0], center[1], center[2], n1, n2, W,
+                                                             lambda, bin_per_m, ref_L, ref_phase, ref_bin_i, ref_bin_f,
+                                                             offsets);
     return cudaGetLastError();
 }
 

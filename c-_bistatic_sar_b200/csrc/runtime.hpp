@@ -224,6 +224,7 @@ struct DemDev {
     std::unique_ptr<DevBuf> xv, yv, z, z32;
     DemView view{};
     int pitch = 0;                                  // row pitch of z32 (floats, multiple of 4)
+    float zlo = INFINITY, zhi = -INFINITY;          // range of z32
     alignas(64) unsigned char tmap[sizeof(CUtensorMap)] = {};
     bool has_tmap = false;
 };
@@ -333,7 +334,12 @@ inline DemDev stage_dem(bsar_ctx* ctx, const bsar_dem* d, bool want_z32)
         r.pitch = (int)((d->nx + 3) & ~int64_t(3));
         std::vector<float> zf((size_t)r.pitch * d->ny, 0.0f);
         for (int64_t j = 0; j < d->ny; j++)
-            for (int64_t i = 0; i < d->nx; i++) zf[j * r.pitch + i] = (float)d->z[j * d->nx + i];
+            for (int64_t i = 0; i < d->nx; i++) {
+                const float z = (float)d->z[j * d->nx + i];
+                zf[j * r.pitch + i] = z;
+                r.zlo = std::min(r.zlo, z);
+                r.zhi = std::max(r.zhi, z);
+            }
         r.z32 = dev_upload(ctx, zf.data(), sizeof(float) * zf.size());
         sync(ctx);   // zf goes out of scope
         v.z32 = r.z32->as<float>();
