@@ -54,9 +54,6 @@ namespace {
 
 constexpr int TI = kMixedTileI;    // tile columns (x); 272 B rows, a multiple of 16 B
 constexpr int TJ = kMixedTileJ;    // tile rows (y)
-// A polish step shorter than this (cell units) is the last: Newton's next one would be about
-// its square, 1e-5 cells, which moves the path by 1e-11 m and which the FP64 step makes.
-constexpr float kConverged = 4e-3f;
 constexpr long kWaitSpins = 1L << 24;
 
 struct Facet32 {
@@ -186,30 +183,17 @@ __device__ __forceinline__ float facet_eval32(const Facet32& F, const float A[3]
     return na * (q1 * rsqrtf(q1)) + nb * (q2 * rsqrtf(q2));
 }
 
-// FP64 final Newton step on facet (fi, fj) from (u, v); returns the optical path of the
-// result.
-__device__ __forceinline__ double final_step64(const DemView& d, int fi, int fj, const double A[3], const double B[3],
-                                               double na, double nb, double u, double v, double* X, double idx_,
-                                               double idy)
+// The crossing after the FP64 final step from (u, v) on facet (fi, fj).
+__device__ __forceinline__ void final_point64(const DemView& d, int fi, int fj, const double A[3], const double B[3],
+                                              double na, double nb, double u, double v, double X[3], double idx_,
+                                              double idy)
 {
     Facet64 F;
     facet_load(d, fi, fj, F);
     facet_newton64(F, A, B, na, nb, idx_, idy, u, v);
-    double x = F.x0 + u * F.dx, y = F.y0 + v * F.dy;
-    double h = F.z00 + F.b * u + F.c * v + F.e * u * v;
-    if ((u == 0.0 || u == 1.0) && (v == 0.0 || v == 1.0)) {
-        // a node: its own coordinates, so that the path is the one node_leg64 gives
-        const int i = fi + (int)u, j = fj + (int)v;
-        x = __ldg(d.xv + i);
-        y = __ldg(d.yv + j);
-        h = __ldg(d.z + (int64_t)j * d.nx + i);
-    }
-    if (X) {
-        X[0] = x;
-        X[1] = y;
-        X[2] = h;
-    }
-    return path64(leg_len64(x, y, h, A), leg_len64(x, y, h, B), na, nb);
+    X[0] = F.x0 + u * F.dx;
+    X[1] = F.y0 + v * F.dy;
+    X[2] = F.z00 + F.b * u + F.c * v + F.e * u * v;
 }
 
 // Node ranking values.  G is the voxel-side endpoint of the path (index ng), E the
@@ -452,7 +436,7 @@ struct Leg {
     float E32[3], G32[3];
     float nE, nG;
     double nE64, nG64;
-    bool g_lower;
+    bool g_lower, to_voxel;
 };
 
 // Window centre of a leg's node scan: the node nearest the flat start.  A start within
@@ -594,30 +578,40 @@ __device__ __forceinline__ int2 rank_list(const DemView& d, const MixedCtx& m, c
     return make_int2(H.i0 + (pk >> 16), H.j0 + (pk & 0xffff));
 }
 
-// From the best node (bi, bj) to the crossing: FP32 polish of the facets around it, FP64
-// final step.  Returns the FP64 optical path; X (optional): the crossing.
-__device__ __forceinline__ double finish_leg(const DemView& d, const MixedCtx& m, const Tile& T, const Leg& l, int bi,
-                                             int bj, double* X = nullptr)
+// The facet that holds the crossing around the best node (bi, bj), by FP32 polish, and the
+// crossing's (u, v) on it.  False: the node itself is the crossing.  Heights from the DEM tile when the node's 3 x 3 neighbourhood lies in it.
+// The nine heights are loaded once (indices clamped to the DEM; a facet that would need a
+// clamped one is not polished), and the path's gradient at the node is formed once: with
+// G = na (N - A)/|N - A| + nb (N - B)/|N - B|, a facet with the node at its corner (u0, v0)
+// has the gradient (Gx + Gz zx, Gy + Gz zy), zx and zy the facet's slopes along the edges
+// through the node (one-sided differences: backward where u0 = 1, forward where u0 = 0).
+// When it points out of the facet on both axes, the corner is that facet's minimum and the
+// facet keeps the node's path; the others take the Newton steps.  Each lane takes its own
+// facets one after the other, so lanes whose crossings lie on different sides of a node step
+// together.
+__device__ __forceinline__ bool polish_leg(const MixedCtx& m, const Tile& T, const Leg& l, int bi, int bj, int& bfi,
+                                           int& bfj, float& bu, float& bv)
 {
-    const float* A32 = l.E32;
-    const float* B32 = l.G32;
-    const float na = l.nE, nb = l.nG;
-    // polish the facets around the best node (FP32); heights from the DEM tile when the
-    //    node's 3 x 3 neighbourhood lies in it.  The nine heights are loaded once (indices
-    //    clamped to the DEM; a facet that would need a clamped one is not polished), and the
-    //    path's gradient at the node is formed once: with G = na (N - A)/|N - A| +
-    //    nb (N - B)/|N - B|, a facet with the node at its corner (u0, v0) has the gradient
-    //    (Gx + Gz zx, Gy + Gz zy), zx and zy the facet's slopes along the edges through the
-    //    node (one-sided differences: backward where u0 = 1, forward where u0 = 0).  When it
-    //    points out of the facet on both axes, the corner is that facet's minimum and the
-    //    facet keeps the node's path; the others take the Newton steps.
+    // the path's direction, which sets the order of its sums
+    float A32[3], B32[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        A32[c] = l.to_voxel ? l.E32[c] : l.G32[c];
+        B32[c] = l.to_voxel ? l.G32[c] : l.E32[c];
+    }
+    const float na = l.to_voxel ? l.nE : l.nG, nb = l.to_voxel ? l.nG : l.nE;
+    const bool xm = bi > 0, xp = bi < m.nx - 1, ym = bj > 0, yp = bj < m.ny - 1;
     const bool nt = T.ok && bi - 1 >= T.i0 && bi + 1 < T.i0 + TI && bj - 1 >= T.j0 && bj + 1 < T.j0 + TJ;
-    auto zt = [&](int i, int j) { return nt ? T.s[(j - T.j0) * TI + (i - T.i0)] : zf(m, i, j); };
-    const int im = max(bi - 1, 0), ip = min(bi + 1, m.nx - 1);
-    const int jm = max(bj - 1, 0), jp = min(bj + 1, m.ny - 1);
-    const float zmm = zt(im, jm), zm0 = zt(im, bj), zmp = zt(im, jp);
-    const float z0m = zt(bi, jm), z00n = zt(bi, bj), z0p = zt(bi, jp);
-    const float zpm = zt(ip, jm), zp0 = zt(ip, bj), zpp = zt(ip, jp);
+    float zmm, zm0, zmp, z0m, z00n, z0p, zpm, zp0, zpp;
+    {
+        const float* r0 = nt ? T.s + (bj - T.j0) * TI + (bi - T.i0) : m.z32 + (int64_t)bj * m.pitch + bi;
+        const int row = nt ? TI : m.pitch;
+        const float *rm = r0 - (ym ? row : 0), *rp = r0 + (yp ? row : 0);
+        const int om = xm ? -1 : 0, op = xp ? 1 : 0;
+        zmm = rm[om], z0m = rm[0], zpm = rm[op];
+        zm0 = r0[om], z00n = r0[0], zp0 = r0[op];
+        zmp = rp[om], z0p = rp[0], zpp = rp[op];
+    }
     float Lnode, gxb, gxf, gyb, gyf;
     {
         float xn = (float)bi * m.stepx, yn = (float)bj * m.stepy;
@@ -633,53 +627,65 @@ __device__ __forceinline__ double finish_leg(const DemView& d, const MixedCtx& m
         gyb = fmaf(Gz, (z00n - z0m) * m.istepy, Gy);
         gyf = fmaf(Gz, (z0p - z00n) * m.istepy, Gy);
     }
-    int bfi = min(bi, m.nx - 2), bfj = min(bj, m.ny - 2);     // fallback facet
-    float bestF = INFINITY, bu = (float)(bi - bfi), bv = (float)(bj - bfj);
+    const bool ixm = !(gxb < 0.0f), ixp = !(gxf > 0.0f), iym = !(gyb < 0.0f), iyp = !(gyf > 0.0f);
+    const unsigned facets = (unsigned)(xm && ym) | (unsigned)(xm && yp) << 1 | (unsigned)(xp && ym) << 2 |
+                            (unsigned)(xp && yp) << 3;
+    unsigned todo = facets & ((unsigned)(ixm || iym) | (unsigned)(ixm || iyp) << 1 | (unsigned)(ixp || iym) << 2 |
+                              (unsigned)(ixp || iyp) << 3);
+    bool moved = false;
+    float best = todo == facets ? INFINITY : Lnode;     // a facet whose minimum is the node gives its path
 #pragma unroll 1
-    for (int k = 0; k < 4; k++) {
+    while (todo) {
+        const int k = __ffs(todo) - 1;
+        todo &= todo - 1;
         const bool kx = k >> 1, ky = k & 1;       // facet on the +x / +y side of the node
-        int fi = bi - 1 + kx, fj = bj - 1 + ky;
-        if (fi < 0 || fj < 0 || fi > m.nx - 2 || fj > m.ny - 2) continue;
-        float u = (float)(bi - fi), v = (float)(bj - fj);
-        float L = Lnode;
-        const bool corner = (kx ? gxf > 0.0f : gxb < 0.0f) && (ky ? gyf > 0.0f : gyb < 0.0f);
-        if (!corner) {
-            Facet32 F;
-            F.x0 = (float)fi * m.stepx;
-            F.y0 = (float)fj * m.stepy;
-            F.dx = m.stepx;
-            F.dy = m.stepy;
-            F.idx = m.istepx;
-            F.idy = m.istepy;
-            // corners (fi, fj), (fi + 1, fj), (fi, fj + 1), (fi + 1, fj + 1) of the 3 x 3 block
-            const float z00 = kx ? (ky ? z00n : z0m) : (ky ? zm0 : zmm);
-            const float z01 = kx ? (ky ? zp0 : zpm) : (ky ? z00n : z0m);
-            const float z10 = kx ? (ky ? z0p : z00n) : (ky ? zmp : zm0);
-            const float z11 = kx ? (ky ? zpp : zp0) : (ky ? z0p : z00n);
-            F.z00 = z00;
-            F.b = z01 - z00;
-            F.c = z10 - z00;
-            F.e = z11 - z01 - z10 + z00;
-            bool moved = false;
+        const int fi = bi - 1 + kx, fj = bj - 1 + ky;
+        Facet32 F;
+        F.x0 = (float)fi * m.stepx;
+        F.y0 = (float)fj * m.stepy;
+        F.dx = m.stepx;
+        F.dy = m.stepy;
+        F.idx = m.istepx;
+        F.idy = m.istepy;
+        // corners (fi, fj), (fi + 1, fj), (fi, fj + 1), (fi + 1, fj + 1) of the 3 x 3 block
+        const float z00 = kx ? (ky ? z00n : z0m) : (ky ? zm0 : zmm);
+        const float z01 = kx ? (ky ? zp0 : zpm) : (ky ? z00n : z0m);
+        const float z10 = kx ? (ky ? z0p : z00n) : (ky ? zmp : zm0);
+        const float z11 = kx ? (ky ? zpp : zp0) : (ky ? z0p : z00n);
+        F.z00 = z00;
+        F.b = z01 - z00;
+        F.c = z10 - z00;
+        F.e = z11 - z01 - z10 + z00;
+        float u = kx ? 0.0f : 1.0f, v = ky ? 0.0f : 1.0f;
+        bool m1 = false;
 #pragma unroll 1
-            for (int it = 0; it < kPolishIters; it++) {
-                const float u0 = u, v0 = v;
-                if (!facet_step32(F, A32, B32, na, nb, u, v)) break;
-                moved = true;
-                if (fabsf(u - u0) + fabsf(v - v0) < kConverged) break;
-            }
-            // a facet whose corner is already its minimum keeps the best node's path
-            if (moved) L = facet_eval32(F, A32, B32, na, nb, u, v);
+        for (int it = 0; it < kPolishIters; it++) {
+            if (!facet_step32(F, A32, B32, na, nb, u, v)) break;
+            m1 = true;
         }
-        if (L < bestF) {
-            bestF = L;
+        const float L = m1 ? facet_eval32(F, A32, B32, na, nb, u, v) : Lnode;
+        if (L < best || (L == best && !moved)) {
+            best = L;
+            moved = m1;
             bu = u;
             bv = v;
             bfi = fi;
             bfj = fj;
         }
     }
-    return final_step64(d, bfi, bfj, l.E, l.G, l.nE64, l.nG64, (double)bu, (double)bv, X, m.idx64, m.idy64);
+    return moved;
+}
+
+// From the best node (bi, bj) to the leg's FP64 path: FP32 polish, FP64 final step.
+// `known`: the node's own path is node_path.
+__device__ __forceinline__ double finish_leg(const DemView& d, const MixedCtx& m, const Tile& T, const Leg& l, int bi,
+                                             int bj, bool known, double node_path)
+{
+    int fi, fj;
+    float u, v;
+    if (polish_leg(m, T, l, bi, bj, fi, fj, u, v))
+        return final_path64(d, fi, fj, l.E, l.G, l.nE64, l.nG64, m.idx64, m.idy64, (double)u, (double)v);
+    return known ? node_path : node_l64(d, bi, bj, l.E, l.G, l.nE64, l.nG64);
 }
 
 // ------------------------------- TMA tile staging -----------------------------------
@@ -830,13 +836,15 @@ __device__ __forceinline__ void voxel_mixed(const BpArgs& a, const MixedCtx& m, 
                 l.nE64 = a.n1;
                 l.nG64 = a.n2;
                 l.g_lower = lower_is_voxel(n1f, n2f, leg == 0);
+                l.to_voxel = leg == 0;
 #pragma unroll 1
                 for (int p = b; p < b + step; p++) {
                     double L = 0.0;
                     int2 node = make_int2(0, 0);
-                    bool solved = false;
+                    bool solved = false, known = false;
                     if (hm > 0 && mode == (kCore | kTables)) {
                         int c;
+                        known = true;
                         L = table_min(ws->u.b.l.tab[leg], hm, p - i, lane, c);
                         solved = (H->pinned >> c) & 1;
                         node = H->node[c];
@@ -870,7 +878,7 @@ __device__ __forceinline__ void voxel_mixed(const BpArgs& a, const MixedCtx& m, 
                             }
                             node = H->node[c];
                         }
-                        L = finish_leg(a.dem, m, T, l, node.x, node.y);
+                        L = finish_leg(a.dem, m, T, l, node.x, node.y, known, L);
                     }
                     double* d = path + (p - b) * 32 + lane;
                     *d = (leg && !m0) ? __dadd_rn(*d, L) : L;
@@ -1102,10 +1110,19 @@ __global__ void k_refraction_mixed(DemView d, MixedCtx m, const double* __restri
         l.nE64 = na;
         l.nG64 = nb;
         l.g_lower = lower_is_voxel(l.nE, l.nG, true);
+        l.to_voxel = true;
         double X[3];
         const VoxelStart vs{height32(m, l.G32[0], l.G32[1]), dem_elevation(d, l.G[0], l.G[1])};
         const int2 node = scan_lane(d, m, T, l, vs, W);
-        finish_leg(d, m, T, l, node.x, node.y, X);
+        int fi, fj;
+        float u, v;
+        if (!polish_leg(m, T, l, node.x, node.y, fi, fj, u, v)) {
+            fi = max(node.x - 1, 0);
+            fj = max(node.y - 1, 0);
+            u = (float)(node.x - fi);
+            v = (float)(node.y - fj);
+        }
+        final_point64(d, fi, fj, l.E, l.G, l.nE64, l.nG64, (double)u, (double)v, X, m.idx64, m.idy64);
         out[3 * k] = X[0];
         out[3 * k + 1] = X[1];
         out[3 * k + 2] = X[2];

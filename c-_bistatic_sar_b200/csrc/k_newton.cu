@@ -97,66 +97,88 @@ __device__ __forceinline__ int2 rank_list64(const DemView& d, const float4* list
     return best;
 }
 
+__device__ __forceinline__ double facet_path(const Facet64& F, const Leg64& l, double u, double v)
+{
+    const double x = F.x0 + u * F.dx, y = F.y0 + v * F.dy, z = F.z00 + F.b * u + F.c * v + F.e * u * v;
+    return path64(leg_len64(x, y, z, l.E), leg_len64(x, y, z, l.G), l.nE, l.nG);
+}
+
 // From the best node (bi, bj) to the path: each of the four facets that have the node as
-// a corner, unless that corner is its minimum (the path's one-sided derivatives at the
-// node), is polished; one more step on the best facet.
-__device__ __forceinline__ double polish64(const DemView& d, const Leg64& l, double istepx, double istepy, int bi, int bj)
+// a corner is polished, unless that corner is its minimum (the path's one-sided derivatives
+// at the node) or its minimum lies on an edge of another one (patch_skips); one more step on
+// the best facet.
+__device__ __forceinline__ double polish64(const DemView& d, const ListGrid& m, const Leg64& l, int bi, int bj)
 {
     const double x = __ldg(d.xv + bi), y = __ldg(d.yv + bj);
-    const int im = max(bi - 1, 0), ip = min(bi + 1, d.nx - 1), jm = max(bj - 1, 0), jp = min(bj + 1, d.ny - 1);
-    const int64_t row = (int64_t)bj * d.nx;
-    const double z = __ldg(d.z + row + bi);
-    double gxb, gxf, gyb, gyf, best;
-    {
-        const double ex = x - l.E[0], ey = y - l.E[1], ez = z - l.E[2];
-        const double gx = x - l.G[0], gy = y - l.G[1], gz = z - l.G[2];
-        const double qe = ex * ex + ey * ey + ez * ez, qg = gx * gx + gy * gy + gz * gz;
-        const double se = l.nE * rsqrt(qe), sg = l.nG * rsqrt(qg);
-        best = path64(leg_len64(x, y, z, l.E), leg_len64(x, y, z, l.G), l.nE, l.nG);
-        const double Fx = se * ex + sg * gx, Fy = se * ey + sg * gy, Fz = se * ez + sg * gz;
-        gxb = Fx + Fz * (z - __ldg(d.z + row + im)) * istepx;
-        gxf = Fx + Fz * (__ldg(d.z + row + ip) - z) * istepx;
-        gyb = Fy + Fz * (z - __ldg(d.z + (int64_t)jm * d.nx + bi)) * istepy;
-        gyf = Fy + Fz * (__ldg(d.z + (int64_t)jp * d.nx + bi) - z) * istepy;
+    const bool xm = bi > 0, xp = bi < d.nx - 1, ym = bj > 0, yp = bj < d.ny - 1;
+    const double* zr = d.z + (int64_t)bj * d.nx + bi;
+    const double z = __ldg(zr);
+    double best = path64(leg_len64(x, y, z, l.E), leg_len64(x, y, z, l.G), l.nE, l.nG);
+    // which facets to polish: FP32 derivatives; a corner within their rounding is polished, and
+    // its Newton step then finds it in FP64
+    NodePatch p;
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        const double* r = zr + (j == 0 ? (ym ? -d.nx : 0) : (j == 2 ? (yp ? d.nx : 0) : 0));
+        p.z[0][j] = (float)(__ldg(r + (xm ? -1 : 0)) - z);
+        p.z[1][j] = (float)(__ldg(r) - z);
+        p.z[2][j] = (float)(__ldg(r + (xp ? 1 : 0)) - z);
     }
-    bool moved = false;
+    p.rE[0] = (float)(x - l.E[0]), p.rE[1] = (float)(y - l.E[1]), p.rE[2] = (float)(z - l.E[2]);
+    p.rG[0] = (float)(x - l.G[0]), p.rG[1] = (float)(y - l.G[1]), p.rG[2] = (float)(z - l.G[2]);
+    const float nE = (float)l.nE, nG = (float)l.nG;
+    patch_gradient(p, m, nE, nG);
+    const unsigned skipped0 = patch_skips(p, m, patch_todo(p, xm, xp, ym, yp), nE, nG);
+    const float noise = 2e-5f * (nE + nG);
+    p.gxb += noise * (1.0f + fabsf(p.z[0][1]) * m.istepx);
+    p.gxf -= noise * (1.0f + fabsf(p.z[2][1]) * m.istepx);
+    p.gyb += noise * (1.0f + fabsf(p.z[1][0]) * m.istepy);
+    p.gyf -= noise * (1.0f + fabsf(p.z[1][2]) * m.istepy);
+    unsigned todo = patch_todo(p, xm, xp, ym, yp), skipped = skipped0;
+    todo &= ~skipped;
+    bool moved = false, settled = true;
     double bu = 0.0, bv = 0.0;
     int bfi = 0, bfj = 0;
-    auto at = [&](const Facet64& F, double u, double v) {
-        const double px = F.x0 + u * F.dx, py = F.y0 + v * F.dy, pz = F.z00 + F.b * u + F.c * v + F.e * u * v;
-        return path64(leg_len64(px, py, pz, l.E), leg_len64(px, py, pz, l.G), l.nE, l.nG);
-    };
 #pragma unroll 1
-    for (int k = 0; k < 4; k++) {
+    while (todo) {
+        const int k = __ffs(todo) - 1;
+        todo &= todo - 1;
         const bool kx = k >> 1, ky = k & 1;
         const int fi = bi - 1 + kx, fj = bj - 1 + ky;
-        if (fi < 0 || fj < 0 || fi > d.nx - 2 || fj > d.ny - 2) continue;
-        if ((kx ? gxf > 0.0 : gxb < 0.0) && (ky ? gyf > 0.0 : gyb < 0.0)) continue;
         Facet64 F;
         facet_load(d, fi, fj, F);
         const double idx = 1.0 / F.dx, idy = 1.0 / F.dy;
-        double u = kx ? 0.0 : 1.0, v = ky ? 0.0 : 1.0;
-        bool m = false;
+        double u = kx ? 0.0 : 1.0, v = ky ? 0.0 : 1.0, step = 0.0;
+        bool m1 = false;
 #pragma unroll 1
         for (int it = 0; it < kPolishIters; it++) {
+            const double ua = u, va = v;
             if (!facet_newton64(F, l.E, l.G, l.nE, l.nG, idx, idy, u, v)) break;
-            m = true;
+            m1 = true;
+            step = fabs(u - ua) + fabs(v - va);
         }
-        const double L = m ? at(F, u, v) : best;
-        if (L < best) {
-            best = L;
-            moved = true;
-            bu = u;
-            bv = v;
-            bfi = fi;
-            bfj = fj;
+        settled = settled && step < 4e-3;
+        if (m1) {
+            const double L = facet_path(F, l, u, v);
+            if (L < best) {
+                best = L;
+                moved = true;
+                bu = u;
+                bv = v;
+                bfi = fi;
+                bfj = fj;
+            }
+        }
+        if (!todo && !settled) {
+            todo = skipped;
+            skipped = 0;
         }
     }
     if (moved) {
         Facet64 F;
         facet_load(d, bfi, bfj, F);
         facet_newton64(F, l.E, l.G, l.nE, l.nG, 1.0 / F.dx, 1.0 / F.dy, bu, bv);
-        best = at(F, bu, bv);
+        best = facet_path(F, l, bu, bv);
     }
     return best;
 }
@@ -186,7 +208,6 @@ __global__ void __launch_bounds__(32 * WPC, WPC == 4 ? 3 : 16 / WPC) k_bp_newton
     m.istepy = (float)(1.0 / d.stepy);
     m.start_band = start_band;
     m.extent = fmaxf((float)d.nx * m.stepx, (float)d.ny * m.stepy);
-    const double istepx = 1.0 / d.stepx, istepy = 1.0 / d.stepy;
     const int64_t kk = (int64_t)blockIdx.x * 32 + lane;
     const int3 vx = voxel_at(a, compact, kk < a.v_count ? kk : a.v_count - 1);
     const double P[3] = {__ldg(a.gx + vx.x), __ldg(a.gy + vx.y), __ldg(a.gz + vx.z)};
@@ -251,7 +272,7 @@ __global__ void __launch_bounds__(32 * WPC, WPC == 4 ? 3 : 16 / WPC) k_bp_newton
                         }
                         node = H->node[c];
                     }
-                    L = polish64(d, l, istepx, istepy, node.x, node.y);
+                    L = polish64(d, m, l, node.x, node.y);
                 }
                 double* path = &ws->path[q][lane];
                 *path = (leg && !m0) ? *path + L : L;
