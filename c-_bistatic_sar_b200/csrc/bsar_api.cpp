@@ -78,6 +78,7 @@ void bsar_destroy(bsar_ctx* ctx)
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    ctx->stager.reset();
     ctx->scenes.clear();
     ctx->twiddles.clear();
     ctx->grid_dev.reset();
@@ -132,7 +133,7 @@ bsar_status bsar_dem_elevation(bsar_ctx* ctx, const bsar_dem* dem, const double*
         auto dxy = dev_upload(ctx, xy, sizeof(double) * 2 * n);
         auto dz = dev_alloc(ctx, sizeof(double) * n);
         launched(ctx, launch_dem_elevation(d.view, dxy->as<double>(), n, dz->as<double>(), ctx->stream), "elevation");
-        cuda_check(cudaMemcpyAsync(z_out, dz->p, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream), "download");
+        copy_d2h(ctx, z_out, dz->p, sizeof(double) * n);
         sync(ctx);
     });
 }
@@ -167,7 +168,7 @@ bsar_status bsar_refraction_points(bsar_ctx* ctx, const bsar_dem* dem, const dou
             launched(ctx, launch_refraction_points(d.view, a->as<double>(), b->as<double>(), n, n1, n2, solver, W,
                                                    o->as<double>(), ctx->stream),
                      "refraction points");
-        cuda_check(cudaMemcpyAsync(out, o->p, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream), "download");
+        copy_d2h(ctx, out, o->p, sizeof(double) * 3 * n);
         sync(ctx);
     });
 }
@@ -199,11 +200,11 @@ bsar_status bsar_slant_range_fermat(bsar_ctx* ctx, const bsar_dem* dem, const do
                                          dr->as<double>(), di->as<double>(), dv->as<double>(),
                                          dl ? dl->as<double>() : nullptr, ctx->stream),
                  "slant range");
-        cuda_check(cudaMemcpyAsync(ranges, dr->p, sizeof(double) * 4 * np, cudaMemcpyDeviceToHost, ctx->stream), "d2h");
-        cuda_check(cudaMemcpyAsync(ida, di->p, sizeof(double) * 3 * np, cudaMemcpyDeviceToHost, ctx->stream), "d2h");
-        cuda_check(cudaMemcpyAsync(volta, dv->p, sizeof(double) * 3 * np, cudaMemcpyDeviceToHost, ctx->stream), "d2h");
+        copy_d2h(ctx, ranges, dr->p, sizeof(double) * 4 * np);
+        copy_d2h(ctx, ida, di->p, sizeof(double) * 3 * np);
+        copy_d2h(ctx, volta, dv->p, sizeof(double) * 3 * np);
         if (refl)
-            cuda_check(cudaMemcpyAsync(refl, dl->p, sizeof(double) * 3 * np, cudaMemcpyDeviceToHost, ctx->stream), "d2h");
+            copy_d2h(ctx, refl, dl->p, sizeof(double) * 3 * np);
         sync(ctx);
     });
 }
@@ -216,12 +217,10 @@ bsar_status bsar_spline_upsample(bsar_ctx* ctx, const double* in, int64_t n, int
         // the reference indexes p[n-2] for every output (src/interpolation.cpp:22-25)
         if (n < 2) fail(BSAR_ERR_INVALID_ARG, "splineInterpolation needs at least 2 samples");
         if (!in || !out) fail(BSAR_ERR_INVALID_ARG, "NULL buffer");
-        auto di = dev_upload(ctx, in, sizeof(double2) * n * batch);
+        auto di = dev_upload(ctx, in, sizeof(double2) * n * batch, true);
         auto dout = dev_alloc(ctx, sizeof(double2) * n * factor * batch);
         launched(ctx, launch_spline(di->as<double2>(), n, batch, factor, dout->as<double2>(), ctx->stream), "spline");
-        cuda_check(cudaMemcpyAsync(out, dout->p, sizeof(double2) * n * factor * batch, cudaMemcpyDeviceToHost,
-                                   ctx->stream),
-                   "download");
+        copy_d2h(ctx, out, dout->p, sizeof(double2) * n * factor * batch);
         sync(ctx);
     });
 }
@@ -238,10 +237,10 @@ bsar_status bsar_fft(bsar_ctx* ctx, double* data, int64_t n, int64_t batch, int3
         }
         if (n > max_fft_len(8)) fail(BSAR_ERR_UNSUPPORTED, "FP64 FFT longer than %lld", (long long)max_fft_len(8));
         const void* tw = twiddles(ctx, n, 8);
-        auto d = dev_upload(ctx, data, sizeof(double2) * n * batch);
+        auto d = dev_upload(ctx, data, sizeof(double2) * n * batch, true);
         launched(ctx, launch_fft_rows(d->as<double2>(), batch, (int)n, ilog2(n), (const double2*)tw, inverse, ctx->stream),
                  "fft");
-        cuda_check(cudaMemcpyAsync(data, d->p, sizeof(double2) * n * batch, cudaMemcpyDeviceToHost, ctx->stream), "d2h");
+        copy_d2h(ctx, data, d->p, sizeof(double2) * n * batch);
         sync(ctx);
     });
 }
@@ -259,12 +258,10 @@ bsar_status bsar_fft_correlate(bsar_ctx* ctx, const double* signal, int64_t ns, 
         const void* tw = twiddles(ctx, P, 8);
         auto ds = dev_alloc(ctx, sizeof(double2) * std::max<int64_t>(ns, 1) * batch);
         if (ns > 0)
-            cuda_check(cudaMemcpyAsync(ds->p, signal, sizeof(double2) * ns * batch, cudaMemcpyHostToDevice, ctx->stream),
-                       "upload");
+            copy_h2d(ctx, ds->p, signal, sizeof(double2) * ns * batch, true);
         auto dr = dev_alloc(ctx, sizeof(double2) * std::max<int64_t>(nref, 1));
         if (nref > 0)
-            cuda_check(cudaMemcpyAsync(dr->p, reference, sizeof(double2) * nref, cudaMemcpyHostToDevice, ctx->stream),
-                       "upload");
+            copy_h2d(ctx, dr->p, reference, sizeof(double2) * nref);
         auto spec = dev_alloc(ctx, sizeof(double2) * P);
         auto dout = dev_alloc(ctx, sizeof(double2) * N * batch);
         launched(ctx, launch_ref_spectrum(dr->as<double2>(), (int)nref, (int)P, ilog2(P), tw, conjugate ? 1 : 0, spec->p,
@@ -283,7 +280,7 @@ bsar_status bsar_fft_correlate(bsar_ctx* ctx, const double* signal, int64_t ns, 
         a.factor = 0;
         a.out64 = dout->as<double2>();
         launched(ctx, launch_pulse_compress(a, ctx->stream), "correlate");
-        cuda_check(cudaMemcpyAsync(out, dout->p, sizeof(double2) * N * batch, cudaMemcpyDeviceToHost, ctx->stream), "d2h");
+        copy_d2h(ctx, out, dout->p, sizeof(double2) * N * batch);
         sync(ctx);
     });
 }
@@ -333,9 +330,7 @@ bsar_status bsar_scene_read_samples(bsar_ctx* ctx, bsar_scene_id id, double* out
     return guarded(ctx, [&] {
         Scene* s = get_scene(ctx, id);
         if (!out) fail(BSAR_ERR_INVALID_ARG, "NULL buffer");
-        cuda_check(cudaMemcpyAsync(out, s->samples->p, sizeof(double2) * s->np * s->ns, cudaMemcpyDeviceToHost,
-                                   ctx->stream),
-                   "download");
+        copy_d2h(ctx, out, s->samples->p, sizeof(double2) * s->np * s->ns);
         sync(ctx);
     });
 }
@@ -363,9 +358,7 @@ bsar_status bsar_scene_read_upsampled(bsar_ctx* ctx, bsar_scene_id id, double* o
         Scene* s = get_scene(ctx, id);
         if (!out) fail(BSAR_ERR_INVALID_ARG, "NULL buffer");
         if (!s->rc[BSAR_FP64].data) compress_scene(ctx, s, BSAR_FP64);
-        cuda_check(cudaMemcpyAsync(out, s->rc[BSAR_FP64].data->p, sizeof(double2) * s->np * s->nr,
-                                   cudaMemcpyDeviceToHost, ctx->stream),
-                   "download");
+        copy_d2h(ctx, out, s->rc[BSAR_FP64].data->p, sizeof(double2) * s->np * s->nr);
         sync(ctx);
     });
 }
@@ -380,15 +373,13 @@ bsar_status bsar_scene_read_stored(bsar_ctx* ctx, bsar_scene_id id, int32_t prec
         if (!rb.data) compress_scene(ctx, s, precision);
         const size_t n = (size_t)s->np * s->nr;
         if (precision == BSAR_FP64) {
-            cuda_check(cudaMemcpyAsync(out, rb.data->p, sizeof(double2) * n, cudaMemcpyDeviceToHost, ctx->stream),
-                       "download");
+            copy_d2h(ctx, out, rb.data->p, sizeof(double2) * n);
             sync(ctx);
             return;
         }
         if (precision == BSAR_MIXED) {
             std::vector<float2> h(n);
-            cuda_check(cudaMemcpyAsync(h.data(), rb.data->p, sizeof(float2) * n, cudaMemcpyDeviceToHost, ctx->stream),
-                       "download");
+            copy_d2h(ctx, h.data(), rb.data->p, sizeof(float2) * n);
             sync(ctx);
             for (size_t i = 0; i < n; i++) {
                 out[2 * i] = h[i].x;
@@ -398,10 +389,8 @@ bsar_status bsar_scene_read_stored(bsar_ctx* ctx, bsar_scene_id id, int32_t prec
         }
         std::vector<__half2> h(n);
         std::vector<float> sc(s->np);
-        cuda_check(cudaMemcpyAsync(h.data(), rb.data->p, sizeof(__half2) * n, cudaMemcpyDeviceToHost, ctx->stream),
-                   "download");
-        cuda_check(cudaMemcpyAsync(sc.data(), rb.scale->p, sizeof(float) * s->np, cudaMemcpyDeviceToHost, ctx->stream),
-                   "download");
+        copy_d2h(ctx, h.data(), rb.data->p, sizeof(__half2) * n);
+        copy_d2h(ctx, sc.data(), rb.scale->p, sizeof(float) * s->np);
         sync(ctx);
         for (size_t i = 0; i < n; i++) {
             const double f = sc[i / s->nr];
@@ -527,7 +516,7 @@ bsar_status bsar_backproject(bsar_ctx* ctx, bsar_scene_id id, const bsar_grid* g
         const int64_t nv = check_grid(g);
         auto img = dev_alloc(ctx, sizeof(double2) * nv);
         backproject(ctx, id, g, o, img->as<double2>());
-        cuda_check(cudaMemcpyAsync(image_out, img->p, sizeof(double2) * nv, cudaMemcpyDeviceToHost, ctx->stream), "d2h");
+        copy_d2h(ctx, image_out, img->p, sizeof(double2) * nv);
         sync(ctx);
         check_device_status(ctx);
     });
@@ -542,7 +531,7 @@ bsar_status bsar_backproject_range(bsar_ctx* ctx, bsar_scene_id id, const bsar_g
         auto img = dev_alloc(ctx, sizeof(double2) * nv);
         cuda_check(cudaMemsetAsync(img->p, 0, sizeof(double2) * nv, ctx->stream), "clear image");
         backproject(ctx, id, g, o, img->as<double2>(), v_begin, v_count);
-        cuda_check(cudaMemcpyAsync(image_out, img->p, sizeof(double2) * nv, cudaMemcpyDeviceToHost, ctx->stream), "d2h");
+        copy_d2h(ctx, image_out, img->p, sizeof(double2) * nv);
         sync(ctx);
         check_device_status(ctx);
     });

@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "kernels.hpp"
+#include "staging.hpp"
 
 using namespace bsar;
 
@@ -100,6 +101,9 @@ struct bsar_ctx {
     // taken with `use_pool` cleared.
     cudaMemPool_t pool = nullptr;
     bool use_pool = false;
+    // large copies between pageable memory and the device (made at the first one)
+    std::unique_ptr<Stager> stager;
+    bool no_stager = false;
     // polls of the mixed kernel's bounded DEM-tile wait (bsar_set_tile_wait_limit)
     int64_t tile_wait_polls = kDefaultTileWaitPolls;
 };
@@ -145,10 +149,39 @@ struct DevBuf {
 
 inline std::unique_ptr<DevBuf> dev_alloc(bsar_ctx* ctx, size_t n) { return std::make_unique<DevBuf>(ctx, n); }
 
-inline std::unique_ptr<DevBuf> dev_upload(bsar_ctx* ctx, const void* host, size_t n)
+// Copies on the context's stream.  Both read or write the caller's pageable memory before
+// they return (a small download, and one into pinned memory, only after a synchronize).
+inline Stager* stager_for(bsar_ctx* ctx, const void* host, size_t n, size_t least)
+{
+    if (!Stager::wanted(host, n, least) || ctx->no_stager) return nullptr;
+    if (!ctx->stager) {
+        ctx->stager = Stager::make(ctx->device);
+        ctx->no_stager = !ctx->stager;
+    }
+    return ctx->stager.get();
+}
+
+// back: the call downloads as much soon after.
+inline void copy_h2d(bsar_ctx* ctx, void* dev, const void* host, size_t n, bool back = false)
+{
+    Stager* s = stager_for(ctx, host, n, back ? Stager::kMinUploadBack : Stager::kMinUpload);
+    cuda_check(s ? s->upload(dev, host, n, ctx->stream)
+                 : cudaMemcpyAsync(dev, host, n, cudaMemcpyHostToDevice, ctx->stream),
+               "upload");
+}
+
+inline void copy_d2h(bsar_ctx* ctx, void* host, const void* dev, size_t n)
+{
+    Stager* s = stager_for(ctx, host, n, Stager::kMinDownload);
+    cuda_check(s ? s->download(host, dev, n, ctx->stream)
+                 : cudaMemcpyAsync(host, dev, n, cudaMemcpyDeviceToHost, ctx->stream),
+               "download");
+}
+
+inline std::unique_ptr<DevBuf> dev_upload(bsar_ctx* ctx, const void* host, size_t n, bool back = false)
 {
     auto b = dev_alloc(ctx, n);
-    if (n) cuda_check(cudaMemcpyAsync(b->p, host, n, cudaMemcpyHostToDevice, ctx->stream), "upload");
+    if (n) copy_h2d(ctx, b->p, host, n, back);
     return b;
 }
 
