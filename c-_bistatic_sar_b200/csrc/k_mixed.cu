@@ -1,7 +1,7 @@
 // k_mixed.cu -- the mixed-precision back-projection kernel.
 //
 // One thread per voxel; the 32 voxels of a warp are a compact block of the grid
-// (compact_voxel) and walk the pulses in order, in blocks of up to 16 consecutive pulses
+// (compact_voxel) and walk the pulses in order, in blocks of up to 32 consecutive pulses
 // whose antennas lie close together.
 //
 // Per pulse block and leg (Tx -> voxel, voxel -> Rx), by the warp together:
@@ -23,13 +23,15 @@
 // A block's legs are solved leg by leg over its pulses, then all its delays, gathers and
 // sums run in one short loop: the warps of an SM stay in small pieces of code.
 //
-// What bounds it: instruction issue and fetch (47 % of issue slots on the medium scene; the
-// rough DEM leaves about a quarter of the leg solves to polish).  Against the scan of every
-// lane's own window with per-lane lower bounds, one B200: 161 x 161 x 81 voxels x 1024
-// pulses on a 0.25 m DEM 528 -> 88 ms; 256 x 256 x 8 x 2048 on 0.125 m 647 -> 48 ms;
-// 97 x 83 x 11 x 701 on 0.2 m (no compile-time scan width) 74.7 -> 5.8 ms.  Block length
-// (kBlockSlope) 0.006 / 0.0125 / 0.025 / 0.05: 25.4 / 24.1 / 26.4 / 30.4 ms on 16 slices of
-// the medium grid; 5 CTAs per SM instead of 4 (96 registers): 15 % slower.
+// What bounds it: instruction fetch.  On the medium scene the rough DEM leaves a quarter of
+// the leg solves to polish, so a warp goes through list building, polish, final step and
+// gathers, some 60 KB of code, and warps wait for instructions longer than for anything
+// else; unrolling the gather loop or inlining rare branches made every scene slower, and
+// three CTAs per SM (168 registers) run faster than four (98.7 against 109.4 ms on 161 x 161
+// x 81 voxels x 1024 pulses) or two.  Rare work is out of line.  Against the scan of every
+// lane's own window with per-lane lower bounds, with pulse compression, one B200: the medium
+// scene 513 ms before, 73 ms; 256 x 256 x 8 x 2048 on a 0.125 m DEM 618, 38 ms; 97 x 83 x 11
+// x 701 on 0.2 m (no compile-time scan width) 72, 5 ms.
 //
 // DEM tile: for wide scans (25 x 25 and generic widths) every CTA stages a TI x TJ FP32
 // tile of the DEM around its voxels (shifted by the scene's mean crossing offset) into
@@ -52,7 +54,7 @@ namespace bsar {
 
 namespace {
 
-constexpr int TI = kMixedTileI;    // tile columns (x); 272 B rows, a multiple of 16 B
+constexpr int TI = kMixedTileI;    // tile columns (x); 176 B rows, a multiple of 16 B
 constexpr int TJ = kMixedTileJ;    // tile rows (y)
 constexpr long kWaitSpins = 1L << 24;
 
@@ -442,7 +444,7 @@ struct Leg {
 // Window centre of a leg's node scan: the node nearest the flat start.  A start within
 // rounding distance of a cell boundary is redone in FP64 so both forms scan the same
 // window.
-__device__ __forceinline__ int2 start_node(const DemView& d, const MixedCtx& m, const Leg& l, const VoxelStart& vs)
+__device__ __noinline__ int2 start_node(const DemView d, const MixedCtx m, const Leg l, const VoxelStart vs)
 {
     const float* Lp = l.g_lower ? l.G32 : l.E32;      // the lower endpoint is normally the voxel itself
     const float* Up = l.g_lower ? l.E32 : l.G32;
@@ -760,23 +762,23 @@ __device__ __forceinline__ MixedCtx req_ctx(const MixedReq& r)
 }
 
 // Shared memory of one warp.  A pulse block has lists for both legs or none: the lists (or
-// their tables) and the block's paths share their place with the table of the scans that
-// rank every node, which take one pulse at a time and keep its paths in the last row.
+// their tables) share their place with the table of the scans that rank every node.
+constexpr int kPathPulses = 8;               // pulses whose legs are solved before they are summed
+// Length of the pulse blocks (pulse_block): 0.011 / 0.013 / 0.016: 37.3 / 36.0 / 34.8 ms on a
+// served burst, 3.55 / 3.58 / 3.47 ms on the small scene, 2.57 / 2.55 / 2.59 ms on an FP16
+// slice; the medium and large scenes stay within 1 %.
+constexpr float kBlockSlope = 0.016f;
+
 template <int WT> struct WarpShared {
     union {
-        struct {
-            BlockLists l;
-            double path[kBlockPulses][32];   // per pulse and lane: the paths of the legs solved one by one
-        } b;
+        BlockLists l;
         float2 table[TableRows<WT>::v * TBJ];
     } u;
+    double path[kPathPulses][32];            // per pulse and lane: the paths of the legs solved one by one
     double ref_L[kBlockPulses];              // the block's anchors
     float4 anchor[kBlockPulses];             // fast-time bin fraction, reduced phase, FP16 scale, bin (int)
     LegList h[2];
 };
-static_assert(sizeof(float2) * TableRows<12>::v * TBJ + 32 * sizeof(double) <= sizeof(float4) * 2 * kListCap +
-                                                                               32 * sizeof(double) * kBlockPulses,
-              "the last row of paths lies beyond the table");
 
 // One voxel of a request over pulses [p0, p1) (k: index in the request's voxel range;
 // k >= v_count repeats the last voxel without storing it, so whole warps stay active).
@@ -803,8 +805,8 @@ __device__ __forceinline__ void voxel_mixed(const BpArgs& a, const MixedCtx& m, 
     float accr = 0.f, acci = 0.f, cmpr = 0.f, cmpi = 0.f;
     int block_end;
     for (int i = CH ? p0 : 0; i < np; i = block_end) {
-        const int n = pulse_block(m, TileHeights(m, T), a.dem, ws->u.b.l, ws->h, a.tx, a.rx, i, np, m.ox, m.oy, P, P32,
-                                  vs.h32, wv, a.n1, a.n2, a.W, m.lists != 0);
+        const int n = pulse_block(m, TileHeights(m, T), a.dem, ws->u.l, ws->h, a.tx, a.rx, i, np, m.ox, m.oy, P, P32,
+                                  vs.h32, wv, a.n1, a.n2, a.W, kBlockSlope, m.lists != 0);
         block_end = i + n;
         if (lane < n) {
             ws->ref_L[lane] = __ldg(a.ref_L + i + lane);
@@ -816,9 +818,9 @@ __device__ __forceinline__ void voxel_mixed(const BpArgs& a, const MixedCtx& m, 
         const int hm0 = ws->h[0].m, hm1 = ws->h[1].m;
         // legs whose listed nodes are all pinned: the paths come from the tables alone
         const int m0 = all_pinned(ws->h[0]) ? hm0 : 0, m1 = all_pinned(ws->h[1]) ? hm1 : 0;
-        const int step = hm0 < 0 ? 1 : block_end - i;      // no lists: one pulse at a time
-        for (int b = i; b < block_end; b += step) {
-            double* path = hm0 < 0 ? ws->u.b.path[kBlockPulses - 1] : ws->u.b.path[0];
+        double* path = ws->path[0];
+        for (int b = i; b < block_end; b += kPathPulses) {
+            const int step = min(kPathPulses, block_end - b);
             // per-pulse legs: n1*r1Tx + n2*r2Tx (Tx -> voxel) + n2*r2Rx + n1*r1Rx (voxel -> Rx);
             // the legs to solve, one after the other over the block's pulses
 #pragma unroll 1
@@ -845,7 +847,7 @@ __device__ __forceinline__ void voxel_mixed(const BpArgs& a, const MixedCtx& m, 
                     if (hm > 0 && mode == (kCore | kTables)) {
                         int c;
                         known = true;
-                        L = table_min(ws->u.b.l.tab[leg], hm, p - i, lane, c);
+                        L = table_min(ws->u.l.tab[leg], hm, p - i, lane, c);
                         solved = (H->pinned >> c) & 1;
                         node = H->node[c];
                     }
@@ -860,11 +862,11 @@ __device__ __forceinline__ void voxel_mixed(const BpArgs& a, const MixedCtx& m, 
                             const Leg lc = l;
                             node = scan_warp<WT>(a.dem, m, T, ws->u.table, lc, vs, a.W);
                         } else if (!(mode & kTables)) {
-                            node = rank_list(a.dem, m, ws->u.b.l.list[leg], *H, l, vs, a.W);
+                            node = rank_list(a.dem, m, ws->u.l.list[leg], *H, l, vs, a.W);
                         } else if (!(mode & kCore)) {
                             // a listed node may lie outside this solve's window
                             const int2 st = start_node(a.dem, m, l, vs);
-                            const NodeTables* t = &ws->u.b.l.tab[leg];
+                            const NodeTables* t = &ws->u.l.tab[leg];
                             double v = INFINITY;
                             int c = 0;
 #pragma unroll 1
@@ -890,8 +892,8 @@ __device__ __forceinline__ void voxel_mixed(const BpArgs& a, const MixedCtx& m, 
                 const int q0 = p - i;
                 double L = (m0 && m1) ? 0.0 : path[(p - b) * 32 + lane];
                 int c;
-                if (m0) L = __dadd_rn(L, table_min(ws->u.b.l.tab[0], m0, q0, lane, c));
-                if (m1) L = __dadd_rn(L, table_min(ws->u.b.l.tab[1], m1, q0, lane, c));
+                if (m0) L = __dadd_rn(L, table_min(ws->u.l.tab[0], m0, q0, lane, c));
+                if (m1) L = __dadd_rn(L, table_min(ws->u.l.tab[1], m1, q0, lane, c));
                 const float dL = (float)(L - ws->ref_L[q0]);
                 const float4 an = ws->anchor[q0];
                 // fast-time bin: integer anchor + FP32 offset
@@ -990,7 +992,7 @@ __device__ __forceinline__ void reduce_chunks(const BpArgs& a, const double2* __
 template <int WT> struct StagesTile { static constexpr bool v = WT == 0 || WT >= 12; };
 
 template <int WT, bool CH>
-__global__ void __launch_bounds__(128, 4) k_bp_mixed(MixedBatch b)
+__global__ void __launch_bounds__(128, 3) k_bp_mixed(MixedBatch b)
 {
     constexpr bool kTile = StagesTile<WT>::v;
     __shared__ alignas(128) float tile_s[kTile ? TI * TJ : 32];
@@ -1140,13 +1142,13 @@ cudaError_t launch_refraction_mixed(const DemView& d, int pitch, const double* p
     return cudaGetLastError();
 }
 
-// Shared-memory carve-out for 4 resident CTAs per SM (DEM tile + 4 warp tables each),
+// Shared-memory carve-out for 3 resident CTAs per SM (DEM tile + 4 warps' lists each),
 // set once per device; the rest of the unified L1 stays cache for the sample gathers.
 template <int WT, bool CH> static void set_carveout()
 {
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, k_bp_mixed<WT, CH>) != cudaSuccess) return;
-    const double need = 4.0 * (double)(fa.sharedSizeBytes + 1024);
+    const double need = 3.0 * (double)(fa.sharedSizeBytes + 1024);
     int pct = (int)(100.0 * need / (228.0 * 1024.0)) + 1;
     pct = pct > 100 ? 100 : pct;
     cudaFuncSetAttribute(k_bp_mixed<WT, CH>, cudaFuncAttributePreferredSharedMemoryCarveout, pct);

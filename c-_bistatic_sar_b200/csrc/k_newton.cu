@@ -1,7 +1,7 @@
 // k_newton.cu -- FP64 back-projection with the Newton solver and per-pulse legs.
 //
 // The layout of the mixed kernel (k_mixed.cu): one thread per voxel, a warp's 32 voxels a
-// compact block of the grid, pulses in blocks of up to 16 whose antennas lie close together,
+// compact block of the grid, pulses in blocks of up to 32 whose antennas lie close together,
 // and per block and leg one candidate list of the DEM nodes that can win the node scan of
 // any of its (voxel, pulse) pairs (node_lists.cuh; the lists' bounds are FP32 with margins,
 // every path, ranking, Newton step, delay, phase and sum here is FP64).  Lists of up to four
@@ -183,9 +183,12 @@ __device__ __forceinline__ double polish64(const DemView& d, const ListGrid& m, 
     return best;
 }
 
+constexpr int kPathPulses = 16;         // pulses whose legs are solved before they are summed
+constexpr float kBlockSlope = 0.013f;   // length of the pulse blocks (pulse_block); 0.016: 4 % slower
+
 struct NewtonWarp {
     BlockLists l;
-    double path[kBlockPulses][32];
+    double path[kPathPulses][32];       // the paths of the legs solved one by one
     LegList h[2];
 };
 
@@ -223,89 +226,92 @@ __global__ void __launch_bounds__(32 * WPC, WPC == 4 ? 3 : 16 / WPC) k_bp_newton
     int n;
     for (int i = p0; i < p1; i += n) {
         n = pulse_block(m, zat, d, ws->l, ws->h, a.tx, a.rx, i, p1, d.x0, d.y0, P, P32, (float)h64, wv, a.n1, a.n2, a.W,
-                        true);
+                        kBlockSlope, true);
         const int m0 = all_pinned(ws->h[0]) ? ws->h[0].m : 0, m1 = all_pinned(ws->h[1]) ? ws->h[1].m : 0;
-        // the legs to solve, one after the other over the block's pulses
+        for (int b = 0; b < n; b += kPathPulses) {
+            const int step = min(kPathPulses, n - b);
+            // the legs to solve, one after the other over the block's pulses
 #pragma unroll 1
-        for (int leg = m0 ? 1 : 0; leg < (m1 ? 1 : 2); leg++) {
-            const LegList* H = &ws->h[leg];
-            const int hm = H->m, mode = H->mode;
-            Leg64 l;
+            for (int leg = m0 ? 1 : 0; leg < (m1 ? 1 : 2); leg++) {
+                const LegList* H = &ws->h[leg];
+                const int hm = H->m, mode = H->mode;
+                Leg64 l;
 #pragma unroll
-            for (int c = 0; c < 3; c++) l.G[c] = P[c];
-            l.nE = a.n1;
-            l.nG = a.n2;
-            l.g_lower = lower_is_voxel((float)a.n1, (float)a.n2, leg == 0);
+                for (int c = 0; c < 3; c++) l.G[c] = P[c];
+                l.nE = a.n1;
+                l.nG = a.n2;
+                l.g_lower = lower_is_voxel((float)a.n1, (float)a.n2, leg == 0);
 #pragma unroll 1
-            for (int q = 0; q < n; q++) {
-                double L = 0.0;
-                int2 node = make_int2(0, 0);
-                bool solved = false;
-                if (hm > 0 && mode == (kCore | kTables)) {
-                    int c;
-                    L = table_min(ws->l.tab[leg], hm, q, lane, c);
-                    solved = (H->pinned >> c) & 1;
-                    node = H->node[c];
-                }
-                if (!solved) {
-                    const double* tr = (leg ? a.rx : a.tx) + 3 * (i + q);
-#pragma unroll
-                    for (int c = 0; c < 3; c++) l.E[c] = __ldg(tr + c);
-                    if (hm < 0) {
-                        node = scan_all64(d, l, h64, a.W);
-                    } else if (!(mode & kTables)) {
-                        node = rank_list64(d, ws->l.list[leg], *H, l, h64, a.W);
-                    } else if (!(mode & kCore)) {
-                        // a listed node may lie outside this solve's window
-                        const int2 st = start_node64(d, l, h64);
-                        const NodeTables* t = &ws->l.tab[leg];
-                        double v = INFINITY;
-                        int c = 0;
-#pragma unroll 1
-                        for (int k = 0; k < hm; k++) {
-                            const int2 nd = H->node[k];
-                            const double u = __dadd_rn(t->E[k][q], t->G[k][lane]);
-                            if (u < v && abs(nd.x - st.x) <= a.W && abs(nd.y - st.y) <= a.W) {
-                                v = u;
-                                c = k;
-                            }
-                        }
+                for (int q = b; q < b + step; q++) {
+                    double L = 0.0;
+                    int2 node = make_int2(0, 0);
+                    bool solved = false;
+                    if (hm > 0 && mode == (kCore | kTables)) {
+                        int c;
+                        L = table_min(ws->l.tab[leg], hm, q, lane, c);
+                        solved = (H->pinned >> c) & 1;
                         node = H->node[c];
                     }
-                    L = polish64(d, m, l, node.x, node.y);
-                }
-                double* path = &ws->path[q][lane];
-                *path = (leg && !m0) ? *path + L : L;
-            }
-        }
-        // delays, gathers and sums of the block's pulses
+                    if (!solved) {
+                        const double* tr = (leg ? a.rx : a.tx) + 3 * (i + q);
+#pragma unroll
+                        for (int c = 0; c < 3; c++) l.E[c] = __ldg(tr + c);
+                        if (hm < 0) {
+                            node = scan_all64(d, l, h64, a.W);
+                        } else if (!(mode & kTables)) {
+                            node = rank_list64(d, ws->l.list[leg], *H, l, h64, a.W);
+                        } else if (!(mode & kCore)) {
+                            // a listed node may lie outside this solve's window
+                            const int2 st = start_node64(d, l, h64);
+                            const NodeTables* t = &ws->l.tab[leg];
+                            double v = INFINITY;
+                            int c = 0;
 #pragma unroll 1
-        for (int q = 0; q < n; q++) {
-            double L = (m0 && m1) ? 0.0 : ws->path[q][lane];
-            int c;
-            if (m0) L += table_min(ws->l.tab[0], m0, q, lane, c);
-            if (m1) L += table_min(ws->l.tab[1], m1, q, lane, c);
-            const double t_val = inv_c * L;                          // proc_test_script.cpp:565
-            const double b = (1.0 + t_val * a.fs_eff) - 1.0;         // :569, :593
-            // (int)floor(b) >= 0 && (int)ceil(b) < nr  <=>  0 <= b <= nr - 1 (NaN fails both)
-            if (b >= 0.0 && b <= (double)(a.nr - 1)) {
-                const double lo_d = floor(b);
-                const int lo = (int)lo_d;                            // nr <= 2^30
-                const double qf = b - lo_d;
-                const double2* row = a.rc64 + (int64_t)(i + q) * a.nr + lo;
-                const double2 s0 = __ldg(row);
-                double vr = s0.x, vi = s0.y;
-                if (qf != 0.0) {
-                    const double2 s1 = __ldg(row + 1);
-                    vr = (1.0 - qf) * s0.x + qf * s1.x;              // :635
-                    vi = (1.0 - qf) * s0.y + qf * s1.y;
+                            for (int k = 0; k < hm; k++) {
+                                const int2 nd = H->node[k];
+                                const double u = __dadd_rn(t->E[k][q], t->G[k][lane]);
+                                if (u < v && abs(nd.x - st.x) <= a.W && abs(nd.y - st.y) <= a.W) {
+                                    v = u;
+                                    c = k;
+                                }
+                            }
+                            node = H->node[c];
+                        }
+                        L = polish64(d, m, l, node.x, node.y);
+                    }
+                    double* path = &ws->path[q - b][lane];
+                    *path = (leg && !m0) ? *path + L : L;
                 }
-                // carrier phase (:573, :638) in turns, reduced before the sine
-                const double turns = rint(L * inv_lambda);
-                double sn, cs;
-                sincospi(2.0 * (fma(-turns, a.lambda, L) * inv_lambda), &sn, &cs);
-                accr += vr * cs - vi * sn;
-                acci += vr * sn + vi * cs;
+            }
+            // delays, gathers and sums of the block's pulses
+#pragma unroll 1
+            for (int q = b; q < b + step; q++) {
+                double L = (m0 && m1) ? 0.0 : ws->path[q - b][lane];
+                int c;
+                if (m0) L += table_min(ws->l.tab[0], m0, q, lane, c);
+                if (m1) L += table_min(ws->l.tab[1], m1, q, lane, c);
+                const double t_val = inv_c * L;                          // proc_test_script.cpp:565
+                const double bin = (1.0 + t_val * a.fs_eff) - 1.0;         // :569, :593
+                // (int)floor(bin) >= 0 && (int)ceil(bin) < nr  <=>  0 <= bin <= nr - 1 (NaN fails both)
+                if (bin >= 0.0 && bin <= (double)(a.nr - 1)) {
+                    const double lo_d = floor(bin);
+                    const int lo = (int)lo_d;                            // nr <= 2^30
+                    const double qf = bin - lo_d;
+                    const double2* row = a.rc64 + (int64_t)(i + q) * a.nr + lo;
+                    const double2 s0 = __ldg(row);
+                    double vr = s0.x, vi = s0.y;
+                    if (qf != 0.0) {
+                        const double2 s1 = __ldg(row + 1);
+                        vr = (1.0 - qf) * s0.x + qf * s1.x;              // :635
+                        vi = (1.0 - qf) * s0.y + qf * s1.y;
+                    }
+                    // carrier phase (:573, :638) in turns, reduced before the sine
+                    const double turns = rint(L * inv_lambda);
+                    double sn, cs;
+                    sincospi(2.0 * (fma(-turns, a.lambda, L) * inv_lambda), &sn, &cs);
+                    accr += vr * cs - vi * sn;
+                    acci += vr * sn + vi * cs;
+                }
             }
         }
     }

@@ -139,8 +139,8 @@ inline __host__ __device__ void compact_voxel(int nx, int ny, int nz, int64_t k,
 
 // DEM tile of the mixed kernel (nodes): TMA box dims.  The x extent is a multiple of
 // 4 floats so every tiled copy row is a multiple of 16 bytes.
-constexpr int kMixedTileI = 68;
-constexpr int kMixedTileJ = 64;
+constexpr int kMixedTileI = 44;
+constexpr int kMixedTileJ = 40;
 
 // One image-formation request of the mixed kernel, as it sits in device memory: the
 // back-projection arguments, the FP32 DEM view and the tensor map of that DEM.

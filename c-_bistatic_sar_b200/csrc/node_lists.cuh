@@ -230,23 +230,40 @@ __device__ __forceinline__ unsigned patch_skips(const NodePatch& p, const ListGr
     return skip & todo;
 }
 
+// The path at (u, v) on facet (fi, fj); on a node, that node's path.  Out of line: the final
+// step rarely needs it.
+static __device__ __noinline__ double facet_path64(const DemView d, int fi, int fj, double Ex, double Ey, double Ez, double Gx,
+                                            double Gy, double Gz, double nE, double nG, double u, double v)
+{
+    const double E[3] = {Ex, Ey, Ez}, G[3] = {Gx, Gy, Gz};
+    Facet64 F;
+    facet_load(d, fi, fj, F);
+    double x = F.x0 + u * F.dx, y = F.y0 + v * F.dy, z = F.z00 + F.b * u + F.c * v + F.e * u * v;
+    if ((u == 0.0 || u == 1.0) && (v == 0.0 || v == 1.0)) {
+        const int i = fi + (int)u, j = fj + (int)v;
+        x = __ldg(d.xv + i);
+        y = __ldg(d.yv + j);
+        z = __ldg(d.z + (int64_t)j * d.nx + i);
+    }
+    return path64(leg_len64(x, y, z, E), leg_len64(x, y, z, G), nE, nG);
+}
+
 // The path after the FP64 final step from (u, v) on facet (fi, fj), idx_, idy: 1 / the
 // facet's extents.  A step below half a millimetre moves the path by its second-order
 // expansion (the third order is below 1e-11 m); a result on a node is that node's path.
-__device__ __forceinline__ double final_path64(const DemView& d, int fi, int fj, const double A[3], const double B[3],
-                                               double na, double nb, double idx_, double idy, double u, double v)
+__device__ __forceinline__ double final_path64(const DemView& d, int fi, int fj, const double E[3], const double G[3],
+                                               double nE, double nG, double idx_, double idy, double u, double v)
 {
     Facet64 F;
     facet_load(d, fi, fj, F);
     double L, gx, gy, hxx, hyy, hxy;
     const double u0 = u, v0 = v;
-    facet_newton64(F, A, B, na, nb, idx_, idy, u, v, L, gx, gy, hxx, hyy, hxy);
-    if ((u == 0.0 || u == 1.0) && (v == 0.0 || v == 1.0)) return node_l64(d, fi + (int)u, fj + (int)v, A, B, na, nb);
+    facet_newton64(F, E, G, nE, nG, idx_, idy, u, v, L, gx, gy, hxx, hyy, hxy);
     const double du = (u - u0) * F.dx, dv = (v - v0) * F.dy;
-    if (fabs(du) + fabs(dv) < 5e-4) return L + (gx * du + gy * dv + 0.5 * (hxx * du * du + hyy * dv * dv) + hxy * du * dv);
-    const double x = F.x0 + u * F.dx, y = F.y0 + v * F.dy;
-    const double h = F.z00 + F.b * u + F.c * v + F.e * u * v;
-    return path64(leg_len64(x, y, h, A), leg_len64(x, y, h, B), na, nb);
+    const bool node = (u == 0.0 || u == 1.0) && (v == 0.0 || v == 1.0);
+    if (!node && fabs(du) + fabs(dv) < 5e-4)
+        return L + (gx * du + gy * dv + 0.5 * (hxx * du * du + hyy * dv * dv) + hxy * du * dv);
+    return facet_path64(d, fi, fj, E[0], E[1], E[2], G[0], G[1], G[2], nE, nG, u, v);
 }
 
 // Flat-interface start (FP32) of the path Up (index nu) -> Lp (index nl) over the height h0:
@@ -269,7 +286,7 @@ __device__ __forceinline__ FlatStart flat_start32(const float Up[3], const float
         float ha = fabsf(Up[2] - h0), hb = fabsf(Lp[2] - h0);
         float s = fminf(fmaxf(__fdividef(D * ha, ha + hb + 1e-30f), 0.f), D);
         float before = s;
-#pragma unroll
+#pragma unroll 1
         for (int it = 0; it < kFlatIters; it++) {
             float q1 = s * s + ha * ha, r = D - s, q2 = r * r + hb * hb;
             float i1 = rsqrtf(q1), i2 = rsqrtf(q2);
@@ -322,8 +339,8 @@ __device__ __forceinline__ bool lower_is_voxel(float nE, float nG, bool to_voxel
 // No list (m = -1): antenna on the side of the larger index, start not converged,
 // intersection empty, or more nodes than the list holds; those blocks scan every window
 // node (scan_warp), as the exhaustive flag does.
-constexpr int kListCap = 96;
-constexpr int kBlockPulses = 16;    // longest pulse block
+constexpr int kListCap = 128;
+constexpr int kBlockPulses = 32;    // longest pulse block
 
 constexpr int kCore = 1, kTables = 2;
 // Lists of at most kTabled nodes carry their FP64 legs (node_tables).
@@ -351,7 +368,7 @@ __device__ __forceinline__ unsigned ordered_bits(float f)   // unsigned order = 
     return u ^ ((u >> 31) ? 0xffffffffu : 0x80000000u);
 }
 
-// gap(N) - slack(N) of the node offset (x, y, z), and the gap itself.
+// A block's centres and S: the gap of a node and its test against the slack.
 struct GapRef {
     float E[3], G[3];     // block and warp centres
     float S[3], eS, gS;   // S and its distances |S - Ec|, |S - Gc|
@@ -371,7 +388,11 @@ __device__ __forceinline__ void gap_set(GapRef& g, float x, float y, float z)
     g.gS = q * rsqrtf(q);
 }
 
-__device__ __forceinline__ float gap_of(const GapRef& g, float x, float y, float z, float& gap)
+// Whether the node may win somewhere in the block, gap <= thr + slack, and its gap.  With
+// slack = |N - S| (cE / dE + cG / dG) the test is squared and multiplied out: the node ranking
+// is bound by the special-function unit, which here takes the two distances' square roots
+// only.
+__device__ __forceinline__ bool gap_keep(const GapRef& g, float x, float y, float z, float thr, float& gap)
 {
     float dx = x - g.E[0], dy = y - g.E[1], dz = z - g.E[2];
     float q = fmaf(dz, dz, fmaf(dx, dx, dy * dy));
@@ -380,14 +401,16 @@ __device__ __forceinline__ float gap_of(const GapRef& g, float x, float y, float
     q = fmaf(dz, dz, fmaf(dx, dx, dy * dy));
     const float v = q * rsqrtf(q);
     dx = x - g.S[0], dy = y - g.S[1], dz = z - g.S[2];
-    q = fmaf(dz, dz, fmaf(dx, dx, dy * dy));
-    const float nS = q * rsqrtf(fmaxf(q, 1e-30f));
+    const float s2 = fmaf(dz, dz, fmaf(dx, dx, dy * dy));
     gap = fmaf(g.re, e - g.eS, v - g.gS);
-    // denominators at or below zero (a voxel or antenna among the nodes): keep the node
-    const float kE = __fdividef(g.cE, fmaxf(e + g.eS - g.rE2, 1e-6f));
-    const float kG = __fdividef(g.cG, fmaxf(v + g.gS - g.rG2, 1e-6f));
-    return gap - nS * (kE + kG);
+    // at or below zero (a voxel or antenna among the nodes): the node is kept
+    const float dE = fmaxf(e + g.eS - g.rE2, 1e-6f), dG = fmaxf(v + g.gS - g.rG2, 1e-6f);
+    const float t = gap - thr, a = t * (dE * dG), b = fmaf(g.cE, dG, g.cG * dE);
+    return t <= 0.0f || a * a <= s2 * (b * b) * 1.00001f;
 }
+
+// (float)i for 0 <= i < 2^23 without the conversion unit.
+__device__ __forceinline__ float small_float(int i) { return __int_as_float(0x4b000000 | i) - 8388608.0f; }
 
 // Builds one leg's list for the block (all 32 lanes call).  E: the block's centre antenna,
 // rEh / rEz / rE the antennas' largest horizontal, vertical and 3-D distance from it, dh0
@@ -404,7 +427,13 @@ __device__ __forceinline__ void build_list(const ListGrid& m, Z zat, float4* lis
     int si = H->si, sj = H->sj;
     __syncwarp();                                  // readers of the previous list are done
     // window centres of the block
-    const FlatStart f = lp_is_g ? flat_start32(E, G, nE, nG, h0) : flat_start32(G, E, nG, nE, h0);
+    float up[3], lo[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        up[c] = lp_is_g ? E[c] : G[c];
+        lo[c] = lp_is_g ? G[c] : E[c];
+    }
+    const FlatStart f = flat_start32(up, lo, lp_is_g ? nE : nG, lp_is_g ? nG : nE, h0);
     const float hE = fabsf(E[2] - h0), hG = fabsf(G[2] - h0), hEm = hE - rEz - dh0;
     const float kappa = __fdividef(nE * hG, nE * hG + nG * hEm);
     const float D = f.D + rEh;
@@ -444,6 +473,9 @@ __device__ __forceinline__ void build_list(const ListGrid& m, Z zat, float4* lis
     g.rG2 = 2.0f * rG;
     gap_set(g, (float)si * m.stepx, (float)sj * m.stepy, zat(si, sj));
     const unsigned below = (1u << lane) - 1u;
+    // lane / nj and 32 / nj (small integers: exact in FP32)
+    const float inj = __fdividef(1.0f, (float)nj);
+    const int li = (int)((small_float(lane) + 0.5f) * inj), di = (int)(32.5f * inj), dj = 32 - di * nj;
     int cnt = 0;
     bool outside = false;
 #pragma unroll 1
@@ -451,20 +483,20 @@ __device__ __forceinline__ void build_list(const ListGrid& m, Z zat, float4* lis
         const float thr = kTieM / nG + 1e-4f + 2e-6f * (g.eS + g.gS) + 5e-7f * m.extent;
         float best = INFINITY;
         int bij = 0;
+        int i = ua + li, j = va + lane - li * nj;
         cnt = 0;
         outside = false;
-        int i = ua + lane / nj, j = va + lane % nj;
 #pragma unroll 1
         for (int base = 0; base < n; base += 32) {
             const bool in = base + lane < n;
             bool keep = false;
             float x = 0.f, y = 0.f, z = 0.f;
             if (in) {
-                x = (float)i * m.stepx;
-                y = (float)j * m.stepy;
+                x = small_float(i) * m.stepx;
+                y = small_float(j) * m.stepy;
                 z = zat(i, j);
                 float gap;
-                keep = gap_of(g, x, y, z, gap) <= thr;
+                keep = gap_keep(g, x, y, z, thr, gap);
                 const bool core = i >= ca && i <= cb && j >= da && j <= db;
                 outside |= keep && !core;
                 if (core && gap < best) {
@@ -476,8 +508,9 @@ __device__ __forceinline__ void build_list(const ListGrid& m, Z zat, float4* lis
             const int pos = cnt + __popc(bal & below);
             if (keep && pos < kListCap) list[pos] = list_entry(x, y, z, i - ua, j - va);
             cnt += __popc(bal);
-            j += 32;
-            while (j > vb) {
+            i += di;
+            j += dj;
+            if (j > vb) {
                 j -= nj;
                 i++;
             }
@@ -492,7 +525,7 @@ __device__ __forceinline__ void build_list(const ListGrid& m, Z zat, float4* lis
         si = ni;
         sj = nj2;
         if (same || cnt <= 1) break;
-        gap_set(g, (float)si * m.stepx, (float)sj * m.stepy, zat(si, sj));
+        gap_set(g, small_float(si) * m.stepx, small_float(sj) * m.stepy, zat(si, sj));
         if (cnt <= kListCap) {
             // list against the better S, in place and in order
             const float thr2 = kTieM / nG + 1e-4f + 2e-6f * (g.eS + g.gS) + 5e-7f * m.extent;
@@ -506,7 +539,7 @@ __device__ __forceinline__ void build_list(const ListGrid& m, Z zat, float4* lis
                 if (base + lane < c0) {
                     q = list[base + lane];
                     float gap;
-                    keep = gap_of(g, q.x, q.y, q.z, gap) <= thr2;
+                    keep = gap_keep(g, q.x, q.y, q.z, thr2, gap);
                     const int pk = __float_as_int(q.w);
                     const int i2 = ua + (pk >> 16), j2 = va + (pk & 0xffff);
                     outside |= keep && !(i2 >= ca && i2 <= cb && j2 >= da && j2 <= db);
@@ -616,20 +649,18 @@ __device__ __forceinline__ WarpVoxels warp_voxels(const float P[3])
     return w;
 }
 
-// Largest antenna movement of a pulse block, from its first pulse: re * distance / |E - G|
-// stays below kBlockSlope (it sets the lists' slack and with it their length), at most
-// kBlockPulses pulses.
-constexpr float kBlockSlope = 0.0125f;
-
 // Takes the next pulse block, from pulse i (< np): as many pulses as keep both antennas close
 // together, and both legs' lists for it (all 32 lanes call; P, P32, h0: the lane's voxel in
-// FP64 and in the FP32 frame and the height under it).  Returns the number of pulses.  Both
+// FP64 and in the FP32 frame and the height under it).  `slope` bounds the antennas' movement
+// from the block's first pulse: re * distance / |E - G| stays below twice it, which sets the
+// lists' slack and with it their length.  Returns the number of pulses, at most kBlockPulses.  Both
 // legs have a list or neither (m = -1), as when `lists` is false.
 template <typename Z>
 __device__ __forceinline__ int pulse_block(const ListGrid& m, Z zat, const DemView& d, BlockLists& bl, LegList* heads,
                                            const double* __restrict__ tx, const double* __restrict__ rx, int i, int np,
                                            double ox, double oy, const double P[3], const float P32[3], float h0v,
-                                           const WarpVoxels& wv, double n1, double n2, int W, bool lists)
+                                           const WarpVoxels& wv, double n1, double n2, int W, float slope,
+                                           bool lists)
 {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -650,7 +681,7 @@ __device__ __forceinline__ int pulse_block(const ListGrid& m, Z zat, const DemVi
         far = fmaxf(far, __fdividef(dx * dx + dy * dy + dz * dz, gx * gx + gy * gy + gz * gz));
     }
     const float re = fminf(__fdividef(n1f, n2f), 1.0f);
-    const unsigned stop = __ballot_sync(full, !(far * re * re <= 4.0f * kBlockSlope * kBlockSlope) && lane > 0);
+    const unsigned stop = __ballot_sync(full, !(far * re * re <= 4.0f * slope * slope) && lane > 0);
     const int n = min(min(stop ? __ffs(stop) - 1 : 32, kBlockPulses), np - i);
     if (!lists) {
         if (lane < 2) heads[lane].m = -1;
@@ -699,7 +730,7 @@ __device__ __forceinline__ int pulse_block(const ListGrid& m, Z zat, const DemVi
                 const double nx = __ldg(d.xv + nd.x), ny = __ldg(d.yv + nd.y);
                 const double nz = __ldg(d.z + (int64_t)nd.y * d.nx + nd.x);
                 const double le = __dmul_rn(n1, leg_len64(nx, ny, nz, El));
-                if (lane < kBlockPulses) bl.tab[leg].E[k][lane] = le;
+                bl.tab[leg].E[k][lane] = le;
                 bl.tab[leg].G[k][lane] = __dmul_rn(n2, leg_len64(nx, ny, nz, P));
             }
         }
