@@ -11,13 +11,17 @@
 //
 // A CTA's warps share 32 voxels and split the pulses into consecutive parts; the parts'
 // sums are added in pulse order.  The split follows the whole grid's size, so a range of
-// the grid has the image's bits.
+// the grid has the image's bits.  Parts differ in work (solves that a list's tables answer
+// against solves that are polished): with one part a warp, the CTA's other warps waited for
+// the slowest for a third of their time, so a warp has one part of 3/4 of its share, and the
+// rest is handed out in parts of a quarter as warps get free.  81 x 77 x 13 voxels x 512
+// pulses: 6.45 to 5.97 ms, one plane 1.34 to 1.15, 60 planes 23.4 to 21.1 (halves and halves:
+// 6.11, 1.15, 21.4).
 //
-// What bounds it: FP64 issue (list tables, sincospi, the polish of about a quarter of the
-// solves).  81 x 77 x 13 voxels x 512 pulses on a 0.25 m DEM, with pulse compression: 4.9 ms
-// on one B200; one warp per voxel with every pulse's own scan of (2W+1)^2 nodes, two FP64
-// square roots each, took 82 ms.  Three CTAs per SM (168 registers, no spills) against four:
-// 7.10 and 7.24 ms.
+// What bounds it: instruction latency and fetch at 12 warps an SM (an issue every third
+// cycle; the FP64 unit is 14 % busy).  The same scene took 82 ms with one warp per voxel and
+// every pulse's own scan of (2W+1)^2 nodes, two FP64 square roots each.  16 warps an SM (128
+// registers) are no faster: 5.95 ms.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -194,12 +198,21 @@ struct NewtonWarp {
 
 }  // namespace
 
+// First pulse of part k of 2 WPC: WPC parts of 3/4 of the pulses, then WPC of the rest.
+template <int WPC> __device__ __forceinline__ int part_begin(int k, int np)
+{
+    const int u = k < WPC ? 3 * k : 2 * WPC + k;     // of 4 WPC units
+    return (int)((int64_t)u * np / (4 * WPC));
+}
+
 template <int WPC>
-__global__ void __launch_bounds__(32 * WPC, WPC == 4 ? 3 : 16 / WPC) k_bp_newton(BpArgs a, float start_band, int compact)
+__global__ void __launch_bounds__(32 * WPC, WPC < 8 ? 12 / WPC : 16 / WPC)
+    k_bp_newton(BpArgs a, float start_band, int compact)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     NewtonWarp* ws = reinterpret_cast<NewtonWarp*>(smem_raw) + (threadIdx.x >> 5);
-    __shared__ double2 part[WPC][32];
+    __shared__ double2 part[2 * WPC][32];
+    __shared__ int next;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const DemView& d = a.dem;
     ListGrid m;
@@ -217,109 +230,115 @@ __global__ void __launch_bounds__(32 * WPC, WPC == 4 ? 3 : 16 / WPC) k_bp_newton
     const float P32[3] = {(float)(P[0] - d.x0), (float)(P[1] - d.y0), (float)P[2]};
     const double h64 = dem_elevation(d, P[0], P[1]);
     const WarpVoxels wv = warp_voxels(P32);
-    if (lane < 2) ws->h[lane].si = ws->h[lane].sj = -1;
-    __syncwarp();
+    if (threadIdx.x == 0) next = WPC;   // the parts after the first WPC go to the warps that are done
+    __syncthreads();
     const double inv_c = 1.0 / a.c, inv_lambda = 1.0 / a.lambda;
     const Heights64 zat(d);
-    const int p0 = (int)((int64_t)w * a.np / WPC), p1 = (int)((int64_t)(w + 1) * a.np / WPC);
-    double accr = 0.0, acci = 0.0;
-    int n;
-    for (int i = p0; i < p1; i += n) {
-        n = pulse_block(m, zat, d, ws->l, ws->h, a.tx, a.rx, i, p1, d.x0, d.y0, P, P32, (float)h64, wv, a.n1, a.n2, a.W,
-                        kBlockSlope, true);
-        const int m0 = all_pinned(ws->h[0]) ? ws->h[0].m : 0, m1 = all_pinned(ws->h[1]) ? ws->h[1].m : 0;
-        for (int b = 0; b < n; b += kPathPulses) {
-            const int step = min(kPathPulses, n - b);
-            // the legs to solve, one after the other over the block's pulses
+    for (int k = w; k < 2 * WPC;) {
+        const int p0 = part_begin<WPC>(k, a.np), p1 = part_begin<WPC>(k + 1, a.np);
+        if (lane < 2) ws->h[lane].si = ws->h[lane].sj = -1;
+        __syncwarp();
+        double accr = 0.0, acci = 0.0;
+        int n;
+        for (int i = p0; i < p1; i += n) {
+            n = pulse_block(m, zat, d, ws->l, ws->h, a.tx, a.rx, i, p1, d.x0, d.y0, P, P32, (float)h64, wv, a.n1, a.n2, a.W,
+                            kBlockSlope, true);
+            const int m0 = all_pinned(ws->h[0]) ? ws->h[0].m : 0, m1 = all_pinned(ws->h[1]) ? ws->h[1].m : 0;
+            for (int b = 0; b < n; b += kPathPulses) {
+                const int step = min(kPathPulses, n - b);
+                // the legs to solve, one after the other over the block's pulses
 #pragma unroll 1
-            for (int leg = m0 ? 1 : 0; leg < (m1 ? 1 : 2); leg++) {
-                const LegList* H = &ws->h[leg];
-                const int hm = H->m, mode = H->mode;
-                Leg64 l;
+                for (int leg = m0 ? 1 : 0; leg < (m1 ? 1 : 2); leg++) {
+                    const LegList* H = &ws->h[leg];
+                    const int hm = H->m, mode = H->mode;
+                    Leg64 l;
 #pragma unroll
-                for (int c = 0; c < 3; c++) l.G[c] = P[c];
-                l.nE = a.n1;
-                l.nG = a.n2;
-                l.g_lower = lower_is_voxel((float)a.n1, (float)a.n2, leg == 0);
+                    for (int c = 0; c < 3; c++) l.G[c] = P[c];
+                    l.nE = a.n1;
+                    l.nG = a.n2;
+                    l.g_lower = lower_is_voxel((float)a.n1, (float)a.n2, leg == 0);
 #pragma unroll 1
-                for (int q = b; q < b + step; q++) {
-                    double L = 0.0;
-                    int2 node = make_int2(0, 0);
-                    bool solved = false;
-                    if (hm > 0 && mode == (kCore | kTables)) {
-                        int c;
-                        L = table_min(ws->l.tab[leg], hm, q, lane, c);
-                        solved = (H->pinned >> c) & 1;
-                        node = H->node[c];
-                    }
-                    if (!solved) {
-                        const double* tr = (leg ? a.rx : a.tx) + 3 * (i + q);
-#pragma unroll
-                        for (int c = 0; c < 3; c++) l.E[c] = __ldg(tr + c);
-                        if (hm < 0) {
-                            node = scan_all64(d, l, h64, a.W);
-                        } else if (!(mode & kTables)) {
-                            node = rank_list64(d, ws->l.list[leg], *H, l, h64, a.W);
-                        } else if (!(mode & kCore)) {
-                            // a listed node may lie outside this solve's window
-                            const int2 st = start_node64(d, l, h64);
-                            const NodeTables* t = &ws->l.tab[leg];
-                            double v = INFINITY;
-                            int c = 0;
-#pragma unroll 1
-                            for (int k = 0; k < hm; k++) {
-                                const int2 nd = H->node[k];
-                                const double u = __dadd_rn(t->E[k][q], t->G[k][lane]);
-                                if (u < v && abs(nd.x - st.x) <= a.W && abs(nd.y - st.y) <= a.W) {
-                                    v = u;
-                                    c = k;
-                                }
-                            }
+                    for (int q = b; q < b + step; q++) {
+                        double L = 0.0;
+                        int2 node = make_int2(0, 0);
+                        bool solved = false;
+                        if (hm > 0 && mode == (kCore | kTables)) {
+                            int c;
+                            L = table_min(ws->l.tab[leg], hm, q, lane, c);
+                            solved = (H->pinned >> c) & 1;
                             node = H->node[c];
                         }
-                        L = polish64(d, m, l, node.x, node.y);
-                    }
-                    double* path = &ws->path[q - b][lane];
-                    *path = (leg && !m0) ? *path + L : L;
-                }
-            }
-            // delays, gathers and sums of the block's pulses
+                        if (!solved) {
+                            const double* tr = (leg ? a.rx : a.tx) + 3 * (i + q);
+#pragma unroll
+                            for (int c = 0; c < 3; c++) l.E[c] = __ldg(tr + c);
+                            if (hm < 0) {
+                                node = scan_all64(d, l, h64, a.W);
+                            } else if (!(mode & kTables)) {
+                                node = rank_list64(d, ws->l.list[leg], *H, l, h64, a.W);
+                            } else if (!(mode & kCore)) {
+                                // a listed node may lie outside this solve's window
+                                const int2 st = start_node64(d, l, h64);
+                                const NodeTables* t = &ws->l.tab[leg];
+                                double v = INFINITY;
+                                int c = 0;
 #pragma unroll 1
-            for (int q = b; q < b + step; q++) {
-                double L = (m0 && m1) ? 0.0 : ws->path[q - b][lane];
-                int c;
-                if (m0) L += table_min(ws->l.tab[0], m0, q, lane, c);
-                if (m1) L += table_min(ws->l.tab[1], m1, q, lane, c);
-                const double t_val = inv_c * L;                          // proc_test_script.cpp:565
-                const double bin = (1.0 + t_val * a.fs_eff) - 1.0;         // :569, :593
-                // (int)floor(bin) >= 0 && (int)ceil(bin) < nr  <=>  0 <= bin <= nr - 1 (NaN fails both)
-                if (bin >= 0.0 && bin <= (double)(a.nr - 1)) {
-                    const double lo_d = floor(bin);
-                    const int lo = (int)lo_d;                            // nr <= 2^30
-                    const double qf = bin - lo_d;
-                    const double2* row = a.rc64 + (int64_t)(i + q) * a.nr + lo;
-                    const double2 s0 = __ldg(row);
-                    double vr = s0.x, vi = s0.y;
-                    if (qf != 0.0) {
-                        const double2 s1 = __ldg(row + 1);
-                        vr = (1.0 - qf) * s0.x + qf * s1.x;              // :635
-                        vi = (1.0 - qf) * s0.y + qf * s1.y;
+                                for (int k = 0; k < hm; k++) {
+                                    const int2 nd = H->node[k];
+                                    const double u = __dadd_rn(t->E[k][q], t->G[k][lane]);
+                                    if (u < v && abs(nd.x - st.x) <= a.W && abs(nd.y - st.y) <= a.W) {
+                                        v = u;
+                                        c = k;
+                                    }
+                                }
+                                node = H->node[c];
+                            }
+                            L = polish64(d, m, l, node.x, node.y);
+                        }
+                        double* path = &ws->path[q - b][lane];
+                        *path = (leg && !m0) ? *path + L : L;
                     }
-                    // carrier phase (:573, :638) in turns, reduced before the sine
-                    const double turns = rint(L * inv_lambda);
-                    double sn, cs;
-                    sincospi(2.0 * (fma(-turns, a.lambda, L) * inv_lambda), &sn, &cs);
-                    accr += vr * cs - vi * sn;
-                    acci += vr * sn + vi * cs;
+                }
+                // delays, gathers and sums of the block's pulses
+#pragma unroll 1
+                for (int q = b; q < b + step; q++) {
+                    double L = (m0 && m1) ? 0.0 : ws->path[q - b][lane];
+                    int c;
+                    if (m0) L += table_min(ws->l.tab[0], m0, q, lane, c);
+                    if (m1) L += table_min(ws->l.tab[1], m1, q, lane, c);
+                    const double t_val = inv_c * L;                          // proc_test_script.cpp:565
+                    const double bin = (1.0 + t_val * a.fs_eff) - 1.0;         // :569, :593
+                    // (int)floor(bin) >= 0 && (int)ceil(bin) < nr  <=>  0 <= bin <= nr - 1 (NaN fails both)
+                    if (bin >= 0.0 && bin <= (double)(a.nr - 1)) {
+                        const double lo_d = floor(bin);
+                        const int lo = (int)lo_d;                            // nr <= 2^30
+                        const double qf = bin - lo_d;
+                        const double2* row = a.rc64 + (int64_t)(i + q) * a.nr + lo;
+                        const double2 s0 = __ldg(row);
+                        double vr = s0.x, vi = s0.y;
+                        if (qf != 0.0) {
+                            const double2 s1 = __ldg(row + 1);
+                            vr = (1.0 - qf) * s0.x + qf * s1.x;              // :635
+                            vi = (1.0 - qf) * s0.y + qf * s1.y;
+                        }
+                        // carrier phase (:573, :638) in turns, reduced before the sine
+                        const double turns = rint(L * inv_lambda);
+                        double sn, cs;
+                        sincospi(2.0 * (fma(-turns, a.lambda, L) * inv_lambda), &sn, &cs);
+                        accr += vr * cs - vi * sn;
+                        acci += vr * sn + vi * cs;
+                    }
                 }
             }
         }
+        part[k][lane] = make_double2(accr, acci);
+        if (lane == 0) k = atomicAdd(&next, 1);
+        k = __shfl_sync(0xffffffffu, k, 0);
     }
-    part[w][lane] = make_double2(accr, acci);
     __syncthreads();
     if (w == 0 && kk < a.v_count) {
-#pragma unroll
-        for (int q = 1; q < WPC; q++) {
+        double accr = 0.0, acci = 0.0;
+        for (int q = 0; q < 2 * WPC; q++) {
             accr += part[q][lane].x;
             acci += part[q][lane].y;
         }
@@ -341,14 +360,17 @@ cudaError_t launch_bp_newton(const BpArgs& a, cudaStream_t st)
     const int64_t plane = (int64_t)a.nx * a.ny;
     const int compact = a.v_begin % plane == 0 && a.v_count % plane == 0;
     const float band = list_start_band(a.dem);
-    // warps per 32 voxels: enough for about three waves of 16 warps per SM, with at least a
-    // pulse block each
+    // warps per 32 voxels: enough for about three waves of 16 warps per SM; more than four only
+    // with at least two pulse blocks each.  Two where that is enough: 60 planes of 6237 voxels
+    // 20.0 ms, with four 21.1; 26 planes 9.24 and 9.69 (one warp: 60 planes 19.5)
+    constexpr int64_t kWarps = 148 * 48;
     const int64_t tiles = (plane * a.nz + 31) / 32;
-    int wpc = 4;
-    while (wpc < 16 && tiles * wpc < (int64_t)148 * 48 && a.np >= 2 * wpc * kBlockPulses) wpc *= 2;
+    int wpc = tiles * 2 < kWarps ? 4 : 2;
+    while (wpc < 16 && tiles * wpc < kWarps && a.np >= 2 * wpc * kBlockPulses) wpc *= 2;
     if (wpc == 16) return launch_wpc<16>(a, band, compact, st);
     if (wpc == 8) return launch_wpc<8>(a, band, compact, st);
-    return launch_wpc<4>(a, band, compact, st);
+    if (wpc == 4) return launch_wpc<4>(a, band, compact, st);
+    return launch_wpc<2>(a, band, compact, st);
 }
 
 }  // namespace bsar

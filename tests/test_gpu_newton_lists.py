@@ -47,3 +47,22 @@ def test_newton_image_matches_the_oracle(ctx, oracle, name):
                               search_nodes=S.search_nodes_for(sc.x_vec, sc.y_vec))
     assert np.abs(want).max() > 0
     assert rel_l2(img, want) <= 1e-9
+
+
+@pytest.mark.parametrize("n_pulses", [1, 7, 50])
+def test_large_grid_has_the_small_grids_image(ctx, n_pulses):
+    """114000 voxels take two warps per 32 voxels, their first three x planes four: both within
+    1e-9 of the oracle, so within 2e-9 of each other."""
+    spec = S.scaled(S.config_spec(2), n_pulses=n_pulses, n_samples=4096, n_scatterers=2, nx=76, ny=50, nz=30, dxy=0.02)
+    sc = S.make_scene(spec, with_raw=False)
+    rng = np.random.default_rng(6)
+    sc.raw = rng.normal(size=(n_pulses, 4096)) + 1j * rng.normal(size=(n_pulses, 4096))
+    sid = bsar.upload_scene(ctx, sc)
+    form = dict(solver="newton", legs="per_pulse", precision="fp64")
+    try:
+        big = ctx.backproject(sid, sc.gx, sc.gy, sc.gz, **form)
+        small = ctx.backproject(sid, sc.gx[:3], sc.gy, sc.gz, **form)
+    finally:
+        ctx.scene_release(sid)
+    assert np.abs(small).max() > 0
+    assert rel_l2(big[:3], small) <= 2e-9
