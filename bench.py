@@ -143,19 +143,20 @@ def l2_copy_gbs(torch, stream, mib: int = 32, reps: int = 50) -> float:
 
 
 def fp32_flops_per_voxel_pulse(W: int) -> int:
-    """Algorithmic FP32 work of the mixed kernel per voxel-pulse (FMA = 2 flops), counted
-    from k_mixed.cu: per Fermat solve a (2W+1)^2 node scan at 17 flops per node, 4 facets x
-    3 polish steps at 80 flops and 4 facet evaluations at 25, a 4-step flat start at 19
-    flops (+ 20 setup); two solves per voxel-pulse plus 40 flops of delay / phase /
-    interpolation / Kahan work."""
-    per_solve = (2 * W + 1) ** 2 * 17 + 4 * 3 * 80 + 4 * 25 + 4 * 19 + 20
+    """FP32 work a voxel-pulse of the mixed form cannot do without (FMA = 2 flops), whatever
+    the scan's half width W: per Fermat solve a 4-step flat start at 19 flops (+ 20 setup),
+    the nine nodes around the crossing ranked at 17 flops, 3 polish steps at 80 on one facet
+    and its evaluation at 25; two solves per voxel-pulse plus 40 flops of delay / phase /
+    interpolation / Kahan work.  The kernel shares node rankings between voxels and pulses
+    and polishes more than one facet where it has to."""
+    per_solve = 9 * 17 + 3 * 80 + 25 + 4 * 19 + 20
     return 2 * per_solve + 40
 
 
 def sfu_ops_per_voxel_pulse(W: int) -> int:
-    """MUFU operations per voxel-pulse: 2 rsqrt per scanned node, 4 per polish step
-    (2 rsqrt + 2 rcp), 2 per facet evaluation, 2 per flat step; sincos = 2."""
-    per_solve = (2 * W + 1) ** 2 * 2 + 4 * 3 * 4 + 4 * 2 + 4 * 2
+    """MUFU operations of the same work: 2 rsqrt per ranked node, 4 per polish step (2 rsqrt
+    + 2 rcp), 2 for the evaluation, 2 per flat step; sincos = 2."""
+    per_solve = 9 * 2 + 3 * 4 + 2 + 4 * 2
     return 2 * per_solve + 2
 
 
@@ -856,8 +857,7 @@ def main():
                 "peak_source": f"nominal 148 SM x 128 FP32 lanes x 2 flop x {sm_mhz:.0f} MHz (no FP32-pipe "
                                f"figure in MEASURED_PEAKS.json)",
                 "sfu": {"achieved_gops": sfu_rate / 1e9, "peak_gops": sfu_peak / 1e9, "frac": sfu_rate / sfu_peak,
-                        "note": "algorithmic count (both legs' rsqrt per scanned node); the warp's shared E-leg "
-                                "table executes about half of them"},
+                        "note": "algorithmic count, as fp32_flops_per_voxel_pulse"},
                 "gather": {"bytes_per_voxel_pulse": 16, "achieved_gbs": 16 * vp / (bp_avg_ms / 1e3) / 1e9,
                            "hbm_peak_gbs": peaks.get("hbm_gbs"), "peak_source": peak_src,
                            "l2_peak_gbs": l2_gbs,

@@ -23,14 +23,14 @@
 // A block's legs are solved leg by leg over its pulses, then all its delays, gathers and
 // sums run in one short loop: the warps of an SM stay in small pieces of code.
 //
-// What bounds it: instruction fetch.  On the medium scene the rough DEM leaves a quarter of
-// the leg solves to polish, so a warp goes through list building, polish, final step and
-// gathers, some 60 KB of code, and warps wait for instructions longer than for anything
-// else; unrolling the gather loop or inlining rare branches made every scene slower, and
+// What bounds it: instruction latency and fetch at 12 warps an SM, an issue in 44 % of the
+// cycles.  On the medium scene the rough DEM leaves a quarter of the leg solves to polish, so
+// a warp goes through list building, polish, final step and gathers, some 100 KB of code;
+// unrolling the gather loop or inlining rare branches made every scene slower, and
 // three CTAs per SM (168 registers) run faster than four (98.7 against 109.4 ms on 161 x 161
 // x 81 voxels x 1024 pulses) or two.  Rare work is out of line.  Against the scan of every
 // lane's own window with per-lane lower bounds, with pulse compression, one B200: the medium
-// scene 513 ms before, 73 ms; 256 x 256 x 8 x 2048 on a 0.125 m DEM 618, 38 ms; 97 x 83 x 11
+// scene 487 ms before, 66 ms; 256 x 256 x 8 x 2048 on a 0.125 m DEM 614, 40 ms; 97 x 83 x 11
 // x 701 on 0.2 m (no compile-time scan width) 72, 5 ms.
 //
 // DEM tile: for wide scans (25 x 25 and generic widths) every CTA stages a TI x TJ FP32
@@ -788,7 +788,6 @@ __device__ __forceinline__ void voxel_mixed(const BpArgs& a, const MixedCtx& m, 
                                             WarpShared<WT>* ws, bool fp16, int compact, int64_t kk, int p0, int p1,
                                             double2* __restrict__ dst)
 {
-    const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int np = CH ? p1 : a.np;
     const float k_bin = (float)(a.fs_eff / a.c);
@@ -983,12 +982,12 @@ __device__ __forceinline__ void reduce_chunks(const BpArgs& a, const double2* __
 // CH: the instantiation for batches holding small-grid requests whose tiles run in pulse
 // chunks (MixedChunks); the last chunk of a tile to finish adds the chunks' sums in chunk
 // order.  Batches without chunks run the other instantiation, which never reads them.
-// The DEM tile is staged only for wide node scans (WT = 12, and the generic width): a
-// 25 x 25 scan builds 30-row warp tables every pulse and reads them from the tile faster
-// than through L1.  For 7 x 7 and 13 x 13 scans the tile's bookkeeping costs registers
-// (twice the spills) and its 17 KB per CTA shrinks L1, and the kernel runs faster with the
-// heights read from global memory -- the same FP32 values, so the same image.  (Measured with
-// the scans that rank every node, which the exhaustive flag still runs.)
+// The DEM tile is staged only for wide node scans (WT = 12, and the generic width), whose
+// exhaustive form builds 30-row warp tables every pulse and reads them from the tile faster
+// than through L1.  For 7 x 7 and 13 x 13 scans the tile's bookkeeping costs registers and
+// its 7 KB per CTA shrinks L1: heights come from global memory, the same FP32 values, so the
+// same image.  (Measured with the scans that rank every node, which the exhaustive flag
+// still runs.)
 template <int WT> struct StagesTile { static constexpr bool v = WT == 0 || WT >= 12; };
 
 template <int WT, bool CH>

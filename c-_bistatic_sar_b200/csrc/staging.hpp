@@ -6,7 +6,7 @@
 // slots of its own: threads claim chunks, copy between the caller's memory and a slot, and
 // enqueue the chunk's transfer on the call's stream, so the copies of some chunks overlap the
 // transfers of others.  The batched matched filter of 256 x 4096 complex128 samples, host to
-// host (16.8 MB each way), took 1.95 ms and takes 1.1 ms.
+// host (16.8 MB each way), took 1.95 ms and takes 1.1 to 1.3 ms.
 //
 // One Stager belongs to one context and is used under the context's lock.  It is made at the
 // first large copy; its threads end and its pinned memory (kSlotBytes x 2 per thread) is
