@@ -19,7 +19,7 @@
 // 6.11, 1.15, 21.4).
 //
 // What bounds it: instruction latency and fetch at 12 warps an SM (an issue every third
-// cycle; the FP64 unit is 14 % busy).  The same scene took 82 ms with one warp per voxel and
+// cycle; the FP64 unit is 16 % busy).  The same scene took 82 ms with one warp per voxel and
 // every pulse's own scan of (2W+1)^2 nodes, two FP64 square roots each.  16 warps an SM (128
 // registers) are no faster: 5.95 ms.
 #include <cuda_runtime.h>
