@@ -413,9 +413,13 @@ bool admit_one(bsar_server* s, std::unique_lock<std::mutex>& lk)
             break;
         }
     if (slot < 0) return false;
-    if (s->reserved + need > s->budget && !s->active.empty()) return false;
+    // also while a finished request's buffers are still held (it is no longer active, but its
+    // budget comes back only when they are freed); a request above the whole budget passes and
+    // fails below
+    if (s->reserved + need > s->budget && s->reserved > 0) return false;
     s->pending.pop_front();
     s->slot_used[slot] = true;
+    const uint64_t held = std::count(s->slot_used, s->slot_used + s->opts.max_inflight, true);
     r->slot = slot;
     r->reserved = need;
     s->reserved += need;
@@ -448,7 +452,9 @@ bool admit_one(bsar_server* s, std::unique_lock<std::mutex>& lk)
         r->state = St::Active;
         r->deadline_s = request_deadline(s, r);
         s->active.push_back(r);
-        s->peak_inflight = std::max<uint64_t>(s->peak_inflight, s->active.size());
+        // requests that held a slot when this one took its own: a small one's items can finish
+        // while the next is still being uploaded
+        s->peak_inflight = std::max<uint64_t>(s->peak_inflight, held);
     } else {
         finish(s, r, st, err);
         s->cv_done.notify_all();
