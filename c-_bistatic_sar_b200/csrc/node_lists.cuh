@@ -139,8 +139,6 @@ struct NodePatch {
     float rE[3], rG[3];     // the node less the antenna, less the voxel
     float Fx, Fy, Fz;       // the path's gradient at the node
     float gxb, gxf, gyb, gyf;   // its one-sided derivatives along the four edges (backward, forward)
-    float S1, S2;           // nE / |rE| + nG / |rG|, and with the squares
-    float dE, dG;           // |rE|, |rG|
 };
 
 __device__ __forceinline__ void patch_gradient(NodePatch& p, const ListGrid& m, float nE, float nG)
@@ -149,8 +147,6 @@ __device__ __forceinline__ void patch_gradient(NodePatch& p, const ListGrid& m, 
     const float qg = p.rG[0] * p.rG[0] + p.rG[1] * p.rG[1] + p.rG[2] * p.rG[2];
     const float se = rsqrtf(qe), sg = rsqrtf(qg);
     const float ge = nE * se, gg = nG * sg;
-    p.dE = qe * se;
-    p.dG = qg * sg;
     p.Fx = ge * p.rE[0] + gg * p.rG[0];
     p.Fy = ge * p.rE[1] + gg * p.rG[1];
     p.Fz = ge * p.rE[2] + gg * p.rG[2];
@@ -158,8 +154,6 @@ __device__ __forceinline__ void patch_gradient(NodePatch& p, const ListGrid& m, 
     p.gxf = fmaf(p.Fz, p.z[2][1] * m.istepx, p.Fx);
     p.gyb = fmaf(p.Fz, -p.z[1][0] * m.istepy, p.Fy);
     p.gyf = fmaf(p.Fz, p.z[1][2] * m.istepy, p.Fy);
-    p.S1 = ge + gg;
-    p.S2 = fmaf(ge, se, gg * sg);
 }
 
 // Facets to polish: those whose corner at the node is not their minimum because the path
@@ -169,65 +163,6 @@ __device__ __forceinline__ unsigned patch_todo(const NodePatch& p, bool xm, bool
     const bool ixm = !(p.gxb < 0.0f), ixp = !(p.gxf > 0.0f), iym = !(p.gyb < 0.0f), iyp = !(p.gyf > 0.0f);
     return (unsigned)(xm && ym && (ixm || iym)) | (unsigned)(xm && yp && (ixm || iyp)) << 1 |
            (unsigned)(xp && ym && (ixp || iym)) << 2 | (unsigned)(xp && yp && (ixp || iyp)) << 3;
-}
-
-// Of those, facets whose minimum lies on the edge they share with another facet to polish,
-// which therefore cannot win.  On the line from an edge into a facet the path is convex, so
-// where it rises at the edge along the whole edge, the facet's minimum is on the edge.  The
-// derivative across the edge is evaluated at both ends; between them it departs from the
-// chord by at most 1/8 of its second derivative, bounded through |d3 norm| <= 3 / d^2 (twist:
-// the change of the facet's cross slope along the edge).  The path falling towards +x and +y
-// (say) leaves one facet of three, falling along one edge only leaves one of two.
-__device__ __forceinline__ unsigned patch_skips(const NodePatch& p, const ListGrid& m, unsigned todo, float nE, float nG)
-{
-    const bool ixm = !(p.gxb < 0.0f), ixp = !(p.gxf > 0.0f), iym = !(p.gyb < 0.0f), iyp = !(p.gyf > 0.0f);
-    if ((todo & (todo - 1)) == 0 || (ixm && ixp) || (iym && iyp)) return 0;
-    const float noise = 1e-5f * (nE + nG);
-    // the gradient at the neighbour at (ox, oy, dz) from the node
-    auto gradient = [&](float ox, float oy, float dz, float F[3]) {
-        const float ex = p.rE[0] + ox, ey = p.rE[1] + oy, ez = p.rE[2] + dz;
-        const float gx = p.rG[0] + ox, gy = p.rG[1] + oy, gz = p.rG[2] + dz;
-        const float ge = nE * rsqrtf(ex * ex + ey * ey + ez * ez), gg = nG * rsqrtf(gx * gx + gy * gy + gz * gz);
-        F[0] = ge * ex + gg * gx;
-        F[1] = ge * ey + gg * gy;
-        F[2] = ge * ez + gg * gz;
-    };
-    // whether a derivative g0 at the node, F1 + Fz1 s1 at the edge's end (cross slopes s0, s1)
-    // points up in direction t all along an edge of squared length l2
-    auto rises = [&](float t, float g0, float F1, float Fz1, float s0, float s1, float l2) {
-        const float l = sqrtf(l2);
-        const float bend = 0.125f * (5.4f * l2 * p.S2 * (1.0f + fmaxf(fabsf(s0), fabsf(s1))) +
-                                     2.7f * l * p.S1 * fabsf(s1 - s0)) + noise;
-        return t * g0 > bend && t * fmaf(Fz1, s1, F1) > bend && l <= 0.25f * fminf(p.dE, p.dG);
-    };
-    unsigned skip = 0;
-    const bool sx = ixm || ixp, sy = iym || iyp;        // the path falls along one x edge, one y edge
-    // the facet between both edges holds the crossing of a path that falls along both
-    const unsigned both = sx && sy ? 1u << ((ixp ? 2 : 0) + (iyp ? 1 : 0)) : 0u;
-    if (both & ~todo) return 0;
-    if (sx) {
-        const float n0 = ixp ? p.z[2][0] : p.z[0][0], n1 = ixp ? p.z[2][1] : p.z[0][1], n2 = ixp ? p.z[2][2] : p.z[0][2];
-        float F[3];
-        gradient(ixp ? m.stepx : -m.stepx, 0.0f, n1, F);
-        const float l2 = fmaf(n1, n1, m.stepx * m.stepx);
-        const bool up = rises(1.0f, p.gyf, F[1], F[2], p.z[1][2] * m.istepy, (n2 - n1) * m.istepy, l2);
-        const bool down = rises(-1.0f, p.gyb, F[1], F[2], -p.z[1][0] * m.istepy, (n1 - n0) * m.istepy, l2);
-        const unsigned f0 = ixp ? 4u : 1u, f1 = f0 << 1;     // the edge's facets on the -y and +y side
-        if (both) skip |= iyp ? (down ? f0 : 0u) : (up ? f1 : 0u);
-        else skip |= (up && (todo & f0)) ? f1 : ((down && (todo & f1)) ? f0 : 0u);
-    }
-    if (sy) {
-        const float n0 = iyp ? p.z[0][2] : p.z[0][0], n1 = iyp ? p.z[1][2] : p.z[1][0], n2 = iyp ? p.z[2][2] : p.z[2][0];
-        float F[3];
-        gradient(0.0f, iyp ? m.stepy : -m.stepy, n1, F);
-        const float l2 = fmaf(n1, n1, m.stepy * m.stepy);
-        const bool up = rises(1.0f, p.gxf, F[0], F[2], p.z[2][1] * m.istepx, (n2 - n1) * m.istepx, l2);
-        const bool down = rises(-1.0f, p.gxb, F[0], F[2], -p.z[0][1] * m.istepx, (n1 - n0) * m.istepx, l2);
-        const unsigned f0 = iyp ? 2u : 1u, f1 = f0 << 2;     // on the -x and +x side
-        if (both) skip |= ixp ? (down ? f0 : 0u) : (up ? f1 : 0u);
-        else skip |= (up && (todo & f0)) ? f1 : ((down && (todo & f1)) ? f0 : 0u);
-    }
-    return skip & todo;
 }
 
 // The path at (u, v) on facet (fi, fj); on a node, that node's path.  Out of line: the final
