@@ -66,3 +66,27 @@ def test_large_grid_has_the_small_grids_image(ctx, n_pulses):
         ctx.scene_release(sid)
     assert np.abs(small).max() > 0
     assert rel_l2(big[:3], small) <= 2e-9
+
+
+@pytest.mark.parametrize("seed,voxel", [(6, (62, 0, 22)), (6, (65, 25, 16)), (6, (56, 35, 3)), (3, (7, 7, 21)),
+                                        (26, (34, 40, 0))])
+def test_every_open_facet_is_polished(ctx, oracle, seed, voxel):
+    """Voxels with a crossing whose edge minimum three Newton steps reach from one of the edge's
+    two facets only.  Paths of 50 m round at 7e-15 m, 1.5e-13 rad of phase; 1e-11 leaves room for
+    some sixty roundings per path, and a facet left out shows as 1e-7."""
+    spec = S.scaled(S.config_spec(2), n_pulses=256, n_samples=4096, n_scatterers=2, seed=seed, nx=81, ny=77, nz=24,
+                    dem_sigma=0.5, eps_r=3.0)
+    sc = S.make_scene(spec, with_raw=False)
+    rng = np.random.default_rng(5)
+    sc.raw = rng.normal(size=(256, 4096)) + 1j * rng.normal(size=(256, 4096))
+    gx, gy, gz = (g[i:i + 1] for g, i in zip((sc.gx, sc.gy, sc.gz), voxel))
+    sid = bsar.upload_scene(ctx, sc)
+    try:
+        img = ctx.backproject(sid, gx, gy, gz, solver="newton", legs="per_pulse", precision="fp64")
+    finally:
+        ctx.scene_release(sid)
+    rc = oracle.spline_upsample(oracle.fft_correlate(sc.raw, sc.reference), spec.upsample)
+    want = oracle.backproject(O.Dem(sc.x_vec, sc.y_vec, sc.z), sc.tx, sc.rx, rc, gx, gy, gz, spec.n1, spec.n2, 3e8,
+                              sc.fs_eff, sc.lam, legs="per", solver="newton",
+                              search_nodes=S.search_nodes_for(sc.x_vec, sc.y_vec))
+    assert rel_l2(img, want) <= 1e-11
