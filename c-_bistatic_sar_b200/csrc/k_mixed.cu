@@ -48,6 +48,7 @@
 
 #include "dev_common.cuh"
 #include "kernels.hpp"
+#include "mixed_solve.cuh"
 #include "node_lists.cuh"
 
 namespace bsar {
@@ -57,19 +58,6 @@ namespace {
 constexpr int TI = kMixedTileI;    // tile columns (x); 176 B rows, a multiple of 16 B
 constexpr int TJ = kMixedTileJ;    // tile rows (y)
 constexpr long kWaitSpins = 1L << 24;
-
-struct Facet32 {
-    float x0, y0, dx, dy, z00, b, c, e;
-    float idx, idy;     // 1 / dx, 1 / dy
-};
-
-struct MixedCtx : ListGrid {
-    const float* __restrict__ z32;  // pitch-padded FP32 heights, z32[j * pitch + i]
-    int pitch;
-    double ox, oy;                  // origin of the FP32 frame (first DEM node)
-    double idx64, idy64;            // 1 / spacing, FP64
-    int lists;                      // node scans may run on candidate lists
-};
 
 // Start heights under a voxel (the lower endpoint of both of its paths when the ground
 // index exceeds the air index): FP32 bilinear for the FP32 start, the FP64 DEM lookup for
@@ -85,8 +73,6 @@ struct Tile {
     int i0, j0;
     bool ok;
 };
-
-__device__ __forceinline__ float zf(const MixedCtx& m, int i, int j) { return __ldg(m.z32 + (int64_t)j * m.pitch + i); }
 
 // Heights for the candidate lists: from the tile when it covers the nodes to rank.
 struct TileHeights {
@@ -104,17 +90,6 @@ struct TileHeights {
         return in_tile ? T.s[(j - T.j0) * TI + (i - T.i0)] : zf(m, i, j);
     }
 };
-
-// FP32 bilinear height (clamped to the DEM) for the flat-interface start.
-__device__ __forceinline__ float height32(const MixedCtx& m, float x, float y)
-{
-    float fx = x * m.istepx, fy = y * m.istepy;
-    int i = min(max((int)floorf(fx), 0), m.nx - 2);
-    int j = min(max((int)floorf(fy), 0), m.ny - 2);
-    float u = fminf(fmaxf(fx - (float)i, 0.f), 1.f), v = fminf(fmaxf(fy - (float)j, 0.f), 1.f);
-    float z00 = zf(m, i, j), z01 = zf(m, i + 1, j), z10 = zf(m, i, j + 1), z11 = zf(m, i + 1, j + 1);
-    return z00 + (z01 - z00) * u + (z10 - z00) * v + (z11 - z01 - z10 + z00) * u * v;
-}
 
 __device__ __forceinline__ float TileHeights::ground(float x, float y) const { return height32(m, x, y); }
 
@@ -184,37 +159,6 @@ __device__ __forceinline__ float facet_eval32(const Facet32& F, const float A[3]
     float q2 = r2x * r2x + r2y * r2y + r2z * r2z;
     return na * (q1 * rsqrtf(q1)) + nb * (q2 * rsqrtf(q2));
 }
-
-// The crossing after the FP64 final step from (u, v) on facet (fi, fj).
-__device__ __forceinline__ void final_point64(const DemView& d, int fi, int fj, const double A[3], const double B[3],
-                                              double na, double nb, double u, double v, double X[3], double idx_,
-                                              double idy)
-{
-    Facet64 F;
-    facet_load(d, fi, fj, F);
-    facet_newton64(F, A, B, na, nb, idx_, idy, u, v);
-    X[0] = F.x0 + u * F.dx;
-    X[1] = F.y0 + v * F.dy;
-    X[2] = F.z00 + F.b * u + F.c * v + F.e * u * v;
-}
-
-// Node ranking values.  G is the voxel-side endpoint of the path (index ng), E the
-// other one (index ne); the scans rank L' = re |N-E| + |N-G| = L / ng with re = ne / ng.
-
-// Branch-free ranking update: best value / position and runner-up value.
-__device__ __forceinline__ void rank(float L, int i, int j, float& v1, float& v2, int& bi, int& bj)
-{
-    v2 = fminf(v2, fmaxf(v1, L));
-    bool p = L < v1;
-    v1 = p ? L : v1;
-    bi = p ? i : bi;
-    bj = p ? j : bj;
-}
-
-struct Rank {
-    float v1, v2;
-    int bi, bj;
-};
 
 // Generic node scan over [ia, ib] x [ja, jb]: both legs per node, z from the tile when
 // `in_tile`, else from global memory.
@@ -321,44 +265,10 @@ __device__ __forceinline__ void scan_table(const MixedCtx& m, const AirTable& AT
     bj = js - W + bc;
 }
 
-// FP64 re-ranking of the nodes within the FP32 ambiguity band, with the FP64 solver's
-// arithmetic and order (i-major, j-minor, strict <).
-__device__ __noinline__ int2 rerank64(const DemView d, const MixedCtx m, const float* ts, int ti0, int tj0, bool tok,
-                                      int is, int js, int Wr, float ex, float ey, float ez, float gx, float gy,
-                                      float gz, float re, float limit, double Ax, double Ay, double Az, double Bx,
-                                      double By, double Bz, double na, double nb, int2 best_ij)
-{
-    const int ia = max(is - Wr, 0), ib = min(is + Wr, m.nx - 1);
-    const int ja = max(js - Wr, 0), jb = min(js + Wr, m.ny - 1);
-    const bool in_tile = tok && ia >= ti0 && ib < ti0 + TI && ja >= tj0 && jb < tj0 + TJ;
-    const double A[3] = {Ax, Ay, Az}, B[3] = {Bx, By, Bz};
-    double best = INFINITY;
-    for (int i = ia; i <= ib; i++) {
-        float xi = (float)i * m.stepx;
-        float dxe = xi - ex, dxg = xi - gx;
-        for (int j = ja; j <= jb; j++) {
-            float yj = (float)j * m.stepy;
-            float dye = yj - ey, dyg = yj - gy;
-            float z = in_tile ? ts[(j - tj0) * TI + (i - ti0)] : zf(m, i, j);
-            float dze = z - ez, dzg = z - gz;
-            float qe = dxe * dxe + dye * dye + dze * dze;
-            float qg = dxg * dxg + dyg * dyg + dzg * dzg;
-            if (re * sqrtf(qe) + sqrtf(qg) <= limit) {
-                double L = node_l64(d, i, j, A, B, na, nb);
-                if (L < best) {
-                    best = L;
-                    best_ij = make_int2(i, j);
-                }
-            }
-        }
-    }
-    return best_ij;
-}
-
-// Warp-cooperative form of rerank64: each lane whose FP32 runner-up lies within the tie
-// band (`need`) has its window re-ranked by the whole warp, 32 nodes at a time, with the
-// same FP32 filter and FP64 node values; the smallest FP64 value with the lowest i-major
-// index wins, which is the node the FP64 scan's strict < keeps.  All 32 lanes call it.
+// FP64 re-ranking of the nodes within the FP32 ambiguity band: each lane whose FP32
+// runner-up lies within it (`need`) has its window re-ranked by the whole warp, 32 nodes at a
+// time; the smallest FP64 value with the lowest i-major index wins, which is the node the
+// FP64 scan's strict < keeps.  All 32 lanes call it.
 __device__ __noinline__ int2 rerank64_warp(const DemView d, const MixedCtx m, const float* ts, int ti0, int tj0,
                                            bool tok, bool need, int is, int js, int Wr, float ex, float ey, float ez,
                                            float gx, float gy, float gz, float re, float limit, double Ax, double Ay,
@@ -458,28 +368,8 @@ __device__ __noinline__ int2 start_node(const DemView d, const MixedCtx m, const
     return c;
 }
 
-// Best node of one lane's own window, every node ranked (FP32, near ties in FP64).
-__device__ __forceinline__ int2 scan_lane(const DemView& d, const MixedCtx& m, const Tile& T, const Leg& l,
-                                          const VoxelStart& vs, int W)
-{
-    const int2 c = start_node(d, m, l, vs);
-    const float* E = l.E32;
-    const float* G = l.G32;
-    const float re = __fdividef(l.nE, l.nG);
-    const float tie = kTieM / l.nG;
-    const int ia = max(c.x - W, 0), ib = min(c.x + W, m.nx - 1);
-    const int ja = max(c.y - W, 0), jb = min(c.y + W, m.ny - 1);
-    const bool in_tile = T.ok && ia >= T.i0 && ib < T.i0 + TI && ja >= T.j0 && jb < T.j0 + TJ;
-    const Rank r = scan_generic(m, T.s, T.i0, T.j0, in_tile, ia, ib, ja, jb, E[0], E[1], E[2], G[0], G[1], G[2], re,
-                                Rank{INFINITY, INFINITY, c.x, c.y});
-    if (r.v2 - r.v1 >= tie) return make_int2(r.bi, r.bj);
-    return rerank64(d, m, T.s, T.i0, T.j0, T.ok, c.x, c.y, W, E[0], E[1], E[2], G[0], G[1], G[2], re, r.v1 + tie,
-                    l.E[0], l.E[1], l.E[2], l.G[0], l.G[1], l.G[2], l.nE64, l.nG64,
-                    make_int2(r.bi, r.bj));
-}
-
-// The same for a whole warp (all 32 lanes call): windows of the common widths ranked from
-// the warp's table, near ties re-ranked by the warp together.  Runs for the exhaustive
+// Best node of every lane's own window, every node ranked (all 32 lanes call): windows of the
+// common widths from the warp's table, near ties re-ranked in FP64 by the warp together.  Runs for the exhaustive
 // flag and where no candidate list holds, so it stays out of the pulse loop's
 // instruction stream.
 template <int WT>
@@ -1070,76 +960,7 @@ __global__ void __launch_bounds__(128, 3) k_bp_mixed(MixedBatch b)
     if (copy_pending) drain_tile(&mbar, parity ^ 1u);
 }
 
-static MixedCtx mixed_ctx(const DemView& d, int pitch)
-{
-    MixedCtx m;
-    m.z32 = d.z32;
-    m.pitch = pitch;
-    m.nx = d.nx;
-    m.ny = d.ny;
-    m.stepx = (float)d.stepx;
-    m.stepy = (float)d.stepy;
-    m.istepx = (float)(1.0 / d.stepx);
-    m.istepy = (float)(1.0 / d.stepy);
-    m.ox = d.x0;
-    m.oy = d.y0;
-    m.idx64 = 1.0 / d.stepx;
-    m.idy64 = 1.0 / d.stepy;
-    m.start_band = list_start_band(d);
-    m.lists = 0;
-    m.extent = 0.0f;
-    return m;
-}
-
-// Crossing points of the mixed solver (FP32 scan and polish, FP64 final step) for n
-// (start, end) pairs: the data behind the mixed form's crossing-point error.
-__global__ void k_refraction_mixed(DemView d, MixedCtx m, const double* __restrict__ p1, const double* __restrict__ p2,
-                                   int64_t n, double na, double nb, int W, double* __restrict__ out)
-{
-    const Tile T{nullptr, 0, 0, false};
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
-        Leg l;
-        for (int c = 0; c < 3; c++) {
-            const double o = c == 0 ? m.ox : (c == 1 ? m.oy : 0.0);
-            l.E[c] = p1[3 * k + c];
-            l.G[c] = p2[3 * k + c];
-            l.E32[c] = (float)(l.E[c] - o);
-            l.G32[c] = (float)(l.G[c] - o);
-        }
-        l.nE = (float)na;
-        l.nG = (float)nb;
-        l.nE64 = na;
-        l.nG64 = nb;
-        l.g_lower = lower_is_voxel(l.nE, l.nG, true);
-        l.to_voxel = true;
-        double X[3];
-        const VoxelStart vs{height32(m, l.G32[0], l.G32[1]), dem_elevation(d, l.G[0], l.G[1])};
-        const int2 node = scan_lane(d, m, T, l, vs, W);
-        int fi, fj;
-        float u, v;
-        if (!polish_leg(m, T, l, node.x, node.y, fi, fj, u, v)) {
-            fi = max(node.x - 1, 0);
-            fj = max(node.y - 1, 0);
-            u = (float)(node.x - fi);
-            v = (float)(node.y - fj);
-        }
-        final_point64(d, fi, fj, l.E, l.G, l.nE64, l.nG64, (double)u, (double)v, X, m.idx64, m.idy64);
-        out[3 * k] = X[0];
-        out[3 * k + 1] = X[1];
-        out[3 * k + 2] = X[2];
-    }
-}
-
 float mixed_start_band(const DemView& d) { return list_start_band(d); }
-
-cudaError_t launch_refraction_mixed(const DemView& d, int pitch, const double* p1, const double* p2, int64_t n,
-                                    double n1, double n2, int W, double* out, cudaStream_t st)
-{
-    int64_t b = (n + 127) / 128;
-    int blocks = (int)(b < 1 ? 1 : (b > 148 * 64 ? 148 * 64 : b));
-    k_refraction_mixed<<<blocks, 128, 0, st>>>(d, mixed_ctx(d, pitch), p1, p2, n, n1, n2, W, out);
-    return cudaGetLastError();
-}
 
 // Shared-memory carve-out for 3 resident CTAs per SM (DEM tile + 4 warps' lists each),
 // set once per device; the rest of the unified L1 stays cache for the sample gathers.
