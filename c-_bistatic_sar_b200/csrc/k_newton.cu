@@ -107,9 +107,43 @@ __device__ __forceinline__ double facet_path(const Facet64& F, const Leg64& l, d
     return path64(leg_len64(x, y, z, l.E), leg_len64(x, y, z, l.G), l.nE, l.nG);
 }
 
-// From the best node (bi, bj) to the path: each of the four facets that have the node as
-// a corner is polished, unless that corner is its minimum (the path's one-sided derivatives
-// at the node); one more step on the best facet.  Leaving out facets whose minimum lies on an
+// polish64 where a facet whose steps ended at the node ties with facets that keep the node:
+// every facet in the solver's order, with its own rounding of the node's path.  The first
+// smallest wins, and its one more step may leave the node (voxels at the surface, whose undamped
+// steps cycle between corners).
+__device__ __noinline__ double polish_tied64(const DemView d, const Leg64 l, int bi, int bj)
+{
+    double best = INFINITY, bu = 0.0, bv = 0.0;
+    Facet64 F;
+    int bk = 0;
+#pragma unroll 1
+    for (int k = 0; k < 4; k++) {
+        const int fi = bi - 1 + (k >> 1), fj = bj - 1 + (k & 1);
+        if (fi < 0 || fj < 0 || fi > d.nx - 2 || fj > d.ny - 2) continue;
+        facet_load(d, fi, fj, F);
+        const double idx = 1.0 / F.dx, idy = 1.0 / F.dy;
+        double u = (double)(bi - fi), v = (double)(bj - fj);
+#pragma unroll 1
+        for (int it = 0; it < kPolishIters; it++)
+            if (!facet_newton64(F, l.E, l.G, l.nE, l.nG, idx, idy, u, v)) break;
+        const double L = facet_path(F, l, u, v);
+        if (L < best) {
+            best = L;
+            bu = u;
+            bv = v;
+            bk = k;
+        }
+    }
+    facet_load(d, bi - 1 + (bk >> 1), bj - 1 + (bk & 1), F);
+    facet_newton64(F, l.E, l.G, l.nE, l.nG, 1.0 / F.dx, 1.0 / F.dy, bu, bv);
+    return facet_path(F, l, bu, bv);
+}
+
+// From the best node (bi, bj) to the path, as the FP64 solver (refraction_newton) forms it: each
+// of the four facets that have the node as a corner is polished, unless that corner is its
+// minimum (the path's one-sided derivatives at the node; such a facet has the node's path); one
+// more step on the best facet.  Where no facet has its minimum at the node, the node's path is
+// not a candidate, even if three steps end above it (voxels at the surface).  Leaving out facets whose minimum lies on an
 // edge of another polished one saved nothing (13 planes of 6237 voxels 5.97 ms, without 5.84;
 // 60 planes 20.0 and 19.6; one plane 1.15 and 1.21), and where three steps had not reached that
 // edge's minimum from the other side, single paths came out 1e-7 m long.
@@ -119,7 +153,7 @@ __device__ __forceinline__ double polish64(const DemView& d, const ListGrid& m, 
     const bool xm = bi > 0, xp = bi < d.nx - 1, ym = bj > 0, yp = bj < d.ny - 1;
     const double* zr = d.z + (int64_t)bj * d.nx + bi;
     const double z = __ldg(zr);
-    double best = path64(leg_len64(x, y, z, l.E), leg_len64(x, y, z, l.G), l.nE, l.nG);
+    const double node = path64(leg_len64(x, y, z, l.E), leg_len64(x, y, z, l.G), l.nE, l.nG);
     // which facets to polish: FP32 derivatives; a corner within their rounding is polished, and
     // its Newton step then finds it in FP64
     NodePatch p;
@@ -140,9 +174,13 @@ __device__ __forceinline__ double polish64(const DemView& d, const ListGrid& m, 
     p.gyb += noise * (1.0f + fabsf(p.z[1][0]) * m.istepy);
     p.gyf -= noise * (1.0f + fabsf(p.z[1][2]) * m.istepy);
     unsigned todo = patch_todo(p, xm, xp, ym, yp);
-    bool moved = false;
-    double bu = 0.0, bv = 0.0;
-    int bfi = 0, bfj = 0;
+    const unsigned facets = (unsigned)(xm && ym) | (unsigned)(xm && yp) << 1 | (unsigned)(xp && ym) << 2 |
+                            (unsigned)(xp && yp) << 3;
+    const bool keeps = todo != facets;     // some facet's minimum is the node
+    bool step = !keeps;
+    double best = keeps ? node : (double)INFINITY;
+    int bfi = min(bi, d.nx - 2), bfj = min(bj, d.ny - 2);     // kept only when no path compares below infinity
+    double bu = (double)(bi - bfi), bv = (double)(bj - bfj);
 #pragma unroll 1
     while (todo) {
         const int k = __ffs(todo) - 1;
@@ -159,19 +197,18 @@ __device__ __forceinline__ double polish64(const DemView& d, const ListGrid& m, 
             if (!facet_newton64(F, l.E, l.G, l.nE, l.nG, idx, idy, u, v)) break;
             m1 = true;
         }
-        if (m1) {
-            const double L = facet_path(F, l, u, v);
-            if (L < best) {
-                best = L;
-                moved = true;
-                bu = u;
-                bv = v;
-                bfi = fi;
-                bfj = fj;
-            }
+        const double L = m1 ? facet_path(F, l, u, v) : node;
+        if (m1 && keeps && fabs(L - node) <= 1e-13 * node) return polish_tied64(d, l, bi, bj);
+        if (L < best) {
+            best = L;
+            step = true;
+            bu = u;
+            bv = v;
+            bfi = fi;
+            bfj = fj;
         }
     }
-    if (moved) {
+    if (step) {
         Facet64 F;
         facet_load(d, bfi, bfj, F);
         facet_newton64(F, l.E, l.G, l.nE, l.nG, 1.0 / F.dx, 1.0 / F.dy, bu, bv);
