@@ -378,8 +378,8 @@ class Context:
                     search_radius_m=0.0, out=None, exhaustive=False):
         """Image [x][y][z] complex128; `out` (C-contiguous complex128 of that shape, e.g.
         a view of pinned memory) receives it instead of a new array.  `exhaustive`: the
-        mixed forms rank every node of each node-scan window (BSAR_BP_EXHAUSTIVE_SCAN;
-        the same image, slower)."""
+        mixed and FP64 Newton forms rank every node of each node-scan window
+        (BSAR_BP_EXHAUSTIVE_SCAN; the same image, slower)."""
         keep, g = self._grid(gx, gy, gz)
         o = BpOpts(SOLVER[solver], LEGS[legs], PRECISION[precision], EXHAUSTIVE if exhaustive else 0,
                    search_radius_m)

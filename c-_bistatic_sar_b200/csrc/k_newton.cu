@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(32 * WPC, WPC < 8 ? 12 / WPC : 16 / WPC)
         int n;
         for (int i = p0; i < p1; i += n) {
             n = pulse_block(m, zat, d, ws->l, ws->h, a.tx, a.rx, i, p1, d.x0, d.y0, P, P32, (float)h64, wv, a.n1, a.n2, a.W,
-                            kBlockSlope, true);
+                            kBlockSlope, !a.exhaustive);
             const int m0 = all_pinned(ws->h[0]) ? ws->h[0].m : 0, m1 = all_pinned(ws->h[1]) ? ws->h[1].m : 0;
             for (int b = 0; b < n; b += kPathPulses) {
                 const int step = min(kPathPulses, n - b);

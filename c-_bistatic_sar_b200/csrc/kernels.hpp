@@ -104,6 +104,7 @@ struct BpArgs {
     int64_t v_begin, v_count;  // voxel range, reference flat order (z -> x -> y)
     double2* out;         // image [x][y][z]
     float zlo, zhi;       // the DEM's range of heights (FP64 grid search)
+    int exhaustive;       // FP64 Newton: 1, node scans rank every node (no candidate lists); the image is the same
     // mixed form: per-pulse FP64 reference optical path and reduced carrier phase
     const double* ref_L;    // np
     const float* ref_phase; // np, (2 pi / lambda) * ref_L reduced to [-pi, pi)

@@ -243,10 +243,12 @@ typedef struct bsar_bp_opts {
     double search_radius_m;  /* Newton node-scan radius (<= 0: 1.5 m) */
 } bsar_bp_opts;
 
-/* bsar_bp_opts.flags.  BSAR_BP_EXHAUSTIVE_SCAN: the mixed forms rank every node of each
- * Fermat node-scan window instead of skipping the rows and column groups that a lower
- * bound proves cannot hold the minimum.  The image is bit-identical either way; the flag
- * exists to verify that, at the cost of speed.  The FP64 forms always scan every node. */
+/* bsar_bp_opts.flags.  BSAR_BP_EXHAUSTIVE_SCAN: the mixed and FP64 Newton forms rank
+ * every node of each Fermat node-scan window instead of the candidate lists that a bound
+ * proves to hold the minimum.  The image is bit-identical either way; the flag exists to
+ * verify that, at the cost of speed.  FP64 Newton with mean legs ranks every node always, and
+ * the grid search, whose FP32 filter leaves out points that a bound proves larger, takes no
+ * notice of the flag. */
 enum { BSAR_BP_EXHAUSTIVE_SCAN = 1 };
 
 /* The imager's voxel loop, proc_test_script.cpp:451-767: for every voxel the Fermat

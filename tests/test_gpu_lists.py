@@ -37,6 +37,16 @@ CASES = {
 @pytest.mark.parametrize("precision", ["mixed", "mixed_fp16"])
 @pytest.mark.parametrize("name", CASES)
 def test_lists_give_the_exhaustive_image(ctx, name, precision):
+    _lists_equal_exhaustive(ctx, name, precision)
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_fp64_lists_give_the_exhaustive_image(ctx, name):
+    """The same of the FP64 Newton kernel, whose lists are bounded in FP32."""
+    _lists_equal_exhaustive(ctx, name, "fp64")
+
+
+def _lists_equal_exhaustive(ctx, name, precision):
     kw, dz, gz, radius = CASES[name]
     sc = S.make_scene(S.scaled(S.config_spec(2), **{**dict(n_pulses=70, n_samples=4096, n_scatterers=3), **kw}),
                       with_raw=False)
