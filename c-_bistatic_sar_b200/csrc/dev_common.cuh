@@ -324,7 +324,7 @@ __device__ __forceinline__ void grid_level_filter(const DemView& d, int pitch, f
     const int t = threadIdx.x;
     const float n1f = (float)n1, n2f = (float)n2;
     const float zerr = 4e-7f * (n1f + n2f);
-    const float z1f = (float)z1, z2f = (float)z2;
+    const float z1f = (float)(z1 - d.z0), z2f = (float)(z2 - d.z0);
     const float base_err = zerr * (fabsf(z1f) + fabsf(z2f));
     double top = minOP;
     if (G == 15) top = fmin(top, point((G - 1) / 2, (G - 1) / 2).op);

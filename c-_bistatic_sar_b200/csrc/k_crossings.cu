@@ -256,7 +256,7 @@ __global__ void k_refraction_mixed(DemView d, MixedCtx m, const double* __restri
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
         Pair p;
         for (int c = 0; c < 3; c++) {
-            const double o = c == 0 ? m.ox : (c == 1 ? m.oy : 0.0);
+            const double o = c == 0 ? m.ox : (c == 1 ? m.oy : m.oz);
             p.A[c] = p1[3 * k + c];
             p.B[c] = p2[3 * k + c];
             p.A32[c] = (float)(p.A[c] - o);
@@ -287,6 +287,7 @@ cudaError_t launch_refraction_mixed(const DemView& d, int pitch, const double* p
     m.istepy = (float)(1.0 / d.stepy);
     m.ox = d.x0;
     m.oy = d.y0;
+    m.oz = d.z0;
     m.idx64 = 1.0 / d.stepx;
     m.idy64 = 1.0 / d.stepy;
     m.start_band = list_start_band(d);

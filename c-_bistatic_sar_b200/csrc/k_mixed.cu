@@ -380,7 +380,6 @@ __device__ __noinline__ int2 scan_warp(const DemView d, const MixedCtx m, const 
     const float* E = l.E32;
     const float* G = l.G32;
     const float re = __fdividef(l.nE, l.nG);
-    const float tie = kTieM / l.nG;
     const int ia = max(c.x - W, 0), ib = min(c.x + W, m.nx - 1);
     const int ja = max(c.y - W, 0), jb = min(c.y + W, m.ny - 1);
     Rank r{INFINITY, INFINITY, c.x, c.y};
@@ -397,6 +396,7 @@ __device__ __noinline__ int2 scan_warp(const DemView d, const MixedCtx m, const 
         r = scan_generic(m, T.s, T.i0, T.j0, in_tile, ia, ib, ja, jb, E[0], E[1], E[2], G[0], G[1], G[2], re, r);
     }
     int2 best = make_int2(r.bi, r.bj);
+    const float tie = tie_band(m, l.nG, r.v1);
     const bool need = !(r.v2 - r.v1 >= tie);
     if (__any_sync(0xffffffffu, need))
         best = rerank64_warp(d, m, T.s, T.i0, T.j0, T.ok, need, c.x, c.y, W, E[0], E[1], E[2], G[0], G[1], G[2], re,
@@ -443,7 +443,6 @@ __device__ __forceinline__ int2 rank_list(const DemView& d, const MixedCtx& m, c
         const float* E = l.E32;
         const float* G = l.G32;
         const float re = __fdividef(l.nE, l.nG);
-        const float tie = kTieM / l.nG;
         float v1 = INFINITY, v2 = INFINITY;
 #pragma unroll 1
         for (int k = 0; k < H.m; k++) {
@@ -462,6 +461,7 @@ __device__ __forceinline__ int2 rank_list(const DemView& d, const MixedCtx& m, c
             v1 = p ? L : v1;
             c = p ? k : c;
         }
+        const float tie = tie_band(m, l.nG, v1);
         if (!(v2 - v1 >= tie))
             c = rerank_list(d, list, H.m, H.mode & kCore, H.i0, H.j0, st.x, st.y, W, E[0], E[1], E[2], G[0], G[1], G[2], re,
                             v1 + tie, l.E[0], l.E[1], l.E[2], l.G[0], l.G[1], l.G[2], l.nE64, l.nG64, c);
@@ -643,6 +643,7 @@ __device__ __forceinline__ MixedCtx req_ctx(const MixedReq& r)
     m.istepy = r.istepy;
     m.ox = r.ox;
     m.oy = r.oy;
+    m.oz = r.a.dem.z0;
     m.idx64 = r.idx64;
     m.idy64 = r.idy64;
     m.start_band = r.start_band;
@@ -686,7 +687,7 @@ __device__ __forceinline__ void voxel_mixed(const BpArgs& a, const MixedCtx& m, 
     const int64_t nr = a.nr;
     const int3 vx = voxel_at(a, compact, kk < a.v_count ? kk : a.v_count - 1);
     const double P[3] = {__ldg(a.gx + vx.x), __ldg(a.gy + vx.y), __ldg(a.gz + vx.z)};
-    const float P32[3] = {(float)(P[0] - m.ox), (float)(P[1] - m.oy), (float)P[2]};
+    const float P32[3] = {(float)(P[0] - m.ox), (float)(P[1] - m.oy), (float)(P[2] - m.oz)};
     const VoxelStart vs{height32(m, P32[0], P32[1]), dem_elevation(a.dem, P[0], P[1])};
     const WarpVoxels wv = warp_voxels(P32);
     if (lane < 2) ws->h[lane].si = ws->h[lane].sj = -1;
@@ -746,7 +747,7 @@ __device__ __forceinline__ void voxel_mixed(const BpArgs& a, const MixedCtx& m, 
                         for (int c = 0; c < 3; c++) l.E[c] = __ldg(tr + c);
                         l.E32[0] = (float)(l.E[0] - m.ox);
                         l.E32[1] = (float)(l.E[1] - m.oy);
-                        l.E32[2] = (float)l.E[2];
+                        l.E32[2] = (float)(l.E[2] - m.oz);
                         if (hm < 0) {
                             const Leg lc = l;
                             node = scan_warp<WT>(a.dem, m, T, ws->u.table, lc, vs, a.W);

@@ -39,10 +39,10 @@ struct Heights64 {
     const DemView& d;
     __device__ __forceinline__ explicit Heights64(const DemView& d_) : d(d_) {}
     __device__ __forceinline__ void cover(int, int, int, int) {}
-    __device__ __forceinline__ float operator()(int i, int j) const { return (float)__ldg(d.z + (int64_t)j * d.nx + i); }
+    __device__ __forceinline__ float operator()(int i, int j) const { return (float)(__ldg(d.z + (int64_t)j * d.nx + i) - d.z0); }
     __device__ __forceinline__ float ground(float x, float y) const
     {
-        return (float)dem_elevation(d, (double)x + d.x0, (double)y + d.y0);
+        return (float)(dem_elevation(d, (double)x + d.x0, (double)y + d.y0) - d.z0);
     }
 };
 
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(32 * WPC, WPC < 8 ? 12 / WPC : 16 / WPC)
     const int64_t kk = (int64_t)blockIdx.x * 32 + lane;
     const int3 vx = voxel_at(a, compact, kk < a.v_count ? kk : a.v_count - 1);
     const double P[3] = {__ldg(a.gx + vx.x), __ldg(a.gy + vx.y), __ldg(a.gz + vx.z)};
-    const float P32[3] = {(float)(P[0] - d.x0), (float)(P[1] - d.y0), (float)P[2]};
+    const float P32[3] = {(float)(P[0] - d.x0), (float)(P[1] - d.y0), (float)(P[2] - d.z0)};
     const double h64 = dem_elevation(d, P[0], P[1]);
     const WarpVoxels wv = warp_voxels(P32);
     if (threadIdx.x == 0) next = WPC;   // the parts after the first WPC go to the warps that are done
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(32 * WPC, WPC < 8 ? 12 / WPC : 16 / WPC)
         double accr = 0.0, acci = 0.0;
         int n;
         for (int i = p0; i < p1; i += n) {
-            n = pulse_block(m, zat, d, ws->l, ws->h, a.tx, a.rx, i, p1, d.x0, d.y0, P, P32, (float)h64, wv, a.n1, a.n2, a.W,
+            n = pulse_block(m, zat, d, ws->l, ws->h, a.tx, a.rx, i, p1, d.x0, d.y0, P, P32, (float)(h64 - d.z0), wv, a.n1, a.n2, a.W,
                             kBlockSlope, !a.exhaustive);
             const int m0 = all_pinned(ws->h[0]) ? ws->h[0].m : 0, m1 = all_pinned(ws->h[1]) ? ws->h[1].m : 0;
             for (int b = 0; b < n; b += kPathPulses) {

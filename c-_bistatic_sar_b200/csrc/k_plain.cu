@@ -173,7 +173,7 @@ template <> struct BpShared<2> { using T = FilterCols<128>; };
 // SOLVER: 0 grid search, 1 Newton, 2 grid search behind the FP32 filter (the same image;
 // zlo, zhi: the DEM's range of heights).
 template <int SOLVER, int LEGS>
-__global__ void __launch_bounds__(128) k_bp_plain(BpArgs a, float zlo, float zhi)
+__global__ void __launch_bounds__(128, SOLVER == 2 ? 6 : 4) k_bp_plain(BpArgs a, float zlo, float zhi)
 {
     __shared__ typename BpShared<SOLVER>::T sh;
     const int pitch = (a.dem.nx + 3) & ~3;

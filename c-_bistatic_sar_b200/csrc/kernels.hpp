@@ -103,7 +103,7 @@ struct BpArgs {
     int W;                // Newton node-scan half width
     int64_t v_begin, v_count;  // voxel range, reference flat order (z -> x -> y)
     double2* out;         // image [x][y][z]
-    float zlo, zhi;       // the DEM's range of heights (FP64 grid search)
+    float zlo, zhi;       // the DEM's range of heights in the FP32 frame (FP64 grid search)
     int exhaustive;       // FP64 Newton: 1, node scans rank every node (no candidate lists); the image is the same
     // mixed form: per-pulse FP64 reference optical path and reduced carrier phase
     const double* ref_L;    // np

@@ -19,7 +19,7 @@ struct Facet32 {
 struct MixedCtx : ListGrid {
     const float* __restrict__ z32;  // pitch-padded FP32 heights, z32[j * pitch + i]
     int pitch;
-    double ox, oy;                  // origin of the FP32 frame (first DEM node)
+    double ox, oy, oz;              // origin of the FP32 frame (first DEM node, DemView::z0)
     double idx64, idy64;            // 1 / spacing, FP64
     int lists;                      // node scans may run on candidate lists
 };

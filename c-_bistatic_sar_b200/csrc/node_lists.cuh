@@ -15,14 +15,17 @@ namespace bsar {
 // error of a node's ranking value measured against FP64 over 6e9 medium-scene solves was
 // 4.8e-6 m (in units of L / ng), so two nodes are mis-ordered only within ~1e-5 m.
 constexpr float kTieM = 5.0e-5f;
+// Longer paths round coarser: 1.6e-7 of the value each, as measured, and the coordinates of a
+// DEM that is kilometres wide.  Below 50 m of value on DEMs up to 100 m it is the band above.
+constexpr float kTieRel = 4.0e-7f, kTieExtent = 1.0e-7f;
 // A FP32 flat start closer than this to a node-cell boundary is redone in FP64: metres
 // of start-position error (the largest measured FP32 start error was 3.1e-5 node units,
 // 7.6e-6 m) plus the FP32 quantisation of the node coordinate (ulps of the largest index).
 constexpr float kStartBandM = 2.5e-5f;
 constexpr float kStartBandUlps = 8.0f;
 
-// The DEM as the lists see it: sizes, FP32 spacing (and its reciprocal), the FP32 frame's
-// origin is the first node.
+// The DEM as the lists see it: sizes, FP32 spacing (and its reciprocal); the FP32 frame's
+// origin is the first node and, in z, DemView::z0.
 struct ListGrid {
     int nx, ny;
     float stepx, stepy;             // uniform node spacing
@@ -30,6 +33,12 @@ struct ListGrid {
     float start_band;               // node units: FP32 starts this close to a cell boundary go FP64
     float extent;                   // largest coordinate of the FP32 frame
 };
+
+// Tie band of ranking values around v (L / ng).
+__device__ __forceinline__ float tie_band(const ListGrid& m, float ng, float v)
+{
+    return fmaxf(kTieM / ng, fmaf(kTieRel, v, kTieExtent * m.extent));
+}
 
 // Start band of a DEM (node units), see kStartBandM.
 inline __host__ __device__ float list_start_band(const DemView& d)
@@ -344,6 +353,13 @@ __device__ __forceinline__ bool gap_keep(const GapRef& g, float x, float y, floa
     return t <= 0.0f || a * a <= s2 * (b * b) * 1.00001f;
 }
 
+// The tie band and a margin for the FP32 rounding of a gap: of its two distances, and of the
+// coordinates of S and of the nodes that can win, which lie within the distances of S.
+__device__ __forceinline__ float gap_margin(const ListGrid& m, const GapRef& g, float nG)
+{
+    return tie_band(m, nG, g.eS + g.gS) + 1e-4f + 2e-6f * (g.eS + g.gS) + 5e-7f * (m.extent + fabsf(g.S[2]));
+}
+
 // (float)i for 0 <= i < 2^23 without the conversion unit.
 __device__ __forceinline__ float small_float(int i) { return __int_as_float(0x4b000000 | i) - 8388608.0f; }
 
@@ -415,7 +431,7 @@ __device__ __forceinline__ void build_list(const ListGrid& m, Z zat, float4* lis
     bool outside = false;
 #pragma unroll 1
     for (int attempt = 0; attempt < 2; attempt++) {
-        const float thr = kTieM / nG + 1e-4f + 2e-6f * (g.eS + g.gS) + 5e-7f * m.extent;
+        const float thr = gap_margin(m, g, nG);
         float best = INFINITY;
         int bij = 0;
         int i = ua + li, j = va + lane - li * nj;
@@ -463,7 +479,7 @@ __device__ __forceinline__ void build_list(const ListGrid& m, Z zat, float4* lis
         gap_set(g, small_float(si) * m.stepx, small_float(sj) * m.stepy, zat(si, sj));
         if (cnt <= kListCap) {
             // list against the better S, in place and in order
-            const float thr2 = kTieM / nG + 1e-4f + 2e-6f * (g.eS + g.gS) + 5e-7f * m.extent;
+            const float thr2 = gap_margin(m, g, nG);
             const int c0 = cnt;
             cnt = 0;
             outside = false;
@@ -504,7 +520,10 @@ __device__ __forceinline__ void build_list(const ListGrid& m, Z zat, float4* lis
 // the derivative is nE u_E.t + nG u_G.t (u: unit vectors from the endpoints), and u turns by
 // at most 2 r / (2 |N - Ec| - r) over a distance r.  Then each of the four facets has its
 // minimum at the node (the corner test of finish_leg), with a margin far above the FP32
-// rounding of the derivatives.  Nodes on the DEM's border have missing facets: never.
+// rounding of the derivatives: of the coordinates (as if the antenna and the voxel moved by
+// it) and of the slopes, two heights' rounding over the spacing (a neighbour's height is the
+// node's and a rise, whose rounding is far below the margin).  Nodes on the DEM's border have
+// missing facets: never.
 template <typename Z>
 __device__ __forceinline__ bool node_pinned(const ListGrid& m, const Z& zat, int i, int j, const float E[3], const float G[3], float rE,
                                             float rG, float nE, float nG)
@@ -513,6 +532,10 @@ __device__ __forceinline__ bool node_pinned(const ListGrid& m, const Z& zat, int
     const float z = zat(i, j);
     const float sxb = (z - zat(i - 1, j)) * m.istepx, sxf = (zat(i + 1, j) - z) * m.istepx;
     const float syb = (z - zat(i, j - 1)) * m.istepy, syf = (zat(i, j + 1) - z) * m.istepy;
+    const float round = 2.5e-7f * (m.extent + fabsf(z));
+    const float slope = 1.3e-7f * (nE + nG) * fabsf(z) * fmaxf(m.istepx, m.istepy);
+    rE += round;
+    rG += round;
     const float x = (float)i * m.stepx, y = (float)j * m.stepy;
     const float ex = x - E[0], ey = y - E[1], ez = z - E[2];
     const float gx = x - G[0], gy = y - G[1], gz = z - G[2];
@@ -523,8 +546,8 @@ __device__ __forceinline__ bool node_pinned(const ListGrid& m, const Z& zat, int
     if (!(dE > rE && dG > rG)) return false;
     const float turn = 2.0f * (nE * __fdividef(rE, dE) + nG * __fdividef(rG, dG)) + 1e-5f * (nE + nG);
     auto tangent = [](float sl) { return sqrtf(1.0f + sl * sl); };
-    return fmaf(Fz, sxf, Fx) > turn * tangent(sxf) && -fmaf(Fz, sxb, Fx) > turn * tangent(sxb) &&
-           fmaf(Fz, syf, Fy) > turn * tangent(syf) && -fmaf(Fz, syb, Fy) > turn * tangent(syb);
+    return fmaf(Fz, sxf, Fx) > turn * tangent(sxf) + slope && -fmaf(Fz, sxb, Fx) > turn * tangent(sxb) + slope &&
+           fmaf(Fz, syf, Fy) > turn * tangent(syf) + slope && -fmaf(Fz, syb, Fy) > turn * tangent(syb) + slope;
 }
 
 // Short lists (kTables): nE |N - E| of every listed node and pulse of the block and
@@ -586,7 +609,7 @@ __device__ __forceinline__ WarpVoxels warp_voxels(const float P[3])
 
 // Takes the next pulse block, from pulse i (< np): as many pulses as keep both antennas close
 // together, and both legs' lists for it (all 32 lanes call; P, P32, h0: the lane's voxel in
-// FP64 and in the FP32 frame and the height under it).  `slope` bounds the antennas' movement
+// FP64 and in the FP32 frame and the height under it there).  `slope` bounds the antennas' movement
 // from the block's first pulse: re * distance / |E - G| stays below twice it, which sets the
 // lists' slack and with it their length.  Returns the number of pulses, at most kBlockPulses.  Both
 // legs have a list or neither (m = -1), as when `lists` is false.
@@ -607,7 +630,7 @@ __device__ __forceinline__ int pulse_block(const ListGrid& m, Z zat, const DemVi
         const double* tr = (leg ? rx : tx) + 3 * pl;
         e[leg][0] = (float)(__ldg(tr) - ox);
         e[leg][1] = (float)(__ldg(tr + 1) - oy);
-        e[leg][2] = (float)__ldg(tr + 2);
+        e[leg][2] = (float)(__ldg(tr + 2) - d.z0);
         const float dx = e[leg][0] - __shfl_sync(full, e[leg][0], 0);
         const float dy = e[leg][1] - __shfl_sync(full, e[leg][1], 0);
         const float dz = e[leg][2] - __shfl_sync(full, e[leg][2], 0);

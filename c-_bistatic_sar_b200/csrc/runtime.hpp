@@ -329,6 +329,23 @@ inline bool equally_spaced(const double* v, int64_t n)
     return true;
 }
 
+// Height origin of the FP32 frame: the median of up to 257 nodes, to 64 m.  FP32 heights near
+// it round below 2e-6 m wherever the terrain lies, and outliers (no-data values) do not move it;
+// terrain within 32 m of zero keeps the origin 0.
+inline double height_origin(const bsar_dem* d)
+{
+    const int64_t n = d->nx * d->ny, m = std::min<int64_t>(n, 257);
+    std::vector<double> v;
+    v.reserve((size_t)m);
+    for (int64_t k = 0; k < m; k++) {
+        const double z = d->z[m > 1 ? k * (n - 1) / (m - 1) : 0];
+        if (std::isfinite(z)) v.push_back(z);
+    }
+    if (v.empty()) return 0.0;
+    std::nth_element(v.begin(), v.begin() + v.size() / 2, v.end());
+    return 64.0 * std::nearbyint(v[v.size() / 2] / 64.0);
+}
+
 inline DemDev stage_dem(bsar_ctx* ctx, const bsar_dem* d, bool want_z32)
 {
     check_dem(d);
@@ -362,13 +379,14 @@ inline DemDev stage_dem(bsar_ctx* ctx, const bsar_dem* d, bool want_z32)
     v.y0 = d->y_vec[0];
     v.stepx = d->nx > 1 ? (d->x_vec[d->nx - 1] - d->x_vec[0]) / (double)(d->nx - 1) : 1.0;
     v.stepy = d->ny > 1 ? (d->y_vec[d->ny - 1] - d->y_vec[0]) / (double)(d->ny - 1) : 1.0;
+    v.z0 = want_z32 ? height_origin(d) : 0.0;
     if (want_z32) {
         // rows padded to a multiple of 4 floats: 16-byte tensor-map strides
         r.pitch = (int)((d->nx + 3) & ~int64_t(3));
         std::vector<float> zf((size_t)r.pitch * d->ny, 0.0f);
         for (int64_t j = 0; j < d->ny; j++)
             for (int64_t i = 0; i < d->nx; i++) {
-                const float z = (float)d->z[j * d->nx + i];
+                const float z = (float)(d->z[j * d->nx + i] - v.z0);
                 zf[j * r.pitch + i] = z;
                 r.zlo = std::min(r.zlo, z);
                 r.zhi = std::max(r.zhi, z);

@@ -64,3 +64,48 @@ def _lists_equal_exhaustive(ctx, name, precision):
         ctx.scene_release(sid)
     assert np.abs(full).max() > 0
     assert np.array_equal(lists, full)
+
+
+# name: (scale of all lengths, height added to everything, scene fields, voxel clusters)
+PLACES = {
+    "terrain at 300 m": (1, 300.0, {}, False),
+    "terrain at 2000 m": (1, 2000.0, {}, False),
+    "terrain at 8000 m": (1, 8000.0, {}, False),
+    "terrain at -9000 m": (1, -9000.3, {}, False),
+    "smooth at 8000 m": (1, 8000.0, dict(dem_sigma=0.002, dem_kind="plane"), False),
+    "one pulse at 8000 m": (1, 8000.0, dict(n_pulses=1), True),
+    "one pulse": (1, 0.0, dict(n_pulses=1), True),
+    "paths of 1 km": (20, 0.0, {}, False),
+    "paths of 5 km": (100, 0.0, {}, False),
+    "paths of 5 km, flat": (100, 0.0, dict(dem_sigma=0.03), False),
+    "paths of 15 km": (300, 0.0, {}, False),
+    "dem of 1.5 km": (1, 0.0, dict(dem_d=0.37, dem_n=4000), False),
+}
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("name", PLACES)
+def test_lists_far_from_the_origin(ctx, name, precision):
+    """Heights, coordinates and paths whose FP32 rounding is far above that of the scenes above;
+    clusters of voxels micrometres apart and one pulse leave the lists' bounds no slack."""
+    k, shift, kw, clusters = PLACES[name]
+    spec = S.scaled(S.config_spec(2), **{**dict(n_pulses=120, n_samples=4096, n_scatterers=2, nx=24, ny=23, nz=4), **kw})
+    sc = S.make_scene(spec, with_raw=False)
+    up = np.array([0.0, 0.0, shift])
+    rng = np.random.default_rng(5)
+    data = rng.normal(size=(spec.n_pulses, 4096)) + 1j * rng.normal(size=(spec.n_pulses, 4096))
+    axes = [sc.gx, sc.gy, sc.gz]
+    if clusters:
+        c = np.arange(4) * 1e-6
+        axes = [(np.linspace(17, 23, 60)[:, None] + c).ravel(), (np.linspace(-3, 3, 60)[:, None] + c).ravel(), -5.0 + c[:2]]
+    dem = bsar.DemArrays(sc.x_vec * k, sc.y_vec * k, sc.z * k + shift)
+    sid = ctx.scene_upload(dem, sc.tx * k + up, sc.rx * k + up, data, kind="compressed", upsample=2, n1=1.0, n2=6.0 ** 0.5,
+                           c=3e8, fc=1e9 / k, fs=1.92e9 / k)
+    how = dict(solver="newton", legs="per_pulse", precision=precision, search_radius_m=1.5 * k)
+    try:
+        full = ctx.backproject(sid, axes[0] * k, axes[1] * k, axes[2] * k + shift, exhaustive=True, **how)
+        lists = ctx.backproject(sid, axes[0] * k, axes[1] * k, axes[2] * k + shift, **how)
+    finally:
+        ctx.scene_release(sid)
+    assert np.abs(full).min() > 0
+    assert np.array_equal(lists, full)

@@ -49,6 +49,29 @@ def test_newton_image_matches_the_oracle(ctx, oracle, name):
     assert rel_l2(img, want) <= 1e-9
 
 
+@pytest.mark.parametrize("height", [300.0, 2000.0, 8000.0, -9000.3])
+@pytest.mark.parametrize("n_pulses", [1, 50])
+def test_raised_terrain(ctx, oracle, height, n_pulses):
+    """Terrain, antennas and voxels far above or below zero, where FP32 heights round at up to
+    half a millimetre: the image is still the oracle's."""
+    spec = S.scaled(S.config_spec(2), n_pulses=n_pulses, n_samples=4096, n_scatterers=2, nx=9, ny=10, nz=2)
+    sc = S.make_scene(spec, with_raw=False)
+    rng = np.random.default_rng(5)
+    sc.raw = rng.normal(size=(n_pulses, 4096)) + 1j * rng.normal(size=(n_pulses, 4096))
+    up = np.array([0.0, 0.0, height])
+    sc.z, sc.tx, sc.rx, sc.gz = sc.z + height, sc.tx + up, sc.rx + up, sc.gz + height
+    sid = bsar.upload_scene(ctx, sc)
+    try:
+        img = ctx.backproject(sid, sc.gx, sc.gy, sc.gz, solver="newton", legs="per_pulse", precision="fp64")
+    finally:
+        ctx.scene_release(sid)
+    rc = oracle.spline_upsample(oracle.fft_correlate(sc.raw, sc.reference), spec.upsample)
+    want = oracle.backproject(O.Dem(sc.x_vec, sc.y_vec, sc.z), sc.tx, sc.rx, rc, sc.gx, sc.gy, sc.gz, spec.n1, spec.n2,
+                              3e8, sc.fs_eff, sc.lam, legs="per", solver="newton",
+                              search_nodes=S.search_nodes_for(sc.x_vec, sc.y_vec))
+    assert rel_l2(img, want) <= 1e-9
+
+
 @pytest.mark.parametrize("n_pulses", [1, 7, 50])
 def test_large_grid_has_the_small_grids_image(ctx, n_pulses):
     """114000 voxels take two warps per 32 voxels, their first three x planes four: both within
