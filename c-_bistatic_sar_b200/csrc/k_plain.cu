@@ -391,8 +391,7 @@ cudaError_t launch_bp_plain(const BpArgs& a, int solver, int legs, cudaStream_t 
     // one warp per voxel; 4 warps per CTA; enough CTAs to cover the voxel range
     int64_t ctas = (a.v_count + 3) / 4;
     int blocks = (int)(ctas > (int64_t)148 * 512 ? (int64_t)148 * 512 : (ctas < 1 ? 1 : ctas));
-    const DemView& d = a.dem;
-    const bool filter = solver == 0 && !d.empty && d.uniform && d.nx >= 2 && d.ny >= 2 && d.z32 && a.n1 > 0 && a.n2 > 0;
+    const bool filter = solver == 0 && grid_filter_ok(a);
     const float zlo = a.zlo, zhi = a.zhi;
     if (filter && legs == 0) k_bp_plain<2, 0><<<blocks, 128, 0, st>>>(a, zlo, zhi);
     else if (filter) k_bp_plain<2, 1><<<blocks, 128, 0, st>>>(a, zlo, zhi);

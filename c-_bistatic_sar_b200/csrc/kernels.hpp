@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdint>
 
 #include "dev_view.hpp"
@@ -185,6 +186,17 @@ struct MixedBatch {
     const MixedChunks* chunks;   // per request, indexed as reqs (the chunked kernel only)
     long long wait_polls;        // polls of the bounded DEM-tile wait before giving up on a tile
 };
+
+// Whether the FP64 grid search runs behind its FP32 filter (dev_common.cuh): positive indices,
+// evenly spaced axes of at least two nodes, FP32 heights that are finite (a finite FP64 height may
+// not be) and whose offsets fit the filter's 32 bits.  Everything else takes the plain search.
+inline bool grid_filter_ok(const BpArgs& a)
+{
+    const DemView& d = a.dem;
+    const int64_t pitch = ((int64_t)d.nx + 3) & ~int64_t(3);
+    return !d.empty && d.uniform && d.nx >= 2 && d.ny >= 2 && d.z32 && a.n1 > 0 && a.n2 > 0 &&
+           std::isfinite(a.zlo) && std::isfinite(a.zhi) && pitch * d.ny <= 0x7fffffff;
+}
 
 cudaError_t launch_bp_plain(const BpArgs& a, int solver, int legs, cudaStream_t st);
 // FP64 Newton, per-pulse legs, a DEM of at least 2 x 2 nodes
