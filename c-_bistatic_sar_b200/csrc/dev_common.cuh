@@ -263,19 +263,21 @@ __device__ __forceinline__ void refraction_grid_warp(const DemView& d, double x1
 //   upper bound   the path at the level's centre point, which is one of its points (level 0)
 //                 or the point the search already holds (later levels); then the smallest
 //                 FP32 value plus its error bound
-//   error bound   2e-6 of the FP32 path plus 4e-7 (n1 + n2) of the heights' magnitudes: FP32
-//                 rounding of offsets, heights and square roots is below 5e-7 of them
+//   error bound   2e-6 of the FP32 path plus (n1 + n2) times 4e-7 of the endpoints' heights and
+//                 2.5e-6 of the DEM's largest: FP32 rounding of offsets, heights and square
+//                 roots is below 5e-7 of them, and an interpolated height is off by the
+//                 weights' 3.6e-7 times the span of its cell's corners, per axis
 //   rows, columns a row's path is at least n1 sqrt(dx1^2 + h1^2) + n2 sqrt(dx2^2 + h2^2), h1
 //                 and h2 the endpoints' distances from the DEM's range of heights; rows and
 //                 columns above the bound for every lane are skipped
 //   outside       an axis value within 1e-9 of the DEM's edge (relative) may fall on either
 //                 side of it, where the lookup jumps: always evaluated
-// Needs indices above zero, evenly spaced axes, at least 2 x 2 nodes, and the FP32 heights.
-// All 32 lanes call.  TPB: the block size.
+// Where it holds: grid_filter_ok (kernels.hpp).  All 32 lanes call.  TPB: the block size.
 // What bounds it: FP32 issue and the FP64 evaluations left (one to three points a level).
-// 41 x 41 x 21 voxels x 256 pulses, mean legs, with upload and upsampling: 107 -> 23.8 ms on
-// one B200 against every point in FP64 (grid_level); an occupancy of 4 CTAs instead of 5:
-// 25.6 ms.
+// 41 x 41 x 21 voxels x 256 pulses, mean legs, with upload and upsampling: 107 -> 23.4 ms on
+// one B200 against every point in FP64 (grid_level).  That is at six CTAs per SM (80 registers);
+// four, which the compiler takes by itself, 25.2 ms; five 27 to 32, seven 29 ms (spills in the
+// point loop).
 template <int TPB> struct FilterCols {
     float4 c[15][TPB];     // (y - y1)^2, (y - y2)^2, weight, row offset (int; < 0: at the edge)
 };
@@ -323,9 +325,9 @@ __device__ __forceinline__ void grid_level_filter(const DemView& d, int pitch, f
     };
     const int t = threadIdx.x;
     const float n1f = (float)n1, n2f = (float)n2;
-    const float zerr = 4e-7f * (n1f + n2f);
     const float z1f = (float)(z1 - d.z0), z2f = (float)(z2 - d.z0);
-    const float base_err = zerr * (fabsf(z1f) + fabsf(z2f));
+    const float base_err = 4e-7f * (n1f + n2f) * (fabsf(z1f) + fabsf(z2f));
+    const float z_err = fmaf(2.5e-6f * (n1f + n2f), fmaxf(fabsf(zlo), fabsf(zhi)), base_err);
     double top = minOP;
     if (G == 15) top = fmin(top, point((G - 1) / 2, (G - 1) / 2).op);
     // bound of the level's minimum, rounded up
@@ -336,7 +338,7 @@ __device__ __forceinline__ void grid_level_filter(const DemView& d, int pitch, f
     auto far = [&](float a2, float b2) {      // a row or column none of whose points can win
         const float qa = a2 + h1, qb = b2 + h2;
         const float L = n1f * (qa * rsqrtf(fmaxf(qa, 1e-30f))) + n2f * (qb * rsqrtf(fmaxf(qb, 1e-30f)));
-        return L - 2e-6f * L - base_err - zerr * fmaxf(fabsf(zlo), fabsf(zhi)) > thr;
+        return L - 2e-6f * L - z_err > thr;
     };
     unsigned keep = 0;                        // columns to visit (of the warp)
 #pragma unroll 1
@@ -372,7 +374,7 @@ __device__ __forceinline__ void grid_level_filter(const DemView& d, int pitch, f
             const float dz1 = z - z1f, dz2 = z - z2f;
             const float q1 = fmaf(dz1, dz1, a2 + c.x), q2 = fmaf(dz2, dz2, b2 + c.y);
             const float L = n1f * (q1 * rsqrtf(fmaxf(q1, 1e-30f))) + n2f * (q2 * rsqrtf(fmaxf(q2, 1e-30f)));
-            const float err = fmaf(2e-6f, L, fmaf(zerr, fabsf(z), base_err));
+            const float err = fmaf(2e-6f, L, z_err);
             const bool edge = off < 0 || fx.edge;
             const float low = edge ? -INFINITY : L - err;
             thr = edge ? thr : fminf(thr, L + err);

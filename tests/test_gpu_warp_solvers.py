@@ -89,3 +89,33 @@ def test_filtered_grid_search_image(ctx, oracle, name, legs):
                               sc.fs_eff, sc.lam, legs="mean" if legs == "mean" else "per", solver="grid")
     assert np.abs(want).max() > 0
     assert rel_l2(img, want) <= 1e-11
+
+
+@pytest.mark.parametrize("value,share,seed", [(-9999.0, 0.2, 0), (-9999.0, 0.2, 1), (-32768.0, 0.02, 2),
+                                              (-32768.0, 0.2, 3), (1e4, 0.2, 0), (1e4, 0.2, 4), (3000.0, 0.2, 5),
+                                              (1e6, 0.2, 0), (3e38, 0.02, 1), (1e39, 0.02, 2), (-1e39, 0.2, 3)])
+def test_filtered_grid_search_beside_outliers(ctx, oracle, value, share, seed):
+    """No-data values and cliffs beside the terrain: the FP32 height of a point in such a cell
+    is off by far more than its own magnitude says."""
+    x, y, _ = _dem("plane")
+    rng = np.random.default_rng([seed, int(100 * share), int(min(abs(value), 1e6))])
+    z = rng.normal(0, 0.05, (40, 48))
+    out = rng.random(z.shape) < share
+    z[out] = value * (1 + 1e-3 * rng.normal(size=out.sum()))
+    n = 64
+    s = np.arange(n) / (n - 1)
+    th = 6 * np.pi * s
+    tx = np.stack([15 * (1 - s) * np.cos(th), 15 * (1 - s) * np.sin(th), np.full(n, 30.0)], 1)
+    rx = tx + [5.0, 0.0, 0.0]
+    axes = 20 + np.arange(8) * 0.37, -1 + np.arange(8) * 0.31, np.array([-6.0, -4.5, -3.0, -1.5])
+    data = rng.normal(size=(n, 1024)) + 1j * rng.normal(size=(n, 1024))
+    sid = ctx.scene_upload(bsar.DemArrays(x, y, z), tx, rx, data, kind="compressed", upsample=4, n1=1.0, n2=2.0, c=3e8,
+                           fc=1e9, fs=1.2e9)
+    try:
+        img = ctx.backproject(sid, *axes, solver="grid", legs="per_pulse", precision="fp64")
+    finally:
+        ctx.scene_release(sid)
+    want = oracle.backproject(O.Dem(x, y, z), tx, rx, oracle.spline_upsample(data, 4), *axes, 1.0, 2.0, 3e8, 4.8e9, 0.3,
+                              legs="per", solver="grid")
+    assert np.abs(want).max() > 0
+    assert rel_l2(img, want) <= 1e-11
