@@ -470,7 +470,7 @@ static void backproject(bsar_ctx* ctx, bsar_scene_id id, const bsar_grid* g, con
     a.out = d_out;
     a.zlo = s->dem.zlo;
     a.zhi = s->dem.zhi;
-    a.exhaustive = (o->flags & BSAR_BP_EXHAUSTIVE_SCAN) ? 1 : 0;
+    a.exhaustive = (o->flags & BSAR_BP_EXHAUSTIVE_SCAN) || !lists_hold(a.n1, a.n2) ? 1 : 0;
     if (o->precision == BSAR_FP64) {
         launched(ctx, launch_bp_plain(a, o->solver, o->legs, ctx->stream), "back-projection (FP64)");
         return;

@@ -187,6 +187,14 @@ struct MixedBatch {
     long long wait_polls;        // polls of the bounded DEM-tile wait before giving up on a tile
 };
 
+// Whether node scans may run on candidate lists, whose slack takes the ratio of the indices as
+// a weight: both are positive numbers, in FP32 too.
+inline bool lists_hold(double n1, double n2)
+{
+    const float a = (float)n1, b = (float)n2;
+    return a > 0.0f && b > 0.0f && std::isfinite(a) && std::isfinite(b);
+}
+
 // Whether the FP64 grid search runs behind its FP32 filter (dev_common.cuh): positive indices,
 // evenly spaced axes of at least two nodes, FP32 heights that are finite (a finite FP64 height may
 // not be) and whose offsets fit the filter's 32 bits.  Everything else takes the plain search.

@@ -280,9 +280,10 @@ __device__ __forceinline__ bool lower_is_voxel(float nE, float nG, bool to_voxel
 // intersection.  When all listed nodes lie in the intersection the starts themselves are
 // not needed; otherwise each solve makes its start and drops the nodes outside its window.
 //
-// No list (m = -1): antenna on the side of the larger index, start not converged,
-// intersection empty, or more nodes than the list holds; those blocks scan every window
-// node (scan_warp), as the exhaustive flag does.
+// No lists at all for indices that are not positive (lists_hold, kernels.hpp).  No list for a
+// block (m = -1): antenna on the side of the larger index, start not converged, intersection
+// empty, or more nodes than the list holds; those blocks scan every window node (scan_warp),
+// as the exhaustive flag does.
 constexpr int kListCap = 128;
 constexpr int kBlockPulses = 32;    // longest pulse block
 

@@ -790,7 +790,7 @@ inline MixedReq mixed_request(const Scene* s, const BpArgs& a, bool fp16, int32_
     r.pitch = s->dem.pitch;
     r.use_tile = s->dem.has_tmap ? 1 : 0;
     r.fp16 = fp16 ? 1 : 0;
-    r.exhaustive = (flags & BSAR_BP_EXHAUSTIVE_SCAN) ? 1 : 0;
+    r.exhaustive = (flags & BSAR_BP_EXHAUSTIVE_SCAN) || !lists_hold(a.n1, a.n2) ? 1 : 0;
     const int64_t plane = (int64_t)a.nx * a.ny;
     r.compact = (a.v_begin % plane == 0 && a.v_count % plane == 0) ? 1 : 0;
     r.stepx = (float)s->dem.view.stepx;

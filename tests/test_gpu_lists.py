@@ -109,3 +109,24 @@ def test_lists_far_from_the_origin(ctx, name, precision):
         ctx.scene_release(sid)
     assert np.abs(full).min() > 0
     assert np.array_equal(lists, full)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("scene", [dict(dem_d=0.1, dem_n=400), dict(dxy=0.2, dz=0.3), dict(dxy=0.2, dem_n=14)])
+@pytest.mark.parametrize("n1,n2", [(-1.0, 8.0), (-0.3, 2.0), (8.0, -0.1), (0.0, 2.0), (2.0, 0.0), (1e-50, 2.0)])
+def test_indices_without_lists(ctx, n1, n2, scene, precision):
+    """Any finite index is accepted; the lists' bounds hold for positive ones only."""
+    sc = S.make_scene(S.scaled(S.config_spec(2), **{**dict(n_pulses=100, n_samples=4096, n_scatterers=2, nx=25, ny=26, nz=3),
+                                                    **scene}), with_raw=False)
+    rng = np.random.default_rng(5)
+    data = rng.normal(size=(100, 4096)) + 1j * rng.normal(size=(100, 4096))
+    sid = ctx.scene_upload(bsar.DemArrays(sc.x_vec, sc.y_vec, sc.z), sc.tx, sc.rx, data, kind="compressed", upsample=2, n1=n1,
+                           n2=n2, c=3e8, fc=1e9, fs=1.92e9)
+    how = dict(solver="newton", legs="per_pulse", precision=precision)
+    try:
+        full = ctx.backproject(sid, sc.gx, sc.gy, sc.gz, exhaustive=True, **how)
+        lists = ctx.backproject(sid, sc.gx, sc.gy, sc.gz, **how)
+    finally:
+        ctx.scene_release(sid)
+    assert np.abs(full).max() > 0
+    assert np.array_equal(lists, full)
