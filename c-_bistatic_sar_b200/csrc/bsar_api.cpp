@@ -481,27 +481,29 @@ static void backproject(bsar_ctx* ctx, bsar_scene_id id, const bsar_grid* g, con
     MixedReq r = mixed_request(s, a, o->precision == BSAR_MIXED_FP16, o->flags);
     // small grids: each tile's pulses in K chunks, so the work items fill the GPU
     const int64_t vtiles = (a.v_count + 127) / 128;
-    int K = mixed_chunks(nv_grid, a.np);
+    const int K = mixed_chunks(nv_grid, a.np);
+    const size_t part_bytes = sizeof(double2) * (size_t)K * (size_t)nv_grid, done_bytes = sizeof(int) * (size_t)vtiles;
     std::unique_ptr<DevBuf> partial, tile_done, chunks;
-    // a budget that has no room for the chunks' sums takes the whole pulse range at once
-    if (ctx->used + sizeof(double2) * (size_t)K * (size_t)nv_grid + sizeof(int) * (size_t)vtiles + sizeof(MixedChunks) >
-        ctx->budget)
-        K = 1;
-    if (K > 1) {
-        partial = dev_alloc(ctx, sizeof(double2) * (size_t)K * (size_t)(g->nx * g->ny * g->nz));
-        tile_done = dev_alloc(ctx, sizeof(int) * (size_t)vtiles);
-        cuda_check(cudaMemsetAsync(tile_done->p, 0, sizeof(int) * (size_t)vtiles, ctx->stream), "memset");
+    // a budget that has no room for the chunks' sums: the chunks in turn, added to the image
+    const bool in_turn = K > 1 && ctx->used + part_bytes + done_bytes + sizeof(MixedChunks) > ctx->budget;
+    if (K > 1 && !in_turn) {
+        partial = dev_alloc(ctx, part_bytes);
+        tile_done = dev_alloc(ctx, done_bytes);
+        cuda_check(cudaMemsetAsync(tile_done->p, 0, done_bytes, ctx->stream), "memset");
         const MixedChunks c{K, 0, partial->as<double2>(), tile_done->as<int>()};
         chunks = dev_upload(ctx, &c, sizeof c);
     }
-    cuda_check(cudaMemcpyAsync(ctx->mixed_req->p, &r, sizeof r, cudaMemcpyHostToDevice, ctx->stream), "h2d");
-    cuda_check(cudaMemsetAsync(ctx->mixed_counter->p, 0, sizeof(int), ctx->stream), "memset");
-    MixedBatch b{ctx->mixed_req->as<MixedReq>(), nullptr, nullptr, (int)(vtiles * K),
+    MixedBatch b{ctx->mixed_req->as<MixedReq>(), nullptr, nullptr, (int)(in_turn ? vtiles : vtiles * K),
                  ctx->mixed_counter->as<int>(), ctx->status->as<int>(), chunks ? chunks->as<MixedChunks>() : nullptr,
-                 (long long)ctx->tile_wait_polls};
+                 (long long)ctx->tile_wait_polls, 0};
     const int grid = (int)std::min<int64_t>(b.ntiles, mixed_grid_ctas());
-    cudaError_t e = launch_bp_mixed(b, a.W, grid, ctx->stream, K > 1);
-    launched(ctx, e, "back-projection (mixed)");
+    for (int c = 0; c < (in_turn ? K : 1); c++) {
+        const MixedReq rc = in_turn ? mixed_chunk_request(r, c, K) : r;
+        b.add = in_turn ? (c ? 2 : 1) : 0;
+        cuda_check(cudaMemcpyAsync(ctx->mixed_req->p, &rc, sizeof rc, cudaMemcpyHostToDevice, ctx->stream), "h2d");
+        cuda_check(cudaMemsetAsync(ctx->mixed_counter->p, 0, sizeof(int), ctx->stream), "memset");
+        launched(ctx, launch_bp_mixed(b, a.W, grid, ctx->stream, K > 1), "back-projection (mixed)");
+    }
 }
 
 bsar_status bsar_set_tile_wait_limit(bsar_ctx* ctx, int64_t polls)

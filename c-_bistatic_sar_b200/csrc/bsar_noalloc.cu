@@ -80,14 +80,14 @@ extern "C" bsar_status bsar_backproject_mixed_noalloc(bsar_ctx* ctx, bsar_scene_
         const size_t o_axes = o_off + up256(32 * (size_t)np);
         const size_t o_img = o_axes + up256(8 * (size_t)(g->nx + g->ny + g->nz));
         const int64_t vtiles = (nv + 127) / 128;
-        int K = mixed_chunks(nv, (int)np);
+        const int K = mixed_chunks(nv, (int)np);
         const size_t o_chk = o_img + up256(16 * (size_t)nv);
         const size_t o_part = o_chk + up256(sizeof(MixedChunks));
-        auto part_bytes = [&] { return up256(16 * (size_t)K * (size_t)nv); };
-        // a scratch that has no room for the chunks' sums takes the whole pulse range at once
-        if (o_part + part_bytes() + up256(4 * (size_t)vtiles) > kScratchBytes) K = 1;
-        const size_t o_done = o_part + part_bytes();
-        const size_t need = K > 1 ? o_done + up256(4 * (size_t)vtiles) : o_chk;
+        const size_t o_done = o_part + up256(16 * (size_t)K * (size_t)nv);
+        const size_t chunked = o_done + up256(4 * (size_t)vtiles);
+        // a scratch that has no room for the chunks' sums: the chunks in turn, added to the image
+        const bool in_turn = K > 1 && chunked > kScratchBytes;
+        const size_t need = K > 1 && !in_turn ? chunked : o_chk;
         if (need > kScratchBytes)
             fail(BSAR_ERR_INVALID_ARG, "the call needs %zu bytes of scratch; the fixed scratch holds %zu", need,
                  kScratchBytes);
@@ -159,18 +159,23 @@ extern "C" bsar_status bsar_backproject_mixed_noalloc(bsar_ctx* ctx, bsar_scene_
         r.off_x = (float)(ox / (2.0 * np));
         r.off_y = (float)(oy / (2.0 * np));
         MixedChunks* d_chunks = nullptr;
-        if (K > 1) {
+        if (K > 1 && !in_turn) {
             const MixedChunks c{K, 0, reinterpret_cast<double2*>(S + o_part), reinterpret_cast<int*>(S + o_done)};
             d_chunks = reinterpret_cast<MixedChunks*>(S + o_chk);
             cuda_check(cudaMemcpyAsync(d_chunks, &c, sizeof c, cudaMemcpyHostToDevice, st), "chunk record");
             cuda_check(cudaMemsetAsync(c.tile_done, 0, 4 * (size_t)vtiles, st), "clear chunk counts");
         }
         MixedReq* d_req = reinterpret_cast<MixedReq*>(S + o_req);
-        cuda_check(cudaMemcpyAsync(d_req, &r, sizeof r, cudaMemcpyHostToDevice, st), "request record");
-        MixedBatch b{d_req, nullptr, nullptr, (int)(vtiles * K), counter, status, d_chunks,
-                     (long long)ctx->tile_wait_polls};
+        MixedBatch b{d_req, nullptr, nullptr, (int)(in_turn ? vtiles : vtiles * K), counter, status, d_chunks,
+                     (long long)ctx->tile_wait_polls, 0};
         const int grid = (int)std::min<int64_t>(b.ntiles, mixed_grid_ctas());
-        launched(ctx, launch_bp_mixed(b, a.W, grid, st, K > 1), "back-projection (mixed, scratch)");
+        for (int c = 0; c < (in_turn ? K : 1); c++) {
+            const MixedReq rc = in_turn ? mixed_chunk_request(r, c, K) : r;
+            b.add = in_turn ? (c ? 2 : 1) : 0;
+            cuda_check(cudaMemcpyAsync(d_req, &rc, sizeof rc, cudaMemcpyHostToDevice, st), "request record");
+            if (c) cuda_check(cudaMemsetAsync(counter, 0, sizeof(int), st), "clear counter");
+            launched(ctx, launch_bp_mixed(b, a.W, grid, st, K > 1), "back-projection (mixed, scratch)");
+        }
         cuda_check(cudaMemcpyAsync(image_out, a.out, 16 * (size_t)nv, cudaMemcpyDeviceToHost, st), "image");
         int hstat = 0;
         cuda_check(cudaMemcpyAsync(&hstat, status, sizeof(int), cudaMemcpyDeviceToHost, st), "status");

@@ -673,11 +673,11 @@ template <int WT> struct WarpShared {
 
 // One voxel of a request over pulses [p0, p1) (k: index in the request's voxel range;
 // k >= v_count repeats the last voxel without storing it, so whole warps stay active).
-// The sum goes to dst at the voxel's image index.
+// The sum goes to dst at the voxel's image index; add: MixedBatch::add.
 template <int WT, bool CH>
 __device__ __forceinline__ void voxel_mixed(const BpArgs& a, const MixedCtx& m, const Tile& T,
                                             WarpShared<WT>* ws, bool fp16, int compact, int64_t kk, int p0, int p1,
-                                            double2* __restrict__ dst)
+                                            double2* __restrict__ dst, int add)
 {
     const int lane = threadIdx.x & 31;
     const int np = CH ? p1 : a.np;
@@ -840,9 +840,15 @@ __device__ __forceinline__ void voxel_mixed(const BpArgs& a, const MixedCtx& m, 
             }
         }
     }
-    if (kk < a.v_count)
-        (CH ? dst : a.out)[((int64_t)vx.x * a.ny + vx.y) * a.nz + vx.z] =
-            make_double2((double)accr - (double)cmpr, (double)acci - (double)cmpi);
+    if (kk < a.v_count) {
+        double2* o = (CH ? dst : a.out) + ((int64_t)vx.x * a.ny + vx.y) * a.nz + vx.z;
+        double2 s = make_double2((double)accr - (double)cmpr, (double)acci - (double)cmpi);
+        if (CH && add) {
+            const double2 q = add == 2 ? *o : make_double2(0.0, 0.0);
+            s = make_double2(q.x + s.x, q.y + s.y);
+        }
+        *o = s;
+    }
 }
 
 // The last of a tile's pulse chunks to finish adds the chunks' sums, in chunk order, into
@@ -912,7 +918,7 @@ __global__ void __launch_bounds__(128, 3) k_bp_mixed(MixedBatch b)
         const BpArgs& a = R.a;
         const MixedCtx m = req_ctx(R);
         // work item -> (128-voxel tile, pulse chunk); the unchunked kernel has one chunk
-        const int K = CH ? max(b.chunks[w.x].nchunk, 1) : 1;
+        const int K = CH && b.chunks ? max(b.chunks[w.x].nchunk, 1) : 1;
         const int tile = CH ? w.y / K : w.y;
         const int chunk = CH ? w.y - tile * K : 0;
         Tile T{tile_s, 0, 0, false};
@@ -934,16 +940,16 @@ __global__ void __launch_bounds__(128, 3) k_bp_mixed(MixedBatch b)
         }
         if constexpr (!CH) {
             voxel_mixed<WT, false>(a, m, T, ws, R.fp16 != 0, R.compact, (int64_t)w.y * 128 + threadIdx.x, 0,
-                                   0, nullptr);
+                                   0, nullptr, 0);
         } else {
             const int p0 = (int)((int64_t)chunk * a.np / K), p1 = (int)((int64_t)(chunk + 1) * a.np / K);
             double2* dst = K == 1 ? a.out : b.chunks[w.x].partial + chunk * ((int64_t)a.nx * a.ny * a.nz);
             voxel_mixed<WT, true>(a, m, T, ws, R.fp16 != 0, R.compact, (int64_t)tile * 128 + threadIdx.x,
-                                  p0, p1, dst);
+                                  p0, p1, dst, b.add);
             // the work item again from shared memory, so none of it stays live over the pulses
             const volatile int* wv = reinterpret_cast<volatile int*>(&work);
             const int2 w2 = make_int2(wv[0], wv[1]);
-            const MixedChunks C = b.chunks[w2.x];
+            const MixedChunks C = b.chunks ? b.chunks[w2.x] : MixedChunks{1, 0, nullptr, nullptr};
             if (C.nchunk > 1) {
                 const int tile2 = w2.y / C.nchunk;
                 __threadfence();   // this chunk's sums before the count that publishes them

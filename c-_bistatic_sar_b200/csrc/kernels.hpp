@@ -183,9 +183,28 @@ struct MixedBatch {
     int ntiles;
     int* counter;            // zeroed before the launch
     int* status;             // device status word (1 = a tile copy timed out)
-    const MixedChunks* chunks;   // per request, indexed as reqs (the chunked kernel only)
+    const MixedChunks* chunks;   // per request, indexed as reqs (the chunked kernel only; null: one chunk)
     long long wait_polls;        // polls of the bounded DEM-tile wait before giving up on a tile
+    int add;                     // chunked kernel, one chunk: 1, the sums are added to 0.0, 2, to the image
 };
+
+// Chunk `c` of `K` of a request as a request of its own: the pulses it holds.
+inline MixedReq mixed_chunk_request(MixedReq r, int c, int K)
+{
+    BpArgs& a = r.a;
+    const int64_t p0 = (int64_t)c * a.np / K, p1 = (int64_t)(c + 1) * a.np / K;
+    a.tx += 3 * p0;
+    a.rx += 3 * p0;
+    a.ref_L += p0;
+    a.ref_phase += p0;
+    a.ref_bin_i += p0;
+    a.ref_bin_f += p0;
+    if (a.rc32) a.rc32 += p0 * a.nr;
+    if (a.rc16) a.rc16 += p0 * a.nr;
+    if (a.scale16) a.scale16 += p0;
+    a.np = (int)(p1 - p0);
+    return r;
+}
 
 // Whether node scans may run on candidate lists, whose slack takes the ratio of the indices as
 // a weight: both are positive numbers, in FP32 too.
@@ -226,7 +245,8 @@ int mixed_grid_ctas();   // persistent grid size (SMs x resident CTAs)
 // against one wave of 128-pulse chunks measured 2.60 against 3.95 ms on a 161 x 161 x 1
 // slice of 1024 pulses and 4.4 against 8.3 ms on 97 x 83 x 11 voxels of 701 pulses.  A
 // property of the request and the device only, so every path gives the same request the
-// same image.
+// same image: where there is no room for the chunks' sums the chunks run one after the other and
+// add to the image (MixedBatch::add).
 constexpr int kMaxChunks = 8;
 constexpr int kMaxChunkedTiles = 4095;
 int mixed_chunks(int64_t voxels, int pulses);
