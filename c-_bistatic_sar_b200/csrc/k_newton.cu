@@ -9,14 +9,14 @@
 // whole block, a solve is two table reads per node.  The other solves rank the list and polish
 // the facets around the best node (active-set Newton, one final step on the winning facet).
 //
-// A CTA's warps share 32 voxels and split the pulses into consecutive parts; the parts'
-// sums are added in pulse order.  The split follows the whole grid's size, so a range of
-// the grid has the image's bits.  Parts differ in work (solves that a list's tables answer
-// against solves that are polished): with one part a warp, the CTA's other warps waited for
-// the slowest for a third of their time, so a warp has one part of 3/4 of its share, and the
-// rest is handed out in parts of a quarter as warps get free.  81 x 77 x 13 voxels x 512
-// pulses: 6.45 to 5.97 ms, one plane 1.34 to 1.15, 60 planes 23.4 to 21.1 (halves and halves:
-// 6.11, 1.15, 21.4).
+// A CTA's warps share 32 voxels and take the pulses in consecutive parts of 16 (at most 32
+// parts), handed out as warps get free: parts differ in work (solves that a list's tables
+// answer against solves that are polished), and with one part a warp the others waited for the
+// slowest for a third of their time.  The parts' sums are added in pulse order.  The split is a
+// function of the pulses alone, so a voxel's value does not depend on the grid it is computed
+// in.  81 x 77 voxels x planes x pulses, parts of 16 / 20 / 24 / 32 pulses: 13 x 512 5.36 / 5.36 /
+// 5.36 / 5.39 ms, 1 x 512 0.81 / 0.89 / 0.95 / 1.09, 60 x 512 21.1 / 20.7 / 20.7 / 20.4, 13 x 128
+// 2.36 / 2.48 / 2.61 / 2.59; with a split that followed the grid's size 5.71, 0.96, 20.0, 2.31.
 //
 // What bounds it: instruction latency and fetch at 12 warps an SM (an issue every third
 // cycle; the FP64 unit is 16 % busy).  The same scene took 82 ms with one warp per voxel and
@@ -228,20 +228,22 @@ struct NewtonWarp {
 
 }  // namespace
 
-// First pulse of part k of 2 WPC: WPC parts of 3/4 of the pulses, then WPC of the rest.
-template <int WPC> __device__ __forceinline__ int part_begin(int k, int np)
+// The parts a CTA's warps take: a function of the pulses alone, so that a voxel's sum has the
+// same order, and its value the same bits, in every grid.
+constexpr int kMaxParts = 32, kPartPulses = 16;
+static int pulse_parts(int np)
 {
-    const int u = k < WPC ? 3 * k : 2 * WPC + k;     // of 4 WPC units
-    return (int)((int64_t)u * np / (4 * WPC));
+    const int n = np / kPartPulses;
+    return n < 1 ? 1 : (n > kMaxParts ? kMaxParts : n);
 }
 
 template <int WPC>
 __global__ void __launch_bounds__(32 * WPC, WPC < 8 ? 12 / WPC : 16 / WPC)
-    k_bp_newton(BpArgs a, float start_band, int compact)
+    k_bp_newton(BpArgs a, float start_band, int compact, int nparts)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     NewtonWarp* ws = reinterpret_cast<NewtonWarp*>(smem_raw) + (threadIdx.x >> 5);
-    __shared__ double2 part[2 * WPC][32];
+    double2 (*part)[32] = reinterpret_cast<double2(*)[32]>(reinterpret_cast<NewtonWarp*>(smem_raw) + WPC);
     __shared__ int next;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const DemView& d = a.dem;
@@ -264,8 +266,8 @@ __global__ void __launch_bounds__(32 * WPC, WPC < 8 ? 12 / WPC : 16 / WPC)
     __syncthreads();
     const double inv_c = 1.0 / a.c, inv_lambda = 1.0 / a.lambda;
     const Heights64 zat(d);
-    for (int k = w; k < 2 * WPC;) {
-        const int p0 = part_begin<WPC>(k, a.np), p1 = part_begin<WPC>(k + 1, a.np);
+    for (int k = w; k < nparts;) {
+        const int p0 = (int)((int64_t)k * a.np / nparts), p1 = (int)((int64_t)(k + 1) * a.np / nparts);
         if (lane < 2) ws->h[lane].si = ws->h[lane].sj = -1;
         __syncwarp();
         double accr = 0.0, acci = 0.0;
@@ -368,7 +370,7 @@ __global__ void __launch_bounds__(32 * WPC, WPC < 8 ? 12 / WPC : 16 / WPC)
     __syncthreads();
     if (w == 0 && kk < a.v_count) {
         double accr = 0.0, acci = 0.0;
-        for (int q = 0; q < 2 * WPC; q++) {
+        for (int q = 0; q < nparts; q++) {
             accr += part[q][lane].x;
             acci += part[q][lane].y;
         }
@@ -378,10 +380,11 @@ __global__ void __launch_bounds__(32 * WPC, WPC < 8 ? 12 / WPC : 16 / WPC)
 
 template <int WPC> static cudaError_t launch_wpc(const BpArgs& a, float band, int compact, cudaStream_t st)
 {
-    const size_t sm = sizeof(NewtonWarp) * WPC;
+    const int nparts = pulse_parts(a.np);
+    const size_t sm = sizeof(NewtonWarp) * WPC + sizeof(double2) * 32 * nparts;
     cudaError_t e = cudaFuncSetAttribute(k_bp_newton<WPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    k_bp_newton<WPC><<<(unsigned)((a.v_count + 31) / 32), 32 * WPC, sm, st>>>(a, band, compact);
+    k_bp_newton<WPC><<<(unsigned)((a.v_count + 31) / 32), 32 * WPC, sm, st>>>(a, band, compact, nparts);
     return cudaGetLastError();
 }
 

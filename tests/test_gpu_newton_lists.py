@@ -91,6 +91,30 @@ def test_large_grid_has_the_small_grids_image(ctx, n_pulses):
     assert rel_l2(big[:3], small) <= 2e-9
 
 
+@pytest.mark.parametrize("n_pulses", [1, 17, 50, 300, 1100])
+def test_a_voxel_has_one_value_in_every_grid(ctx, n_pulses):
+    """Grids that take 2 to 16 warps per 32 voxels, ranges of them and single voxels: the same
+    bits, since the order of a voxel's sum follows the pulses alone."""
+    spec = S.scaled(S.config_spec(2), n_pulses=n_pulses, n_samples=4096, n_scatterers=2, nx=61, ny=63, nz=31, dxy=0.02)
+    sc = S.make_scene(spec, with_raw=False)
+    rng = np.random.default_rng(6)
+    sc.raw = rng.normal(size=(n_pulses, 4096)) + 1j * rng.normal(size=(n_pulses, 4096))
+    sid = bsar.upload_scene(ctx, sc)
+    form = dict(solver="newton", legs="per_pulse", precision="fp64")
+    try:
+        big = ctx.backproject(sid, sc.gx, sc.gy, sc.gz, **form)
+        for x, y, z in ((slice(0, 61), slice(0, 63), slice(3, 4)), (slice(5, 9), slice(7, 16), slice(2, 5)),
+                        (slice(0, 61), slice(0, 63), slice(0, 13)), (slice(60, 61), slice(2, 3), slice(30, 31))):
+            small = ctx.backproject(sid, sc.gx[x], sc.gy[y], sc.gz[z], **form)
+            assert np.array_equal(small, big[x, y, z])
+        part = ctx.backproject_range(sid, sc.gx, sc.gy, sc.gz, 1001, 5002, **form)
+    finally:
+        ctx.scene_release(sid)
+    flat = np.arange(1001, 1001 + 5002)                      # z -> x -> y
+    at = (flat // 63) % 61, flat % 63, flat // (61 * 63)
+    assert np.array_equal(part[at], big[at])
+
+
 @pytest.mark.parametrize("seed,voxel", [(6, (62, 0, 22)), (6, (65, 25, 16)), (6, (56, 35, 3)), (3, (7, 7, 21)),
                                         (26, (34, 40, 0))])
 def test_every_open_facet_is_polished(ctx, oracle, seed, voxel):
