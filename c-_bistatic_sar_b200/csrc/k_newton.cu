@@ -9,7 +9,7 @@
 // whole block, a solve is two table reads per node.  The other solves rank the list and polish
 // the facets around the best node (active-set Newton, one final step on the winning facet).
 //
-// A CTA's warps share 32 voxels and take the pulses in consecutive parts of 16 (at most 32
+// A CTA's warps share 32 voxels and take the pulses in consecutive parts of 16 (8 to 32
 // parts), handed out as warps get free: parts differ in work (solves that a list's tables
 // answer against solves that are polished), and with one part a warp the others waited for the
 // slowest for a third of their time.  The parts' sums are added in pulse order.  The split is a
@@ -233,8 +233,8 @@ struct NewtonWarp {
 constexpr int kMaxParts = 32, kPartPulses = 16;
 static int pulse_parts(int np)
 {
-    const int n = np / kPartPulses;
-    return n < 1 ? 1 : (n > kMaxParts ? kMaxParts : n);
+    const int least = np < 8 ? np : 8, n = np / kPartPulses;
+    return n < least ? least : (n > kMaxParts ? kMaxParts : n);
 }
 
 template <int WPC>
