@@ -198,7 +198,7 @@ __device__ __forceinline__ double polish64(const DemView& d, const ListGrid& m, 
             m1 = true;
         }
         const double L = m1 ? facet_path(F, l, u, v) : node;
-        if (m1 && keeps && fabs(L - node) <= 1e-13 * node) return polish_tied64(d, l, bi, bj);
+        if (m1 && keeps && u == (kx ? 0.0 : 1.0) && v == (ky ? 0.0 : 1.0)) return polish_tied64(d, l, bi, bj);
         if (L < best) {
             best = L;
             step = true;
