@@ -478,7 +478,9 @@ __device__ __forceinline__ int2 rank_list(const DemView& d, const MixedCtx& m, c
 // has the gradient (Gx + Gz zx, Gy + Gz zy), zx and zy the facet's slopes along the edges
 // through the node (one-sided differences: backward where u0 = 1, forward where u0 = 0).
 // When it points out of the facet on both axes, the corner is that facet's minimum and the
-// facet keeps the node's path; the others take the Newton steps.  Each lane takes its own
+// facet keeps the node's path; the others take the Newton steps.  A facet whose steps end back
+// on the node ties with those that keep it, and the first in order wins, as in the FP64 solver:
+// one more step would leave the node (voxels at the surface).  Each lane takes its own
 // facets one after the other, so lanes whose crossings lie on different sides of a node step
 // together.
 __device__ __forceinline__ bool polish_leg(const MixedCtx& m, const Tile& T, const Leg& l, int bi, int bj, int& bfi,
@@ -525,7 +527,9 @@ __device__ __forceinline__ bool polish_leg(const MixedCtx& m, const Tile& T, con
     unsigned todo = facets & ((unsigned)(ixm || iym) | (unsigned)(ixm || iyp) << 1 | (unsigned)(ixp || iym) << 2 |
                               (unsigned)(ixp || iyp) << 3);
     bool moved = false;
-    float best = todo == facets ? INFINITY : Lnode;     // a facet whose minimum is the node gives its path
+    // a facet whose minimum is the node gives its path; the first of them
+    const int first = todo == facets ? 4 : __ffs(facets & ~todo) - 1;
+    float best = todo == facets ? INFINITY : Lnode;
 #pragma unroll 1
     while (todo) {
         const int k = __ffs(todo) - 1;
@@ -555,6 +559,7 @@ __device__ __forceinline__ bool polish_leg(const MixedCtx& m, const Tile& T, con
             if (!facet_step32(F, A32, B32, na, nb, u, v)) break;
             m1 = true;
         }
+        if (k > first && u == (kx ? 0.0f : 1.0f) && v == (ky ? 0.0f : 1.0f)) continue;
         const float L = m1 ? facet_eval32(F, A32, B32, na, nb, u, v) : Lnode;
         if (L < best || (L == best && !moved)) {
             best = L;
