@@ -394,7 +394,9 @@ typedef struct bsar_server_stats {
     double p50_ms, p99_ms, mean_ms, max_ms;   /* submission -> image on the host */
     double voxel_pulses;                      /* work of the completed requests   */
     double busy_s;                            /* first submission -> last completion */
-    uint64_t peak_inflight;                   /* most requests admitted at once  */
+    uint64_t peak_inflight;                   /* most requests admitted at once: from the slot
+                                                 and budget a request takes until its image is
+                                                 on the host or it has failed              */
     uint64_t peak_reserved_bytes;             /* most HBM reserved at once       */
     double batch_busy_s;                      /* time with a batch on the device, as the
                                                  server thread sees launches and completions */
