@@ -1,9 +1,10 @@
 // dev_common.cuh -- device-side DEM view and the reference's DEM / Fermat arithmetic.
 //
-// Everything in the FP64 section is written to reproduce the reference's results bit
-// for bit: the translation units that include it are compiled with --fmad=false, and
-// every expression keeps the reference's operation order (sqrt and division are IEEE
-// correctly rounded in CUDA, as on the host).
+// Everything in the FP64 section keeps the reference's operation order (sqrt and division
+// are IEEE correctly rounded in CUDA, as on the host).  The units whose results reproduce the
+// reference's bit for bit are compiled with --fmad=false (k_plain.cu, k_pulse.cu, k_synth.cu);
+// k_mixed.cu, k_newton.cu and k_crossings.cu use the DEM lookup, the flat start and the facets
+// with contraction on, within their tolerances.
 #pragma once
 
 #include <cstdint>

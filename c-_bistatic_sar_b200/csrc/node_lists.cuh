@@ -1,5 +1,5 @@
 // node_lists.cuh -- candidate lists of a node scan, shared by a warp's (antenna, voxel)
-// pairs, for the mixed (k_mixed.cu) and the FP64 (k_plain.cu) back-projection.  FP32
+// pairs, for the mixed (k_mixed.cu) and the FP64 Newton (k_newton.cu) back-projection.  FP32
 // arithmetic with explicit FMA where a value must not depend on the unit's --fmad setting.
 #pragma once
 

@@ -97,6 +97,9 @@ typedef struct bsar_fermat_opts {
 /* ---------------------------------------------------------------------------------
  * Context
  * ------------------------------------------------------------------------------- */
+/* Copies of large pageable buffers (32 MB up, or 8 MB in calls that return as much, and 2 MB
+ * down) go through up to five threads and 12 MB of pinned host memory that a context makes at
+ * the first such copy and keeps until bsar_destroy.  Pinned buffers take neither. */
 bsar_status bsar_create(bsar_ctx** out, const bsar_opts* opts);
 void bsar_destroy(bsar_ctx* ctx);
 const char* bsar_status_string(bsar_status status);
