@@ -281,10 +281,11 @@ __global__ void __launch_bounds__(32 * WPC, WPC < 8 ? 12 / WPC : 16 / WPC)
     __syncthreads();
     const double inv_c = 1.0 / a.c, inv_lambda = 1.0 / a.lambda;
     const Heights64 zat(d);
+    // a first guess for each list, from part to part (the list does not depend on it)
+    if (lane < 2) ws->h[lane].si = ws->h[lane].sj = -1;
+    __syncwarp();
     for (int k = w; k < nparts;) {
         const int p0 = (int)((int64_t)k * a.np / nparts), p1 = (int)((int64_t)(k + 1) * a.np / nparts);
-        if (lane < 2) ws->h[lane].si = ws->h[lane].sj = -1;
-        __syncwarp();
         double accr = 0.0, acci = 0.0;
         int n;
         for (int i = p0; i < p1; i += n) {
