@@ -14,14 +14,15 @@
 // answer against solves that are polished), and with one part a warp the others waited for the
 // slowest for a third of their time.  The parts' sums are added in pulse order.  The split is a
 // function of the pulses alone, so a voxel's value does not depend on the grid it is computed
-// in.  81 x 77 voxels x planes x pulses, parts of 16 / 20 / 24 / 32 pulses: 13 x 512 5.36 / 5.36 /
-// 5.36 / 5.39 ms, 1 x 512 0.81 / 0.89 / 0.95 / 1.09, 60 x 512 21.1 / 20.7 / 20.7 / 20.4, 13 x 128
-// 2.36 / 2.48 / 2.61 / 2.59; with a split that followed the grid's size 5.71, 0.96, 20.0, 2.31.
+// in.  81 x 77 voxels x planes x pulses at two warps per 32 voxels, parts of 16 / 20 / 24 / 32
+// pulses: 13 x 512 5.36 / 5.36 / 5.36 / 5.39 ms, 1 x 512 0.81 / 0.89 / 0.95 / 1.09, 60 x 512 21.1 /
+// 20.7 / 20.7 / 20.4, 13 x 128 2.36 / 2.48 / 2.61 / 2.59.  At four and eight warps (launch_bp_newton)
+// 13 x 512 4.85, 1 x 512 0.82, 60 x 512 19.6; a split that followed the grid's size took 5.71, 0.96
+// and 20.0.
 //
-// What bounds it: instruction latency and fetch at 12 warps an SM (an issue every third
-// cycle; the FP64 unit is 16 % busy).  The same scene took 82 ms with one warp per voxel and
-// every pulse's own scan of (2W+1)^2 nodes, two FP64 square roots each.  16 warps an SM (128
-// registers) are no faster: 5.95 ms.
+// What bounds it: instruction latency and fetch at 12 to 16 warps an SM (an issue in 39 % of the
+// cycles; the FP64 unit is 18 % busy).  The same scene took 82 ms with one warp per voxel and
+// every pulse's own scan of (2W+1)^2 nodes, two FP64 square roots each.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -410,16 +411,17 @@ cudaError_t launch_bp_newton(const BpArgs& a, cudaStream_t st)
     const int compact = a.v_begin % plane == 0 && a.v_count % plane == 0;
     const float band = list_start_band(a.dem);
     // warps per 32 voxels: enough for about three waves of 16 warps per SM; more than four only
-    // with at least two pulse blocks each.  Two where that is enough: 60 planes of 6237 voxels
-    // 20.0 ms, with four 21.1; 26 planes 9.24 and 9.69 (one warp: 60 planes 19.5)
+    // with at least two pulse blocks each, eight from 512 pulses on (16 parts of a warp's own
+    // keep them busy): 81 x 77 x 13 voxels x 512 pulses 4.85 ms, with four 5.27; 60 planes 19.6 and
+    // 19.8; 161 x 161 x 81 x 1024 141.6 and 143.4, x 100 43.4 and 39.1.  Two are slower on every
+    // grid (60 planes 20.7)
     constexpr int64_t kWarps = 148 * 48;
     const int64_t tiles = (plane * a.nz + 31) / 32;
-    int wpc = tiles * 2 < kWarps ? 4 : 2;
+    int wpc = a.np >= 512 ? 8 : 4;
     while (wpc < 16 && tiles * wpc < kWarps && a.np >= 2 * wpc * kBlockPulses) wpc *= 2;
     if (wpc == 16) return launch_wpc<16>(a, band, compact, st);
     if (wpc == 8) return launch_wpc<8>(a, band, compact, st);
-    if (wpc == 4) return launch_wpc<4>(a, band, compact, st);
-    return launch_wpc<2>(a, band, compact, st);
+    return launch_wpc<4>(a, band, compact, st);
 }
 
 }  // namespace bsar

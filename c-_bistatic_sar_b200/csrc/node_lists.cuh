@@ -533,10 +533,10 @@ __device__ __forceinline__ bool node_pinned(const ListGrid& m, const Z& zat, int
     const float z = zat(i, j);
     const float sxb = (z - zat(i - 1, j)) * m.istepx, sxf = (zat(i + 1, j) - z) * m.istepx;
     const float syb = (z - zat(i, j - 1)) * m.istepy, syf = (zat(i, j + 1) - z) * m.istepy;
-    const float round = 2.5e-7f * (m.extent + fabsf(z));
+    const float coord = 2.5e-7f * (m.extent + fabsf(z));
     const float slope = 1.3e-7f * (nE + nG) * fabsf(z) * fmaxf(m.istepx, m.istepy);
-    rE += round;
-    rG += round;
+    rE += coord;
+    rG += coord;
     const float x = (float)i * m.stepx, y = (float)j * m.stepy;
     const float ex = x - E[0], ey = y - E[1], ez = z - E[2];
     const float gx = x - G[0], gy = y - G[1], gz = z - G[2];

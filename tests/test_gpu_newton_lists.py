@@ -93,7 +93,7 @@ def test_large_grid_has_the_small_grids_image(ctx, n_pulses):
 
 @pytest.mark.parametrize("n_pulses", [1, 17, 50, 300, 1100])
 def test_a_voxel_has_one_value_in_every_grid(ctx, n_pulses):
-    """Grids that take 2 to 16 warps per 32 voxels, ranges of them and single voxels: the same
+    """Grids that take 4 to 16 warps per 32 voxels, ranges of them and single voxels: the same
     bits, since the order of a voxel's sum follows the pulses alone."""
     spec = S.scaled(S.config_spec(2), n_pulses=n_pulses, n_samples=4096, n_scatterers=2, nx=61, ny=63, nz=31, dxy=0.02)
     sc = S.make_scene(spec, with_raw=False)
