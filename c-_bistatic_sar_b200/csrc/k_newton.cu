@@ -20,8 +20,8 @@
 // 13 x 512 4.85, 1 x 512 0.82, 60 x 512 19.6; a split that followed the grid's size took 5.71, 0.96
 // and 20.0.
 //
-// What bounds it: instruction latency and fetch at 12 to 16 warps an SM (an issue in 39 % of the
-// cycles; the FP64 unit is 18 % busy).  The same scene took 82 ms with one warp per voxel and
+// What bounds it: instruction latency and fetch at 12 to 16 warps an SM (an issue in 44 % of the
+// cycles; the FP64 unit is 20 % busy).  The same scene took 82 ms with one warp per voxel and
 // every pulse's own scan of (2W+1)^2 nodes, two FP64 square roots each.
 #include <cuda_runtime.h>
 
